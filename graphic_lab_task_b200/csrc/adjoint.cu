@@ -197,7 +197,7 @@ lrt_status check_material_ranges(lrt_scene* s, const char* who, const uint32_t* 
 // schedule (natural tile order with LRT_TRACE_NATURAL_ORDER, the only flag).
 lrt_status lambert_begin(lrt_scene* s, const char* who, const float* rays_dev, uint64_t n, uint32_t width,
                          uint32_t height, const float* light, uint32_t flags, cudaStream_t stream, StreamSlot** slot,
-                         DevScene* S, int* grid)
+                         DevScene* S, int* blocks)
 {
   lrt_status st = begin(s, stream, slot, S);
   if (st != LRT_OK) return st;
@@ -209,8 +209,7 @@ lrt_status lambert_begin(lrt_scene* s, const char* who, const float* rays_dev, u
   if ((st = check_rays(s, rays_dev)) != LRT_OK) return st;
   const uint64_t warps =
       width ? uint64_t((width + kImgTileW - 1) / kImgTileW) * ((height + kImgTileH - 1) / kImgTileH) : (n + 31) / 32;
-  *grid = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(s->dev->grid),
-                                                       (warps * 32 + kTraceThreads - 1) / kTraceThreads)));
+  *blocks = blocks_for(warps);
   return LRT_OK;
 }
 
@@ -240,9 +239,9 @@ lrt_status render_lambert(lrt_scene* s, const float* rays_dev, uint64_t n, uint3
 {
   StreamSlot* slot = nullptr;
   DevScene S;
-  int grid = 1;
+  int blocks = 1;
   lrt_status st = lambert_begin(s, "lrt_render_lambert", rays_dev, n, width, height, light, flags, stream, &slot, &S,
-                                &grid);
+                                &blocks);
   if (st != LRT_OK) return st;
   if ((st = check_rays(s, image_dev)) != LRT_OK) return st;
   if (n == 0) return LRT_OK;
@@ -253,7 +252,7 @@ lrt_status render_lambert(lrt_scene* s, const float* rays_dev, uint64_t n, uint3
   if ((st = sched_prepare(s, stream, width, height, natural, &rd, &wr)) != LRT_OK) return st;
   cudaError_t e = lrt_exact::launch_render_lambert(S, reinterpret_cast<const float4*>(rays_dev), n,
                                                    make_float3(light[0], light[1], light[2]), image_dev, &slot->work,
-                                                   &slot->err, s->dev->stackCap, grid, stream, width, height, rd, wr);
+                                                   &slot->err, s->dev->stackCap, blocks, stream, width, height, rd, wr);
   if (e != cudaSuccess) return cuda_fail(s, e, "render launch");
   sched_commit(s, stream, width, height, natural);
   return LRT_OK;
@@ -265,9 +264,9 @@ lrt_status adjoint_lambert(lrt_scene* s, const float* rays_dev, uint64_t n, uint
 {
   StreamSlot* slot = nullptr;
   DevScene S;
-  int grid = 1;
+  int blocks = 1;
   lrt_status st = lambert_begin(s, "lrt_adjoint_lambert_sbs", rays_dev, n, width, height, light, flags, stream, &slot,
-                                &S, &grid);
+                                &S, &blocks);
   if (st != LRT_OK) return st;
   if (!dimage_dev || !grad_dev) return fail(s, LRT_ERR_INVALID_ARGUMENT, "lrt_adjoint_lambert_sbs: NULL argument");
   if (n == 0) return LRT_OK;
@@ -278,7 +277,7 @@ lrt_status adjoint_lambert(lrt_scene* s, const float* rays_dev, uint64_t n, uint
   if ((st = sched_prepare(s, stream, width, height, natural, &rd, &wr)) != LRT_OK) return st;
   cudaError_t e = lrt_exact::launch_adjoint_lambert(S, reinterpret_cast<const float4*>(rays_dev), n,
                                                     make_float3(light[0], light[1], light[2]), dimage_dev, grad_dev,
-                                                    &slot->work, &slot->err, s->dev->stackCap, grid, stream, width,
+                                                    &slot->work, &slot->err, s->dev->stackCap, blocks, stream, width,
                                                     height, rd, wr);
   if (e != cudaSuccess) return cuda_fail(s, e, "adjoint launch");
   sched_commit(s, stream, width, height, natural);
@@ -292,7 +291,7 @@ lrt_status adjoint_lambert(lrt_scene* s, const float* rays_dev, uint64_t n, uint
 // and the sums (8 + 16 + 16 bytes per pixel) are kept with the scene.
 lrt_status render_outline_border(lrt_scene* s, const DevScene& S, StreamSlot* slot, const DevCamera& cam,
                                  const DevLights& L, const DevMaterials& M, const DevRenderModes& RM,
-                                 uint32_t* image_dev, int grid, cudaStream_t stream)
+                                 uint32_t* image_dev, int blocks, cudaStream_t stream)
 {
   DeviceScene* d = s->dev;
   const uint64_t n = uint64_t(cam.width) * cam.height;
@@ -318,7 +317,7 @@ lrt_status render_outline_border(lrt_scene* s, const DevScene& S, StreamSlot* sl
     uint32_t* wr = nullptr;
     lrt_status st = sched_prepare(s, stream, cam.width, cam.height, false, &rd, &wr);
     if (st != LRT_OK) return st;
-    e = lrt_exact::launch_outline_fill(S, cam, L, M, RM, smp, tm, col, &slot->work, &slot->err, d->stackCap, grid,
+    e = lrt_exact::launch_outline_fill(S, cam, L, M, RM, smp, tm, col, &slot->work, &slot->err, d->stackCap, blocks,
                                        stream, rd, wr);
     if (e != cudaSuccess) return cuda_fail(s, e, "outline G-buffer launch");
     sched_commit(s, stream, cam.width, cam.height, false);
@@ -445,7 +444,7 @@ lrt_status lrt_render_rgba8(lrt_scene* s, const lrt_camera* camera, const lrt_li
   std::memcpy(L.background, background, sizeof(L.background));
   DeviceScene* d = s->dev;
   const uint64_t tiles = uint64_t((cam.width + 7) / 8) * ((cam.height + 3) / 4);
-  const int grid = int(std::min<uint64_t>(uint64_t(d->grid), (tiles * 32 + kTraceThreads - 1) / kTraceThreads));
+  const int blocks = blocks_for(tiles);
   const uint32_t* rd = nullptr;
   uint32_t* wr = nullptr;
   DevMaterials M{};
@@ -457,14 +456,10 @@ lrt_status lrt_render_rgba8(lrt_scene* s, const lrt_camera* camera, const lrt_li
   M.texs = d->texTable;
   M.texCount = d->texTable ? uint32_t(s->texDims.size() / 2) : 0u;
   M.triTc = d->triTc;
-  if (mode == LRT_RENDER_MODE_OUTLINE_BORDER) return render_outline_border(s, S, slot, cam, L, M, RM, image_dev, grid, stream);
+  if (mode == LRT_RENDER_MODE_OUTLINE_BORDER) return render_outline_border(s, S, slot, cam, L, M, RM, image_dev, blocks, stream);
   if ((st = sched_prepare(s, stream, cam.width, cam.height, false, &rd, &wr)) != LRT_OK) return st;
-  // one LAMBERT_NO_TEX sample of a brick-only scene: the 80-register kernel and its grid
-  const bool bricks = d->bricksOnly && mode == LRT_RENDER_MODE_LAMBERT_NO_TEX && RM.samples == 1 && !RM.transparency;
-  const int rgrid = bricks ? int(std::min<uint64_t>(uint64_t(d->gridBricks), (tiles * 32 + kTraceThreads - 1) / kTraceThreads))
-                           : grid;
   const cudaError_t e = lrt_exact::launch_render_rgba8(S, cam, L, image_dev, &slot->work, &slot->err, d->stackCap,
-                                                       rgrid, stream, rd, wr, &M, &RM, bricks);
+                                                       blocks, stream, rd, wr, &M, &RM);
   if (e != cudaSuccess) return cuda_fail(s, e, "render launch");
   sched_commit(s, stream, cam.width, cam.height, false);
   return LRT_OK;
@@ -574,12 +569,12 @@ lrt_status lrt_fill_gbuffer_transparency(lrt_scene* s, const lrt_camera* camera,
   M.offsets = reinterpret_cast<const uint2*>(d->matOffsets);
   std::memcpy(M.background, background, sizeof(M.background));
   const uint64_t tiles = uint64_t((cam.width + 7) / 8) * ((cam.height + 3) / 4);
-  const int grid = int(std::min<uint64_t>(uint64_t(d->grid), (tiles * 32 + kTraceThreads - 1) / kTraceThreads));
+  const int blocks = blocks_for(tiles);
   const uint32_t* rd = nullptr;
   uint32_t* wr = nullptr;
   if ((st = sched_prepare(s, stream, cam.width, cam.height, false, &rd, &wr)) != LRT_OK) return st;
   const cudaError_t e = lrt_exact::launch_fill_gbuffer_transparency(
-      S, cam, M, reinterpret_cast<float4*>(transparency_dev), hits_dev, &slot->work, &slot->err, d->stackCap, grid,
+      S, cam, M, reinterpret_cast<float4*>(transparency_dev), hits_dev, &slot->work, &slot->err, d->stackCap, blocks,
       stream, rd, wr);
   if (e != cudaSuccess) return cuda_fail(s, e, "transparency launch");
   sched_commit(s, stream, cam.width, cam.height, false);

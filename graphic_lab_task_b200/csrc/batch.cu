@@ -26,7 +26,6 @@ struct lrt_camera_batch {
   std::vector<uint64_t> offsets; // ncams + 1
   lrt::DevBatchShape shape{8, 4, 1, 0};
   uint32_t ntiles = 0;
-  int grid = 0;
   // device / pinned state
   lrt::DevBatchCamera* hostTable = nullptr; // pinned, copied by the graph's memcpy node
   lrt::DevBatchCamera* devTable = nullptr;
@@ -80,12 +79,9 @@ lrt_status set_shape(lrt_camera_batch* b, const DevBatchShape& sh)
   if (sh.stackCap < s->info.maxBlasDepth + 1 || sh.stackCap > kMaxStackDev + 1)
     return fail(s, LRT_ERR_INVALID_ARGUMENT, "batch shape: stack capacity %u outside [%u, %u]", sh.stackCap,
                 s->info.maxBlasDepth + 1, kMaxStackDev + 1);
-  int perSm = 0, sms = 0;
-  cudaError_t e = lrt_exact::cameras_occupancy(sh.stackCap, &perSm);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-  if (e != cudaSuccess) return cuda_fail(s, e, "batch occupancy");
+  cudaError_t e = lrt_exact::set_cameras_smem(s->dev->S.kind);
+  if (e != cudaSuccess) return cuda_fail(s, e, "batch shared memory");
   b->shape = sh;
-  b->grid = std::max(1, perSm) * sms;
   fill_table(b);
   if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
   if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
@@ -110,9 +106,8 @@ cudaError_t enqueue(lrt_camera_batch* b, lrt_hit* hits, cudaStream_t stream, con
   if (e == cudaSuccess) e = cudaMemsetAsync(b->state, 0, sizeof(unsigned long long), stream);
   if (e == cudaSuccess) {
     const DevScene S = scene_params(b->scene);
-    const int grid = int(std::min<uint64_t>(uint64_t(b->grid), (uint64_t(b->ntiles) * 32 + kTraceThreads - 1) / kTraceThreads));
     e = lrt_exact::launch_trace_cameras(S, b->devTable, b->ncams, b->ntiles, b->shape, hits, b->state,
-                                        reinterpret_cast<uint32_t*>(b->state + 1), std::max(1, grid), stream, lights,
+                                        reinterpret_cast<uint32_t*>(b->state + 1), blocks_for(b->ntiles), stream, lights,
                                         image);
   }
   return e;

@@ -166,21 +166,18 @@ lrt_status launch(lrt_scene* s, const float4* rays, lrt_hit* hits, uint64_t n, c
   }
   const uint64_t warps = img_w ? uint64_t((img_w + kImgTileW - 1) / kImgTileW) * ((img_h + kImgTileH - 1) / kImgTileH)
                                : (n + group - 1) / group;
-  // image-order traces of brick-only scenes use the 80-register kernel (its own grid)
-  const bool bricks = img_w && !count && d->bricksOnly;
-  const int grid = int(std::min<uint64_t>(uint64_t(bricks ? d->gridBricks : d->grid),
-                                          (warps * 32 + kTraceThreads - 1) / kTraceThreads));
+  const int blocks = blocks_for(warps);
   const bool natural = !img_w || count || (flags & LRT_TRACE_NATURAL_ORDER);
   const uint32_t* rd = nullptr;
   uint32_t* wr = nullptr;
   lrt_status st = sched_prepare(s, stream, img_w, img_h, natural, &rd, &wr);
   if (st != LRT_OK) return st;
   if (flags & LRT_TRACE_FAST_MATH)
-    e = lrt_fast::launch_trace(S, rays, hits, n, &slot->work, slot->counters, err, d->stackCap, grid, stream, count,
-                               img_w, img_h, rd, wr, group, bricks);
+    e = lrt_fast::launch_trace(S, rays, hits, n, &slot->work, slot->counters, err, d->stackCap, blocks, stream, count,
+                               img_w, img_h, rd, wr, group);
   else
-    e = lrt_exact::launch_trace(S, rays, hits, n, &slot->work, slot->counters, err, d->stackCap, grid, stream,
-                                count, img_w, img_h, rd, wr, group, bricks);
+    e = lrt_exact::launch_trace(S, rays, hits, n, &slot->work, slot->counters, err, d->stackCap, blocks, stream,
+                                count, img_w, img_h, rd, wr, group);
   if (e != cudaSuccess) return cuda_fail(s, e, "trace launch");
   sched_commit(s, stream, img_w, img_h, natural);
   return LRT_OK;
@@ -402,11 +399,13 @@ lrt_status device_upload(lrt_scene* s)
   // scenes: raise it once to the largest stack any scene may use.
   e = lrt_exact::set_trace_smem(kMaxStack + 1);
   if (e == cudaSuccess) e = lrt_fast::set_trace_smem(kMaxStack + 1);
-  int perSm = 0, perSmBricks = 0, sms = 0;
-  d->bricksOnly = !h.geomTags.empty() &&
-                  std::all_of(h.geomTags.begin(), h.geomTags.end(), [](uint32_t t) { return t == LRT_TAG_SDF_BRICK; });
-  if (e == cudaSuccess) e = lrt_exact::trace_occupancy(d->stackCap, &perSm);
-  if (e == cudaSuccess) e = lrt_exact::trace_occupancy(d->stackCap, &perSmBricks, true);
+  int perSm = 0, sms = 0;
+  uint32_t kinds = 0;
+  for (uint32_t t : h.geomTags)
+    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
+           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
+  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
+  if (e == cudaSuccess) e = lrt_exact::trace_occupancy(d->stackCap, S.kind, &perSm);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
   if (e == cudaSuccess) e = cudaMalloc(&d->slots, sizeof(StreamSlot) * kMaxStreams);
   if (e == cudaSuccess) {
@@ -419,7 +418,7 @@ lrt_status device_upload(lrt_scene* s)
     return st;
   }
   d->grid = std::max(1, perSm) * sms;
-  d->gridBricks = std::max(1, perSmBricks) * sms;
+  S.sms = uint32_t(sms);
   // The allocation-free trace's static array is looked up here, with the
   // scene's device current, not in the trace call: under lazy module loading
   // the first lookup loads this file's module and places the array in device
@@ -718,12 +717,12 @@ extern "C" lrt_status lrt_trace_nearest_noalloc(lrt_scene* s, const float* rays,
     if (e != cudaSuccess) return cuda_fail(s, e, "rays host->static scratch");
   }
   const uint64_t warps = (n + 31) / 32;
-  const int grid = int(std::min<uint64_t>(uint64_t(d->grid), (warps * 32 + kTraceThreads - 1) / kTraceThreads));
+  const int blocks = blocks_for(warps);
   if (flags & LRT_TRACE_FAST_MATH)
-    e = lrt_fast::launch_trace(S, krays, khits, n, &slot->work, slot->counters, &slot->err, d->stackCap, grid,
+    e = lrt_fast::launch_trace(S, krays, khits, n, &slot->work, slot->counters, &slot->err, d->stackCap, blocks,
                                stream, false);
   else
-    e = lrt_exact::launch_trace(S, krays, khits, n, &slot->work, slot->counters, &slot->err, d->stackCap, grid,
+    e = lrt_exact::launch_trace(S, krays, khits, n, &slot->work, slot->counters, &slot->err, d->stackCap, blocks,
                                 stream, false);
   if (e != cudaSuccess) return cuda_fail(s, e, "trace launch");
   if (!onDevice) {

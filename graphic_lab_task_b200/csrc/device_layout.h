@@ -152,6 +152,13 @@ constexpr uint64_t kPrefetchMaxBytes = 48ull << 20;
 constexpr uint64_t kPrefetchMinRays = 4096;
 constexpr uint32_t kPrefetchChunk = 4096; // bytes per prefetch instruction
 
+// Geometry kinds a trace kernel is compiled for.  The leaf code of every kind
+// shares the traversal's registers, and what does not fit is spilled in every
+// loop, so a scene without bricks, and one of bricks only, have kernels of
+// their own.
+constexpr uint32_t kKindTriangles = 1, kKindNodes = 2; // triangles; frame-octree and SVS nodes
+constexpr uint32_t kKindBricks = 4, kKindNoBricks = kKindTriangles | kKindNodes, kKindAll = 7;
+
 struct DevScene {
   const lrt_bvh_node* tlas;
   const lrt_bvh_node_pair* pairs;
@@ -171,6 +178,8 @@ struct DevScene {
   const DevSbs* sbs;
   uint32_t flags;
   uint32_t voxelStepCap; // bounded SBS voxel march (kMaxVoxelSteps unless set)
+  uint32_t kind;         // kernel kind of the scene: kKindBricks, kKindNoBricks or kKindAll
+  uint32_t sms;          // the device's multiprocessors (persistent grids are multiples of it)
   // byte ranges streamed into L2 at the start of a trace launch (16-byte
   // aligned bases, sizes multiples of 16; 0 bytes: none)
   const char* pfPtr[kPrefetchRanges];

@@ -51,11 +51,7 @@ struct DeviceScene {
   std::vector<void*> allocs;
   DevScene S{};
   uint32_t stackCap = 0;
-  int grid = 0;
-  // every geometry is a sparse-brick set: image-order traces use the
-  // 80-register kernel and its grid
-  bool bricksOnly = false;
-  int gridBricks = 0;
+  int grid = 0; // blocks in one wave of the scene's trace kernel
   StreamSlot* slots = nullptr; // device, kMaxStreams
   std::map<cudaStream_t, int> slotOf;
   const lrt_bvh_node_pair* pairsOrig = nullptr; // unpruned node pairs (used once SBS values change)
@@ -133,6 +129,14 @@ struct DeviceScene {
       for (uint32_t* b : kv.second.buf) cudaFree(b);
   }
 };
+
+// Blocks that `warps` work items fill; the launchers bound them by one wave of
+// their kernel.
+inline int blocks_for(uint64_t warps)
+{
+  const uint64_t b = (warps * 32 + kTraceThreads - 1) / kTraceThreads;
+  return int(b < 1 ? 1 : b < 0x7FFFFFFFull ? b : 0x7FFFFFFFull);
+}
 
 // device.cu
 uint32_t preset_flags(const lrt_preset& p);

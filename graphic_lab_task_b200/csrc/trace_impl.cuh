@@ -6,7 +6,7 @@
 //
 // Structure follows the reference path function by function:
 //   trace_one        RayQuery_NearestHit        MultiRenderer/BVH2Common.cpp:3322-3392
-//   blas             BVH2TraverseF32            :3239-3320
+//   walk_*           its TLAS loop and BVH2TraverseF32 :3239-3320
 //   leaf             IntersectAllPrimitivesInLeaf :47-124
 //   triangles        IntersectAllTrianglesInLeaf  :1571-1635
 //   octree_node      OctreeNodeIntersect + RayNodeIntersection :727-749, 141-218
@@ -18,6 +18,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "device_layout.h"
 #include "lrt_math.h"
@@ -45,13 +46,50 @@ struct HitRecord {
                     // with the values (no dt/dtheta term)
 };
 
+// The nearest hit while a ray is being traversed: lrt_hit without the words
+// that are only written once the traversal has ended (finish_hit).  u, v are a
+// triangle hit's barycentrics ((1, 0) for a miss, (0, 0) for an SDF hit).
+struct Hit {
+  float t;
+  uint32_t primId, instId, geomId;
+  float u, v;
+};
+
+// Blocks per SM that the register allocation of a kernel is bounded for, by
+// the scene's geometry kind (device_layout.h) and what the launch waits for:
+// a frame of a few waves is as long as its slowest tiles' chains of dependent
+// steps and wants them free of spills, a launch of many waves wants warps.
+// Measured (us; 5 / 6 / 8 blocks of 128 threads = 96 / 80 / 64 registers):
+//   bricks: 512^3 model at 1920x1080 493 / 503 / -, fused render 382 / 402 / -,
+//     64 cameras (51 M rays) 13,319 / 12,546 / -, Lambert step 3,429 / 3,254 / -
+//   no bricks: 4096^2 instanced primary rays - / 5,737 / 5,573, sorted bounce
+//     - / 6,211 / 5,940, a 200k-triangle mesh at 256^2 - / 102 / 108, a voxel
+//     set at 1001x777 (ANALYTIC) - / 290 / 311
+//   all kinds: mixed scene at 1280x720 556 / 577 / 672 (7 blocks)
+constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
+constexpr int kManyWaves = 12;       // k_trace takes the kernel for many from here on
+constexpr int min_blocks(uint32_t kind, int size)
+{
+  return kind == kKindBricks ? (size == kMany ? 6 : 5) : kind == kKindNoBricks ? (size == kMany ? 8 : 6) : 5;
+}
+
+// f(std::integral_constant<uint32_t, kind>) for a scene's kernel kind.
+template <class F>
+auto with_kind(uint32_t kind, F f)
+{
+  if (kind == kKindBricks) return f(std::integral_constant<uint32_t, kKindBricks>());
+  if (kind == kKindNoBricks) return f(std::integral_constant<uint32_t, kKindNoBricks>());
+  return f(std::integral_constant<uint32_t, kKindAll>());
+}
+
 // Traversal context.  COUNT adds the work counters, RECORD the hit record,
 // SOLVERS the ANALYTIC / NEWTON / IT node solvers (ST and BBOX are always
 // there); the plain trace kernel instantiates none.  nrec points at this thread's
 // kNormalWords shared-memory words (thread-strided), where a sphere-traced
 // hit leaves what its normal is computed from once the traversal has ended.
-template <bool COUNT, bool RECORD = false, bool SOLVERS = false>
+template <bool COUNT, bool RECORD = false, bool SOLVERS = false, uint32_t KIND = kKindAll>
 struct Ctx {
+  static constexpr uint32_t kKind = KIND;
   static constexpr bool kCount = COUNT;
   static constexpr bool kRecord = RECORD;
   static constexpr bool kSolvers = SOLVERS;
@@ -240,10 +278,89 @@ __device__ __forceinline__ bool sdf_root_newton(const float* c, float qFar, floa
   return rtn >= 0 && rtn <= qFar && fabsf(f) < EPS;
 }
 
+// Whether a sphere trace from start_q (voxel units, values the voxel's
+// corners, start_dist > EPS its first distance) cannot end in a hit: the
+// field along the ray stays above EPS on [0, qFar].  On the ray the trilinear
+// field is a cubic whose Bernstein coefficients over [0, qFar] are the means
+// of its values at the corners of the box spanned by the ray's two ends with
+// 0, 1, 2 and 3 coordinates of the far end (the blossom of x*y*z terms), and
+// a cubic is nowhere below its smallest coefficient.  The margin covers the
+// rounding of these 36 operations and of the distances the trace itself
+// would compute: with both ends within half a voxel of the voxel the terms
+// are at most 8 vmax, each distance carries at most 20 roundings of them
+// (1e-5 vmax) and each position 2e-7 of a voxel per axis (3e-6 vmax).  A
+// trace past qFar is a miss whatever its distance, one stopped by its step
+// limit has a distance above EPS, and a NaN compares false (not rejected).
+// A grazing ray's traces are what a brick march spends most on (per 32 rays of
+// a 1920x1080 frame 32 tracing iterations with 2.6 lanes each, a third of the
+// instructions): 60 operations here save them all where the ray passes by.
+// With the march below going on to the next voxel in reach, so that lanes
+// trace together, and the brick kernels free of other leaf code: that frame
+// 550 -> 493 us, 64 cameras 13.85 -> 12.5 ms.
+__device__ __forceinline__ bool out_of_reach(const float* v, f3 q, f3 dir, float qFar, float sign, float start_dist)
+{
+  const f3 e = mk3(fmaf(qFar, dir.x, q.x), fmaf(qFar, dir.y, q.y), fmaf(qFar, dir.z, q.z));
+  float f[2][4]; // x at q, e; (y, z) corners
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float dx = v[k + 4] - v[k];
+    f[0][k] = fmaf(q.x, dx, v[k]);
+    f[1][k] = fmaf(e.x, dx, v[k]);
+  }
+  float g[2][2][2]; // x, y at q, e; z corners
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float dy = f[i][k + 2] - f[i][k];
+      g[i][0][k] = fmaf(q.y, dy, f[i][k]);
+      g[i][1][k] = fmaf(e.y, dy, f[i][k]);
+    }
+  float h[2][2][2]; // x, y, z at q, e
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float dz = g[i][k][1] - g[i][k][0];
+      h[i][k][0] = fmaf(q.z, dz, g[i][k][0]);
+      h[i][k][1] = fmaf(e.z, dz, g[i][k][0]);
+    }
+  const float b1 = sign * (h[1][0][0] + h[0][1][0] + h[0][0][1]);
+  const float b2 = sign * (h[1][1][0] + h[1][0][1] + h[0][1][1]);
+  const float b3 = sign * h[1][1][1];
+  const float vmax = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))),
+                           fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
+  const float out = fmaxf(fmaxf(fmaxf(fabsf(q.x - 0.5f), fabsf(q.y - 0.5f)), fmaxf(fabsf(q.z - 0.5f), fabsf(e.x - 0.5f))),
+                          fmaxf(fabsf(e.y - 0.5f), fabsf(e.z - 0.5f)));
+  const float m = fmaf(4e-5f, vmax, 1e-6f);
+  return out <= 1.0f && start_dist > m && b1 > 3.0f * m && b2 > 3.0f * m && b3 > m;
+}
+
+// The first distance of LocalSurfaceIntersection's march (BVH2Common.cpp:
+// 364-372) at the voxel's entry, and whether the rest of it can hit.
+template <bool REACH, class CTX>
+__device__ __forceinline__ bool surface_start(CTX& c, f3 ray_dir, const float* values, float qNear, float qFar,
+                                              f3 start_q, float& start_sign, float& start_dist)
+{
+  const DevScene& S = c.S;
+  const float EPS = 1e-6f;
+  start_sign = 1;
+  start_dist = trilinear(values, start_q + qNear * ray_dir);
+  c.inc(kCntStSteps);
+  if (S.flags & kFlagSurfaceMode) start_sign = ssign(start_dist);
+  start_dist *= start_sign;
+  if (start_dist <= EPS || (S.flags & kFlagBBoxMode)) return true;
+  const uint32_t solver = CTX::kSolvers ? (S.flags >> kFlagSolverShift) & 7u : kSolverST;
+  // the counting kernels trace every voxel, so that their step counts are the reference's
+  if (REACH && !CTX::kCount && (solver == kSolverST || solver == kSolverIT))
+    return !out_of_reach(values, start_q, ray_dir, qFar, start_sign, start_dist);
+  return true;
+}
+
 template <class CTX>
-__device__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId, uint32_t geomId,
+__device__ __forceinline__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId, uint32_t geomId,
                               const float* values, uint32_t primId, float d, float qNear, float qFar, f2 fNearFar,
-                              f3 start_q, lrt_hit& hit)
+                              f3 start_q, float start_sign, float start_dist, Hit& hit)
 {
   const DevScene& S = c.S;
   const float EPS = 1e-6f;
@@ -251,11 +368,6 @@ __device__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId
   float t = qNear;
   bool early_hit = false, hitf = false;
   unsigned iter = 0;
-  float start_sign = 1;
-  float start_dist = trilinear(values, start_q + t * ray_dir);
-  c.inc(kCntStSteps);
-  if (S.flags & kFlagSurfaceMode) start_sign = ssign(start_dist);
-  start_dist *= start_sign;
   const uint32_t solver = CTX::kSolvers ? (S.flags >> kFlagSolverShift) & 7u : kSolverST;
   if (start_dist <= EPS || (S.flags & kFlagBBoxMode)) {
     early_hit = true;
@@ -301,10 +413,9 @@ __device__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId
   }
   const float tReal = fNearFar.x + d * t;
   if (t <= qFar && hitf && tReal < hit.t) {
-    // The normal is evaluated once the traversal has ended (trace_one), from
+    // The normal is evaluated once the traversal has ended (finish_hit), from
     // what it depends on, kept here: lanes whose hits are found in different
     // iterations of the surrounding loops then compute their normals together.
-    f2 en = encode_normal(mk3(0, 0, 1));
     if (S.flags & kFlagNeedNormal) {
       const uint32_t st = blockDim.x;
       // the sample point: start_q itself for the BBOX mode's early hits
@@ -315,7 +426,6 @@ __device__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId
       c.nrec[3 * st] = q.z;
 #pragma unroll
       for (int i = 0; i < 8; i++) c.nrec[(4 + i) * st] = values[i];
-      en = mk2(0.0f, 0.0f);
       c.inc(kCntNormals);
     }
     if (CTX::kRecord) {
@@ -332,16 +442,14 @@ __device__ void local_surface(CTX& c, uint32_t type, f3 ray_dir, uint32_t instId
     hit.primId = (S.flags & kFlagStIterations) ? iter : primId;
     hit.instId = instId;
     hit.geomId = geomId | (type << 24);
-    hit.coords[0] = 0;
-    hit.coords[1] = 0;
-    hit.coords[2] = en.x;
-    hit.coords[3] = en.y;
+    hit.u = 0;
+    hit.v = 0;
   }
 }
 
 template <class CTX>
 __device__ void octree_node(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3 inv_dir, float tNear,
-                            uint32_t instId, uint32_t geomId, uint32_t bvhNodeId, lrt_hit& hit)
+                            uint32_t instId, uint32_t geomId, uint32_t bvhNodeId, Hit& hit)
 {
   const DevScene& S = c.S;
   float values[8];
@@ -382,7 +490,10 @@ __device__ void octree_node(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3
   const float qFar = (fNearFar.y - fNearFar.x) / d;
   const float qNear = tNear > fNearFar.x ? (tNear - fNearFar.x) / d : 0.0f;
   if (qNear > 0.0f) return; // ray starts inside this node (BVH2Common.cpp:744-745)
-  local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, qNear, qFar, fNearFar, start_q, hit);
+  float start_sign, start_dist;
+  if (surface_start<false>(c, ray_dir, values, qNear, qFar, start_q, start_sign, start_dist))
+    local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, qNear, qFar, fNearFar, start_q, start_sign,
+                  start_dist, hit);
 }
 
 // FAST: the ray's origin, direction and inverse are finite, so the brick
@@ -393,7 +504,7 @@ __device__ void octree_node(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3
 // do not depend on the sign of a zero, so every hit is unchanged.
 template <bool FAST, class CTX>
 __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3 inv_dir, float tNear,
-                             uint32_t instId, uint32_t geomId, uint32_t bvhNodeId, lrt_hit& hit)
+                             uint32_t instId, uint32_t geomId, uint32_t bvhNodeId, Hit& hit)
 {
   const DevScene& S = c.S;
   const DevSbs& sb = S.sbs[g.sdfId];
@@ -422,44 +533,59 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
   const float* dense = S.sbsDense + sb.denseBase + uint64_t(primId) * sb.denseStride;
   float values[8];
   uint32_t steps = 0;
+  // The march goes on to the next voxel whose sphere trace may hit, in which
+  // the warp's lanes then trace together.
   while (bnf.x < bnf.y && hit.t == old_t) {
-    if (steps++ >= S.voxelStepCap) {
-      c.err |= kErrVoxelCap;
-      break;
-    }
-    c.inc(kCntVoxels);
-    const f3 hit_pos = ray_pos + bnf.x * ray_dir;
-    const f3 local_pos = (hit_pos - brick_min_pos) * scale;
-    const f3 voxelPos = mk3(floorf(sclamp_pos(local_pos.x, 1e-6f, hiClamp)),
-                            floorf(sclamp_pos(local_pos.y, 1e-6f, hiClamp)),
-                            floorf(sclamp_pos(local_pos.z, 1e-6f, hiClamp)));
-    const f3 min_pos = brick_min_pos + d * voxelPos;
-    const f3 max_pos = min_pos + d * mk3(1, 1, 1);
-    const uint32_t vx = uint32_t(voxelPos.x), vy = uint32_t(voxelPos.y), vz = uint32_t(voxelPos.z);
-    const uint32_t vid = (vx * bs + vy) * bs + vz;
-    // surface bit == (min of the 8 corner values <= 0), precomputed
-    const bool surface = (__ldg(mask + 1 + (vid >> 5)) >> (vid & 31)) & 1u;
-    // the voxel's exit always (for the advance), its entry only where a
-    // sphere trace may start
-    const Slabs vsl = slabs(ray_pos, inv_dir, min_pos, max_pos);
-    const float vfar = slab_far<FAST>(vsl);
-    if (surface && tNear < slab_near<FAST>(vsl)) {
-      const f2 fNearFar = mk2(slab_near<FAST>(vsl), vfar);
-      c.inc(kCntVoxelLoads);
-      // 8 corners of the voxel from the dense (bs+1)^3 grid, x-major
-      const float* base = dense + (vx * V1 + vy) * V1 + vz;
-      values[0] = __ldg(base);
-      values[1] = __ldg(base + 1);
-      values[2] = __ldg(base + V1);
-      values[3] = __ldg(base + V1 + 1);
-      values[4] = __ldg(base + V1 * V1);
-      values[5] = __ldg(base + V1 * V1 + 1);
-      values[6] = __ldg(base + V1 * V1 + V1);
-      values[7] = __ldg(base + V1 * V1 + V1 + 1);
-      const f3 start_pos = ray_pos + fNearFar.x * ray_dir;
-      const f3 start_q = (start_pos - min_pos) * scale;
-      const float qFar = (fNearFar.y - fNearFar.x) * scale;
-      local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, 0.0f, qFar, fNearFar, start_q, hit);
+    bool found = false;
+    f3 start_q = mk3(0, 0, 0);
+    f2 fNearFar = mk2(0, 0);
+    float qFar = 0, start_sign = 1, start_dist = 0;
+    uint32_t vx = 0, vy = 0, vz = 0;
+    do {
+      if (steps++ >= S.voxelStepCap) {
+        c.err |= kErrVoxelCap;
+        bnf.x = bnf.y; // ends the march
+        break;
+      }
+      c.inc(kCntVoxels);
+      const f3 hit_pos = ray_pos + bnf.x * ray_dir;
+      const f3 local_pos = (hit_pos - brick_min_pos) * scale;
+      const f3 voxelPos = mk3(floorf(sclamp_pos(local_pos.x, 1e-6f, hiClamp)),
+                              floorf(sclamp_pos(local_pos.y, 1e-6f, hiClamp)),
+                              floorf(sclamp_pos(local_pos.z, 1e-6f, hiClamp)));
+      const f3 min_pos = brick_min_pos + d * voxelPos;
+      const f3 max_pos = min_pos + d * mk3(1, 1, 1);
+      vx = uint32_t(voxelPos.x), vy = uint32_t(voxelPos.y), vz = uint32_t(voxelPos.z);
+      const uint32_t vid = (vx * bs + vy) * bs + vz;
+      // surface bit == (min of the 8 corner values <= 0), precomputed
+      const bool surface = (__ldg(mask + 1 + (vid >> 5)) >> (vid & 31)) & 1u;
+      // the voxel's exit always (for the advance), its entry only where a
+      // sphere trace may start
+      const Slabs vsl = slabs(ray_pos, inv_dir, min_pos, max_pos);
+      const float vfar = slab_far<FAST>(vsl);
+      if (surface && tNear < slab_near<FAST>(vsl)) {
+        fNearFar = mk2(slab_near<FAST>(vsl), vfar);
+        c.inc(kCntVoxelLoads);
+        // 8 corners of the voxel from the dense (bs+1)^3 grid, x-major
+        const float* base = dense + (vx * V1 + vy) * V1 + vz;
+        values[0] = __ldg(base);
+        values[1] = __ldg(base + 1);
+        values[2] = __ldg(base + V1);
+        values[3] = __ldg(base + V1 + 1);
+        values[4] = __ldg(base + V1 * V1);
+        values[5] = __ldg(base + V1 * V1 + 1);
+        values[6] = __ldg(base + V1 * V1 + V1);
+        values[7] = __ldg(base + V1 * V1 + V1 + 1);
+        const f3 start_pos = ray_pos + fNearFar.x * ray_dir;
+        start_q = (start_pos - min_pos) * scale;
+        qFar = (fNearFar.y - fNearFar.x) * scale;
+        found = surface_start<CTX::kKind == kKindBricks>(c, ray_dir, values, 0.0f, qFar, start_q, start_sign, start_dist);
+      }
+      bnf.x += smax(0.0f, vfar - bnf.x) + 1e-6f;
+    } while (CTX::kKind == kKindBricks && !found && bnf.x < bnf.y);
+    if (found) {
+      local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, 0.0f, qFar, fNearFar, start_q, start_sign,
+                    start_dist, hit);
       if (CTX::kRecord && hit.t < old_t && sb.colorLayout) {
         // indices of the 8 corner values in the float array (indexed layouts)
         const uint32_t V = sb.vsize, P = sb.pad;
@@ -471,11 +597,10 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
         c.rec.sbs = true;
       }
     }
-    bnf.x += smax(0.0f, vfar - bnf.x) + 1e-6f;
   }
   if (hit.t < old_t && sb.colorLayout) {
     // The colour of the hit (indexed layouts) is evaluated once the traversal
-    // has ended (trace_one, sbs_hit_colour) from the hit point and the brick,
+    // has ended (finish_hit, sbs_hit_colour) from the hit point and the brick,
     // kept here, so that lanes whose hits come in different iterations of the
     // traversal compute their colours together.
     const f3 pos = ray_pos + hit.t * ray_dir;
@@ -525,7 +650,7 @@ __device__ __forceinline__ void sbs_hit_colour(CTX& c, const DevSbs& sb, lrt_hit
 
 template <class CTX>
 __device__ void triangles(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, float tNear, uint32_t instId,
-                          uint32_t geomId, uint32_t a_start, uint32_t a_count, lrt_hit& hit)
+                          uint32_t geomId, uint32_t a_start, uint32_t a_count, Hit& hit)
 {
   const DevScene& S = c.S;
   const float4* tri = S.triSoup + 3 * (uint64_t(g.triBase) + a_start);
@@ -545,12 +670,10 @@ __device__ void triangles(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, floa
       hit.primId = a_start + i;
       hit.instId = instId;
       hit.geomId = geomId | (LRT_TYPE_MESH_TRIANGLE << 24);
-      hit.coords[0] = u;
-      hit.coords[1] = v;
       // the geometric normal is computed once the traversal has ended
-      // (trace_one, triangle_normal), from the triangle the hit names
-      hit.coords[2] = 0;
-      hit.coords[3] = 0;
+      // (finish_hit, triangle_normal), from the triangle the hit names
+      hit.u = u;
+      hit.v = v;
     }
   }
 }
@@ -571,23 +694,22 @@ __device__ __forceinline__ f2 triangle_normal(const DevScene& S, const DevGeom& 
 template <class CTX>
 __device__ __forceinline__ uint32_t leaf(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3 inv, bool fast,
                                          float tNear, uint32_t aabbId, uint32_t instId, uint32_t geomId,
-                                         lrt_hit& hit)
+                                         Hit& hit)
 {
   const float tPrev = hit.t;
   c.inc(kCntLeafCalls);
   const uint32_t packed = __ldg(c.S.primIdCount + g.aabbBase + aabbId);
   const uint32_t a_start = packed & 0x0FFFFFFFu;
   const uint32_t a_count = (packed & 0x70000000u) >> 28;
-  switch (g.tag) {
-    case LRT_TAG_TRIANGLE: triangles(c, g, ray_pos, ray_dir, tNear, instId, geomId, a_start, a_count, hit); break;
-    case LRT_TAG_SDF_NODE: octree_node(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit); break;
-    case LRT_TAG_SDF_BRICK:
-      if (fast)
-        octree_brick<true>(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit);
-      else
-        octree_brick<false>(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit);
-      break;
-    default: break;
+  if ((CTX::kKind & kKindTriangles) && g.tag == LRT_TAG_TRIANGLE) {
+    triangles(c, g, ray_pos, ray_dir, tNear, instId, geomId, a_start, a_count, hit);
+  } else if ((CTX::kKind & kKindNodes) && g.tag == LRT_TAG_SDF_NODE) {
+    octree_node(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit);
+  } else if ((CTX::kKind & kKindBricks) && g.tag == LRT_TAG_SDF_BRICK) {
+    if (fast)
+      octree_brick<true>(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit);
+    else
+      octree_brick<false>(c, g, ray_pos, ray_dir, inv, tNear, instId, geomId, a_start, hit);
   }
   return (hit.t >= tPrev) ? LRT_TAG_NONE : g.tag;
 }
@@ -643,37 +765,6 @@ __device__ __forceinline__ bool blas_descend(CTX& c, const float4* pairs, uint32
   return true;
 }
 
-// BVH2TraverseF32 with the stack in shared memory (thread-strided).
-template <class CTX>
-__device__ void blas(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap, f3 ray_pos, f3 ray_dir,
-                     float tNear, uint32_t instId, uint32_t geomId, bool stopOnFirstHit, lrt_hit& hit)
-{
-  const DevScene& S = c.S;
-  const DevGeom g = S.geoms[geomId];
-  const float4* pairs = reinterpret_cast<const float4*>(S.pairs + g.bvhOffset);
-  int top = 0;
-  uint32_t leftNodeOffset = 0;
-  bool hitFound = false;
-  stack[0] = 0;
-  const f3 inv = safe_inverse(ray_dir);
-  const bool fast = fast_nodes(S, ray_pos, ray_dir, inv);
-  while (top >= 0 && !hitFound) {
-    const bool ok = fast ? blas_descend<true>(c, pairs, stack, stride, cap, ray_pos, inv, tNear, hit.t, top,
-                                              leftNodeOffset)
-                         : blas_descend<false>(c, pairs, stack, stride, cap, ray_pos, inv, tNear, hit.t, top,
-                                               leftNodeOffset);
-    if (!ok) return;
-    if (top >= 0 && leftNodeOffset != 0xFFFFFFFFu) {
-      const float tNearSdf = smax(tNear, 0.01f); // SDF_BIAS (BVH2Common.cpp:3306-3307)
-      const uint32_t tag =
-          leaf(c, g, ray_pos, ray_dir, inv, fast, tNearSdf, leftNodeOffset & 0x0FFFFFFFu, instId, geomId, hit);
-      hitFound = (tag != 0) && (tag != LRT_TAG_TRIANGLE || stopOnFirstHit);
-    }
-    top--;
-    leftNodeOffset = stack[(top > 0 ? top : 0) * stride];
-  }
-}
-
 // The stackless TLAS walk of RayQuery_NearestHit (BVH2Common.cpp:3346-3358)
 // up to the next intersected leaf or the end of the escape chain.
 template <bool FAST, class CTX>
@@ -694,49 +785,122 @@ __device__ __forceinline__ void tlas_walk(CTX& c, f3 pos, f3 inv, float tmin, fl
   } while (travFlags != (kLeafBit | 1u) && nodeIdx != 0 && nodeIdx < 0xFFFFFFFEu);
 }
 
-// RayQuery_NearestHit for one ray.
+// RayQuery_NearestHit of one ray in phases (trace_one):
+//   walk_begin    the ray
+//   walk_tlas     the TLAS loop up to the next instance (or the ray's end)
+//   walk_descend  BVH2TraverseF32's descent to the next BLAS leaf
+//   walk_leaf     that leaf, and the pop after it
+// The order of node, leaf and instance visits is that of the reference's
+// nested loops, so every comparison and every hit is the same.
+struct Walk {
+  f3 pos, dir;       // the ray
+  float tmin;
+  f3 rp, rd, inv;    // the ray in the current instance's space, inv = SafeInverse(rd)
+  Hit hit;
+  uint32_t nodeIdx;  // next TLAS node
+  uint32_t instId, geomId;
+  uint32_t cur;      // BLAS: next node word
+  int top;           // BLAS: stack entries, negative when it has ended
+  bool stopOnFirst, fast; // fast: the instance-space ray takes the one-instruction box tests
+};
+// What the ray does next.
+constexpr uint32_t kRayDone = 1, kRayTlas = 2, kRayBlas = 3;
+
+__device__ __forceinline__ void walk_begin(Walk& w, float4 pn, float4 df)
+{
+  float dirW = df.w;
+  w.stopOnFirst = (dirW <= 0.0f);
+  if (w.stopOnFirst) dirW *= -1.0f;
+  w.pos = mk3(pn.x, pn.y, pn.z);
+  w.dir = mk3(df.x, df.y, df.z);
+  w.tmin = pn.w;
+  w.hit.t = dirW;
+  w.hit.primId = 0xFFFFFFFFu;
+  w.hit.instId = 0xFFFFFFFFu;
+  w.hit.geomId = 0xFFFFFFFFu;
+  w.hit.u = 1.0f;
+  w.hit.v = 0.0f;
+  w.nodeIdx = 0;
+}
+
+// The TLAS loop of RayQuery_NearestHit (BVH2Common.cpp:3346-3375) up to the
+// next instance, whose BLAS it enters; kRayDone if the ray has ended.
 template <class CTX>
-__device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap, float4 pn, float4 df,
-                          lrt_hit& hit)
+__device__ __forceinline__ uint32_t walk_tlas(CTX& c, Walk& w, uint32_t* stack)
 {
   const DevScene& S = c.S;
-  float dirW = df.w;
-  const bool stopOnFirstHit = (dirW <= 0.0f);
-  if (stopOnFirstHit) dirW *= -1.0f;
-  const f3 pos = mk3(pn.x, pn.y, pn.z), dir = mk3(df.x, df.y, df.z);
-  const float tmin = pn.w;
-  const f3 inv = safe_inverse(dir);
-  hit.t = dirW;
-  hit.primId = 0xFFFFFFFFu;
-  hit.instId = 0xFFFFFFFFu;
-  hit.geomId = 0xFFFFFFFFu;
-  hit.coords[0] = 1.0f;
-  hit.coords[1] = 0.0f;
+  const f3 inv = safe_inverse(w.dir);
+  const bool fast = fast_nodes(S, w.pos, w.dir, inv);
+  uint32_t travFlags = 0, leftOffset = 0;
+  if (fast)
+    tlas_walk<true>(c, w.pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
+  else
+    tlas_walk<false>(c, w.pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
+  // without a leaf the walk has reached the end of the escape chain
+  if (travFlags != (kLeafBit | 1u)) return kRayDone;
+  w.instId = leftOffset & 0x0FFFFFFFu;
+  const DevInstance& I = S.instances[w.instId];
+  c.inc(kCntInstances);
+  w.geomId = I.geomId;
+  w.rp = matmul4(I.transformInv, w.pos, 1.0f);
+  w.rd = matmul4(I.transformInv, w.dir, 0.0f);
+  w.inv = safe_inverse(w.rd);
+  w.fast = fast_nodes(S, w.rp, w.rd, w.inv);
+  w.top = 0;
+  w.cur = 0;
+  stack[0] = 0;
+  return kRayBlas;
+}
+
+template <class CTX>
+__device__ __forceinline__ void walk_descend(CTX& c, Walk& w, uint32_t* stack, uint32_t stride, uint32_t cap)
+{
+  const float4* pairs = reinterpret_cast<const float4*>(c.S.pairs + c.S.geoms[w.geomId].bvhOffset);
+  const bool ok =
+      w.fast ? blas_descend<true>(c, pairs, stack, stride, cap, w.rp, w.inv, w.tmin, w.hit.t, w.top, w.cur)
+             : blas_descend<false>(c, pairs, stack, stride, cap, w.rp, w.inv, w.tmin, w.hit.t, w.top, w.cur);
+  if (!ok) w.top = -1; // overflow (c.err): the BLAS and then the ray end
+}
+
+// The leaf the descent stopped at (if any) and the next stack entry; returns
+// the ray's next state: kRayBlas while the BLAS goes on, then kRayTlas
+// or, at the end of the TLAS, kRayDone.
+template <class CTX>
+__device__ __forceinline__ uint32_t walk_leaf(CTX& c, Walk& w, uint32_t* stack, uint32_t stride)
+{
+  bool ended = false;
+  if (w.top >= 0 && w.cur != 0xFFFFFFFFu) {
+    const DevGeom g = c.S.geoms[w.geomId];
+    const float tNearSdf = smax(w.tmin, 0.01f); // SDF_BIAS (BVH2Common.cpp:3306-3307)
+    const uint32_t tag =
+        leaf(c, g, w.rp, w.rd, w.inv, w.fast, tNearSdf, w.cur & 0x0FFFFFFFu, w.instId, w.geomId, w.hit);
+    ended = (tag != 0) && (tag != LRT_TAG_TRIANGLE || w.stopOnFirst);
+  }
+  w.top--;
+  w.cur = stack[(w.top > 0 ? w.top : 0) * stride];
+  if (w.top >= 0 && !ended) return kRayBlas;
+  const bool more = w.nodeIdx < 0xFFFFFFFEu && !(w.stopOnFirst && w.hit.primId != 0xFFFFFFFFu) &&
+                    !(c.err & kErrStackOverflow);
+  return more ? kRayTlas : kRayDone;
+}
+
+// What the leaf tests left for the end of the traversal: the final hit's
+// normal, an SBS hit's colour and the triangle primId remap.
+template <class CTX>
+__device__ __forceinline__ void finish_hit(CTX& c, const Hit& w, lrt_hit& hit)
+{
+  const DevScene& S = c.S;
+  hit.t = w.t;
+  hit.primId = w.primId;
+  hit.instId = w.instId;
+  hit.geomId = w.geomId;
+  hit.coords[0] = w.u;
+  hit.coords[1] = w.v;
   hit.coords[2] = 0.0f;
   hit.coords[3] = 0.0f;
-  uint32_t nodeIdx = 0;
-  const bool fast = fast_nodes(S, pos, dir, inv);
-  do {
-    uint32_t travFlags = 0, leftOffset = 0;
-    if (fast)
-      tlas_walk<true>(c, pos, inv, tmin, hit.t, nodeIdx, travFlags, leftOffset);
-    else
-      tlas_walk<false>(c, pos, inv, tmin, hit.t, nodeIdx, travFlags, leftOffset);
-    if (travFlags == (kLeafBit | 1u)) {
-      const uint32_t instId = leftOffset & 0x0FFFFFFFu;
-      const DevInstance& I = S.instances[instId];
-      c.inc(kCntInstances);
-      const f3 rp = matmul4(I.transformInv, pos, 1.0f);
-      const f3 rd = matmul4(I.transformInv, dir, 0.0f);
-      blas(c, stack, stride, cap, rp, rd, tmin, instId, I.geomId, stopOnFirstHit, hit);
-      if (c.err & kErrStackOverflow) break;
-    }
-  } while (nodeIdx < 0xFFFFFFFEu && !(stopOnFirstHit && hit.primId != 0xFFFFFFFFu));
-  // What the leaf tests left for the end of the traversal: the final hit's
-  // normal, an SBS hit's colour and the triangle primId remap.
   if (hit.geomId < 0xFFFFFFFFu) {
     const DevGeom& g = S.geoms[hit.geomId & 0x00FFFFFFu];
-    if ((hit.geomId >> 24) == LRT_TYPE_MESH_TRIANGLE) {
+    if ((CTX::kKind & kKindTriangles) && (hit.geomId >> 24) == LRT_TYPE_MESH_TRIANGLE) {
       if (S.flags & kFlagNeedNormal) {
         const f2 en = triangle_normal(S, g, hit.primId, hit.instId);
         hit.coords[2] = en.x;
@@ -750,13 +914,31 @@ __device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap
         hit.coords[2] = en.x;
         hit.coords[3] = en.y;
       }
-      if (g.tag == LRT_TAG_SDF_BRICK) {
+      if ((CTX::kKind & kKindBricks) && g.tag == LRT_TAG_SDF_BRICK) {
         const DevSbs& sb = S.sbs[g.sdfId];
         if (sb.colorLayout) sbs_hit_colour(c, sb, hit);
       }
     }
   }
   if (hit.primId != 0xFFFFFFFFu) c.inc(kCntHits);
+}
+
+// RayQuery_NearestHit for one ray.
+template <class CTX>
+__device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap, float4 pn, float4 df,
+                          lrt_hit& hit)
+{
+  Walk w;
+  walk_begin(w, pn, df);
+  while (walk_tlas(c, w, stack) == kRayBlas) {
+    uint32_t next;
+    do {
+      walk_descend(c, w, stack, stride, cap);
+      next = walk_leaf(c, w, stack, stride);
+    } while (next == kRayBlas);
+    if (next == kRayDone) break;
+  }
+  finish_hit(c, w.hit, hit);
 }
 
 // Longest-first order of the tiles of an image-order launch.  Each launch
@@ -910,13 +1092,9 @@ __device__ __forceinline__ void l2_prefetch_scene(const DevScene& S)
 }
 
 //
-// MINB: blocks per SM the register allocation is bounded for (7: 72
-// registers; 6: 80 registers, used for the image-order launches of scenes
-// whose geometries are all sparse-brick sets, where the brick march and the
-// sphere trace spill at 72, and for row-order launches smaller than one wave,
-// which wait on their slowest warp's chain of dependent steps).
-template <bool COUNT, bool SOLVERS, bool IMG, int MINB = 7>
-__global__ void __launch_bounds__(kTraceThreads, MINB) k_trace(DevScene S, const float4* __restrict__ rays,
+// KIND, SIZE: see min_blocks.
+template <bool COUNT, bool SOLVERS, bool IMG, uint32_t KIND, int SIZE>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_trace(DevScene S, const float4* __restrict__ rays,
                                                          lrt_hit* __restrict__ hits, uint64_t n,
                                                          unsigned long long* __restrict__ work_counter,
                                                          unsigned long long* __restrict__ counters,
@@ -928,7 +1106,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace(DevScene S, const
   extern __shared__ uint32_t smem_stack[];
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<COUNT, false, SOLVERS> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<COUNT, false, SOLVERS, KIND> c(S, normal_words(smem_stack, stack_cap));
   __shared__ WarpClock wclock[IMG ? kTraceThreads / 32 : 1];
   const uint64_t tilesX = (uint64_t(img_w) + kImgTileW - 1) / kImgTileW;
   if (IMG && lane == 0) {
@@ -1416,8 +1594,8 @@ __device__ float4 resolve_mode_colour(CTX& c, const DevLights& L, const DevMater
 //
 // RENDER: instead of hits, each pixel's RGBA8 colour (resolve_rgba8: the
 // LAMBERT_NO_TEX resolve with L and the tonemap) goes to image[rayOffset + y*width + x].
-template <bool RENDER>
-__global__ void __launch_bounds__(kTraceThreads, 7) k_trace_cameras(DevScene S, const DevBatchCamera* __restrict__ cams,
+template <bool RENDER, uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_trace_cameras(DevScene S, const DevBatchCamera* __restrict__ cams,
                                                                  uint32_t ncams, uint32_t ntiles, DevBatchShape shape,
                                                                  lrt_hit* __restrict__ hits,
                                                                  unsigned long long* __restrict__ work_counter,
@@ -1428,7 +1606,7 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_cameras(DevScene S, 
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false> c(S, normal_words(smem_stack, shape.stackCap));
+  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, shape.stackCap));
   for (;;) {
     unsigned long long tile = 0;
     if (lane == 0) tile = atomicAdd(work_counter, 1ull);
@@ -1469,30 +1647,35 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_cameras(DevScene S, 
 
 cudaError_t launch_trace_cameras(const DevScene& S, const DevBatchCamera* cams, uint32_t ncams, uint32_t ntiles,
                                  const DevBatchShape& shape, lrt_hit* hits, unsigned long long* work_counter,
-                                 uint32_t* err_word, int grid, cudaStream_t stream, const DevLights* lights,
+                                 uint32_t* err_word, int blocks, cudaStream_t stream, const DevLights* lights,
                                  uint32_t* image)
 {
   const size_t smem = trace_smem_bytes(shape.stackCap);
-  if (image) {
-    cudaError_t e = cudaFuncSetAttribute(k_trace_cameras<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
-    if (e != cudaSuccess) return e;
-    k_trace_cameras<true><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
-                                                                 err_word, *lights, image);
-  } else {
-    k_trace_cameras<false><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
-                                                                  err_word, DevLights{}, nullptr);
-  }
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
+    if (image) {
+      cudaError_t e = cudaFuncSetAttribute(k_trace_cameras<true, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           int(trace_smem_bytes(kMaxStackDev + 1)));
+      if (e != cudaSuccess) return e;
+      k_trace_cameras<true, K><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
+                                                                   err_word, *lights, image);
+    } else {
+      k_trace_cameras<false, K><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
+                                                                    err_word, DevLights{}, nullptr);
+    }
+    return cudaGetLastError();
+  });
 }
 
-cudaError_t cameras_occupancy(uint32_t stack_cap, int* blocks_per_sm)
+// The shared-memory limit of the batched trace (set once per batch, not per
+// launch: a captured launch must not set attributes).
+cudaError_t set_cameras_smem(uint32_t kind)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
-  cudaError_t e = cudaFuncSetAttribute(k_trace_cameras<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_trace_cameras<false>, kTraceThreads, smem);
+  return with_kind(kind, [&](auto k) {
+    return cudaFuncSetAttribute(k_trace_cameras<false, decltype(k)::value>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(trace_smem_bytes(kMaxStackDev + 1)));
+  });
 }
 
 // Lambert shading of a hit, MultiRenderer::ResolveCommon for
@@ -1516,10 +1699,8 @@ __device__ __forceinline__ float lambert(const lrt_hit& h, f3 dir, f3 L)
 // triangle and turned towards the viewer as in loadNormalTcFromGbuffer :27-75,
 // SDF normals decoded from the hit) and Tonemap (:536-542) into RGBA8.  A warp
 // takes 8x4-pixel tiles from a global counter.
-// MINB as for k_trace: 6 (80 registers) for one LAMBERT_NO_TEX sample of a
-// scene whose geometries are all sparse-brick sets, else 7 (72 registers).
-template <bool MODES, int MINB = 7>
-__global__ void __launch_bounds__(kTraceThreads, MINB) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
+template <bool MODES, uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
                                                                 uint32_t* __restrict__ image,
                                                                 unsigned long long* __restrict__ work_counter,
                                                                 uint32_t* __restrict__ err_word, uint32_t stack_cap,
@@ -1530,7 +1711,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_render_rgba8(DevScene S
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1601,7 +1782,8 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_render_rgba8(DevScene S
 // does (the OUTLINE_PRIM colour), or the background for a miss.  The colour
 // is resolved here, with the trace's context, because a triangle's normal
 // needs the triangle record the traversal found.
-__global__ void __launch_bounds__(kTraceThreads, 7) k_outline_fill(DevScene S, DevCamera cam, DevLights L,
+template <uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_outline_fill(DevScene S, DevCamera cam, DevLights L,
                                                                 DevMaterials M, DevRenderModes RM, uint32_t smp,
                                                                 float2* __restrict__ tm, float4* __restrict__ col,
                                                                 unsigned long long* __restrict__ work_counter,
@@ -1613,7 +1795,7 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_outline_fill(DevScene S, D
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1688,7 +1870,8 @@ __global__ void __launch_bounds__(256) k_outline_resolve(const float2* __restric
 
 // kernel1D_FillGbufferWithTransparency (MultiRenderer.cpp:204-221) for one
 // sample: anyhit_loop per pixel of the camera (8x4-pixel tiles per warp).
-__global__ void __launch_bounds__(kTraceThreads, 7) k_fill_gbuffer_transparency(
+template <uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_fill_gbuffer_transparency(
     DevScene S, DevCamera cam, DevMaterials M, float4* __restrict__ transparency, lrt_hit* __restrict__ gbuffer,
     unsigned long long* __restrict__ work_counter, uint32_t* __restrict__ err_word, uint32_t stack_cap,
     const uint32_t* __restrict__ sched_rd, uint32_t* sched_wr)
@@ -1697,7 +1880,7 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_fill_gbuffer_transparency(
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1766,8 +1949,8 @@ __device__ __forceinline__ bool next_ray(uint64_t n, uint32_t img_w, uint32_t im
 }
 
 // Forward render: image[i] = Lambert shade of ray i's nearest hit.
-template <bool IMG>
-__global__ void __launch_bounds__(kTraceThreads, 7) k_render_lambert(DevScene S, const float4* __restrict__ rays,
+template <bool IMG, uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_render_lambert(DevScene S, const float4* __restrict__ rays,
                                                                   uint64_t n, float3 light, float* __restrict__ image,
                                                                   unsigned long long* __restrict__ work_counter,
                                                                   uint32_t* __restrict__ err_word, uint32_t stack_cap,
@@ -1786,7 +1969,7 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_render_lambert(DevScene S,
     wc->longest = 0;
     wc->busy = 0;
   }
-  Ctx<false> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
   const f3 L = mk3(light.x, light.y, light.z);
   uint64_t i = 0;
   bool valid = false;
@@ -1811,8 +1994,8 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_render_lambert(DevScene S,
 // and dLoss/dI * dI/dtheta_i is added to grad[idx_i] for the 8 corners.
 // Rays whose dLoss/dI is 0 are skipped.  Hits off indexed SBS bricks
 // contribute nothing.
-template <bool IMG>
-__global__ void __launch_bounds__(kTraceThreads, 7) k_adjoint_lambert(DevScene S, const float4* __restrict__ rays,
+template <bool IMG, uint32_t KIND>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjoint_lambert(DevScene S, const float4* __restrict__ rays,
                                                                    uint64_t n, float3 light,
                                                                    const float* __restrict__ dimage,
                                                                    float* __restrict__ grad,
@@ -1841,7 +2024,7 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_adjoint_lambert(DevScene S
     if (!valid) continue;
     const float dLdI = __ldg(dimage + i);
     if (dLdI == 0.0f) continue;
-    Ctx<false, true> c(S, normal_words(smem_stack, stack_cap));
+    Ctx<false, true, false, KIND> c(S, normal_words(smem_stack, stack_cap));
     const float4 pn = __ldg(rays + 2 * i), df = __ldg(rays + 2 * i + 1);
     lrt_hit h;
     trace_one(c, stack, blockDim.x, stack_cap, pn, df, h);
@@ -1890,38 +2073,46 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_adjoint_lambert(DevScene S
 }
 
 cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const DevLights& lights, uint32_t* image,
-                                unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int grid,
+                                unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int blocks,
                                 cudaStream_t stream, const uint32_t* sched_rd, uint32_t* sched_wr,
-                                const DevMaterials* materials, const DevRenderModes* rm, bool bricks_only)
+                                const DevMaterials* materials, const DevRenderModes* rm)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
   // one sample of LAMBERT_NO_TEX keeps its own instantiation (the benchmarked
-  // render; bounded to 80 registers for brick-only scenes); the other modes,
-  // several samples and transparency share the general one
+  // render); the other modes, several samples and transparency share the
+  // general one
   const bool modes = rm && (rm->mode != LRT_RENDER_MODE_LAMBERT_NO_TEX || rm->samples != 1 || rm->transparency);
-  auto kernel = modes ? k_render_rgba8<true> : bricks_only ? k_render_rgba8<false, 6> : k_render_rgba8<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  DevRenderModes one{};
-  one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
-  one.samples = 1;
-  kernel<<<grid, kTraceThreads, smem, stream>>>(S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd,
-                                                sched_wr, materials ? *materials : DevMaterials{}, rm ? *rm : one);
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
+    auto kernel = modes ? k_render_rgba8<true, K> : k_render_rgba8<false, K>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+    if (e != cudaSuccess) return e;
+    DevRenderModes one{};
+    one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
+    one.samples = 1;
+    kernel<<<grid, kTraceThreads, smem, stream>>>(S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd,
+                                                  sched_wr, materials ? *materials : DevMaterials{}, rm ? *rm : one);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_outline_fill(const DevScene& S, const DevCamera& cam, const DevLights& lights,
                                const DevMaterials& M, const DevRenderModes& RM, uint32_t smp, float2* tm, float4* col,
-                               unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int grid,
+                               unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int blocks,
                                cudaStream_t stream, const uint32_t* sched_rd, uint32_t* sched_wr)
 {
-  cudaError_t e = cudaFuncSetAttribute(k_outline_fill, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  k_outline_fill<<<grid, kTraceThreads, trace_smem_bytes(stack_cap), stream>>>(
-      S, cam, lights, M, RM, smp, tm, col, work_counter, err_word, stack_cap, sched_rd, sched_wr);
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
+    cudaError_t e = cudaFuncSetAttribute(k_outline_fill<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+    if (e != cudaSuccess) return e;
+    k_outline_fill<K><<<grid, kTraceThreads, trace_smem_bytes(stack_cap), stream>>>(
+        S, cam, lights, M, RM, smp, tm, col, work_counter, err_word, stack_cap, sched_rd, sched_wr);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_outline_resolve(const float2* tm, const float4* col, uint32_t w, uint32_t h, uint32_t smp,
@@ -1935,49 +2126,61 @@ cudaError_t launch_outline_resolve(const float2* tm, const float4* col, uint32_t
 
 cudaError_t launch_fill_gbuffer_transparency(const DevScene& S, const DevCamera& cam, const DevMaterials& M,
                                              float4* transparency, lrt_hit* gbuffer, unsigned long long* work_counter,
-                                             uint32_t* err_word, uint32_t stack_cap, int grid, cudaStream_t stream,
+                                             uint32_t* err_word, uint32_t stack_cap, int blocks, cudaStream_t stream,
                                              const uint32_t* sched_rd, uint32_t* sched_wr)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
-  cudaError_t e = cudaFuncSetAttribute(k_fill_gbuffer_transparency, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  k_fill_gbuffer_transparency<<<grid, kTraceThreads, smem, stream>>>(S, cam, M, transparency, gbuffer, work_counter,
-                                                                     err_word, stack_cap, sched_rd, sched_wr);
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
+    cudaError_t e = cudaFuncSetAttribute(k_fill_gbuffer_transparency<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+    if (e != cudaSuccess) return e;
+    k_fill_gbuffer_transparency<K><<<grid, kTraceThreads, smem, stream>>>(S, cam, M, transparency, gbuffer, work_counter,
+                                                                       err_word, stack_cap, sched_rd, sched_wr);
+    return cudaGetLastError();
+  });
 }
 
 // img_w > 0: the n = img_w * img_h rays are an image (row-major pixels)
 // traced in 8x4-pixel tiles in the order of the tile schedule (sched_rd,
 // sched_wr; nullptr for natural order).
 cudaError_t launch_render_lambert(const DevScene& S, const float4* rays, uint64_t n, float3 light, float* image,
-                                  unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int grid,
+                                  unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int blocks,
                                   cudaStream_t stream, uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd,
                                   uint32_t* sched_wr)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
-  auto kernel = img_w ? k_render_lambert<true> : k_render_lambert<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
-                                                img_h, sched_rd, sched_wr);
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
+    auto kernel = img_w ? k_render_lambert<true, K> : k_render_lambert<false, K>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
+                                                  img_h, sched_rd, sched_wr);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_adjoint_lambert(const DevScene& S, const float4* rays, uint64_t n, float3 light,
                                    const float* dimage, float* grad, unsigned long long* work_counter,
-                                   uint32_t* err_word, uint32_t stack_cap, int grid, cudaStream_t stream,
+                                   uint32_t* err_word, uint32_t stack_cap, int blocks, cudaStream_t stream,
                                    uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
-  auto kernel = img_w ? k_adjoint_lambert<true> : k_adjoint_lambert<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(trace_smem_bytes(kMaxStackDev + 1)));
-  if (e != cudaSuccess) return e;
-  kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
-                                                img_w, img_h, sched_rd, sched_wr);
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
+    auto kernel = img_w ? k_adjoint_lambert<true, K> : k_adjoint_lambert<false, K>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
+                                                  img_w, img_h, sched_rd, sched_wr);
+    return cudaGetLastError();
+  });
 }
 
 // Eye rays of one camera (MultiRenderer::initEyeRay), row-major pixels.
@@ -1996,9 +2199,8 @@ __global__ void k_eye_rays(DevCamera cam, float4* __restrict__ rays)
 // Host-side launchers (one copy per namespace; declared in trace_api.h).
 cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, uint64_t n,
                                 unsigned long long* work_counter, unsigned long long* counters, uint32_t* err_word,
-                                uint32_t stack_cap, int grid, cudaStream_t stream, bool count, uint32_t img_w,
-                                uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr, uint32_t group,
-                                bool bricks_only)
+                                uint32_t stack_cap, int blocks, cudaStream_t stream, bool count, uint32_t img_w,
+                                uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr, uint32_t group)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
   // the ANALYTIC / NEWTON / IT node solvers live in their own instantiation,
@@ -2007,24 +2209,31 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
   const bool solvers = solver != kSolverST && solver != kSolverBBox;
   // image order (IMG) is its own instantiation, so that the tile schedule
   // costs the row-order kernel nothing
-  auto go = [&](auto kernel) {
-    kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, hits, n, work_counter, counters, err_word, stack_cap, img_w,
-                                                  img_h, sched_rd, sched_wr, group);
+  auto go = [&](auto kernel, int most) {
+    kernel<<<std::min(blocks, most * int(S.sms)), kTraceThreads, smem, stream>>>(
+        S, rays, hits, n, work_counter, counters, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr, group);
+    return cudaGetLastError();
   };
-  if (img_w) {
-    if (count && solvers) go(k_trace<true, true, true>);
-    else if (count) go(k_trace<true, false, true>);
-    else if (solvers) go(k_trace<false, true, true>);
-    else if (bricks_only) go(k_trace<false, false, true, 6>);
-    else go(k_trace<false, false, true>);
-  } else {
-    if (count && solvers) go(k_trace<true, true, false>);
-    else if (count) go(k_trace<true, false, false>);
-    else if (solvers) go(k_trace<false, true, false>);
-    else if (group < 32) go(k_trace<false, false, false, 6>); // latency-bound: fewer spills per step
-    else go(k_trace<false, false, false>);
+  if (count) { // the counting kernels are compiled for all kinds
+    constexpr int B = min_blocks(kKindAll, kFrame);
+    if (img_w)
+      return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>, B)
+                     : go(k_trace<true, false, true, kKindAll, kFrame>, B);
+    return solvers ? go(k_trace<true, true, false, kKindAll, kFrame>, B)
+                   : go(k_trace<true, false, false, kKindAll, kFrame>, B);
   }
-  return cudaGetLastError();
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    constexpr int F = min_blocks(K, kFrame), M = min_blocks(K, kMany);
+    // the node solvers spill at any bound: their kernels keep the wider one
+    if (solvers)
+      return img_w ? go(k_trace<false, true, true, K, kFrame>, F) : go(k_trace<false, true, false, K, kFrame>, F);
+    // only scenes without bricks gain from the narrow one here
+    if constexpr (K == kKindNoBricks)
+      if (uint64_t(blocks) >= uint64_t(kManyWaves) * M * S.sms)
+        return img_w ? go(k_trace<false, false, true, K, kMany>, M) : go(k_trace<false, false, false, K, kMany>, M);
+    return img_w ? go(k_trace<false, false, true, K, kFrame>, F) : go(k_trace<false, false, false, K, kFrame>, F);
+  });
 }
 
 cudaError_t set_trace_smem(uint32_t stack_cap)
@@ -2034,28 +2243,30 @@ cudaError_t set_trace_smem(uint32_t stack_cap)
   auto set = [&](auto kernel) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   };
-  set(k_trace<true, false, false>);
-  set(k_trace<true, true, false>);
-  set(k_trace<false, true, false>);
-  set(k_trace<false, false, false>);
-  set(k_trace<true, false, true>);
-  set(k_trace<true, true, true>);
-  set(k_trace<false, true, true>);
-  set(k_trace<false, false, true>);
-  set(k_trace<false, false, true, 6>);
-  set(k_trace<false, false, false, 6>);
+  set(k_trace<true, false, false, kKindAll, kFrame>);
+  set(k_trace<true, true, false, kKindAll, kFrame>);
+  set(k_trace<true, false, true, kKindAll, kFrame>);
+  set(k_trace<true, true, true, kKindAll, kFrame>);
+  set(k_trace<false, false, false, kKindNoBricks, kMany>);
+  set(k_trace<false, false, true, kKindNoBricks, kMany>);
+  for (uint32_t kind : {kKindBricks, kKindNoBricks, kKindAll})
+    with_kind(kind, [&](auto k) {
+      constexpr uint32_t K = decltype(k)::value;
+      set(k_trace<false, false, false, K, kFrame>);
+      set(k_trace<false, false, true, K, kFrame>);
+      set(k_trace<false, true, false, K, kFrame>);
+      set(k_trace<false, true, true, K, kFrame>);
+    });
   return e;
 }
 
-cudaError_t trace_occupancy(uint32_t stack_cap, int* blocks_per_sm, bool bricks_only)
+cudaError_t trace_occupancy(uint32_t stack_cap, uint32_t kind, int* blocks_per_sm)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
-  // (k_render_rgba8<false, 6> has the same bound and shared memory)
-  if (bricks_only)
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_trace<false, false, true, 6>,
-                                                         kTraceThreads, smem);
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_trace<false, false, false>, kTraceThreads,
-                                                       smem);
+  return with_kind(kind, [&](auto k) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        blocks_per_sm, k_trace<false, false, true, decltype(k)::value, kFrame>, kTraceThreads, smem);
+  });
 }
 
 cudaError_t launch_eye_rays(const DevCamera& cam, float4* rays, cudaStream_t stream)
