@@ -31,6 +31,11 @@ constexpr int kPipeStreams = kPipeTrace + kPipeTraceStreams;
 constexpr uint64_t kPipeChunk = 262144;   // 8 MiB of rays in, 8 MiB of hits out
 constexpr uint64_t kPipeChunkMin = 32768; // first and last chunks
 constexpr uint64_t kPipeMinRays = 262144;
+// Host-pointer traces of fewer rays go through page-locked memory that the
+// kernel reads and writes over the bus; its size in rays grows in powers of
+// two from kStageMinRays.
+constexpr uint64_t kStageMinRays = 4096;
+constexpr uint64_t kStageHeader = 256; // error word
 
 // Tile schedule of the image-order launches of one image size on one stream
 // (sched_next in trace_impl.cuh): two device buffers of sched_words(tiles)
@@ -90,7 +95,11 @@ struct DeviceScene {
   // ray count of the last device-pointer lrt_trace_nearest on each stream: a
   // trace of the same count again has its 32-ray groups scheduled
   std::map<cudaStream_t, uint64_t> lastRays;
-  // staging buffers for host-pointer calls
+  // page-locked staging of the host-pointer calls that the kernel serves over
+  // the bus itself (trace_host_staged): an error word, rays, hits
+  unsigned char* stage = nullptr;
+  uint64_t stageCap = 0; // rays
+  // staging buffers for the other host-pointer calls
   float4* rays = nullptr;
   lrt_hit* hits = nullptr;
   uint64_t cap = 0;
@@ -114,6 +123,7 @@ struct DeviceScene {
     }
     if (pipeStart) cudaEventDestroy(pipeStart);
     for (void* p : allocs) cudaFree(p);
+    if (stage) cudaFreeHost(stage);
     if (rays) cudaFree(rays);
     if (hits) cudaFree(hits);
     if (tileScratch) cudaFree(tileScratch);

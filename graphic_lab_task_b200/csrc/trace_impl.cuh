@@ -1115,6 +1115,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_trace
     wclock[threadIdx.x >> 5].busy = 0;
   }
   l2_prefetch_scene(S);
+  uint64_t mine_from = (uint64_t(blockIdx.x) * (kTraceThreads / 32) + (threadIdx.x >> 5)) * group;
   for (;;) {
     unsigned long long base = 0;
     bool mine = true; // this lane's pixel belongs to the work item
@@ -1129,8 +1130,13 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_trace
       base = uint64_t(item_tile(item)) * 32;
       mine = item_has_lane(item, lane);
     } else { // in rays, `group` (32, 16 or 8) to a warp
-      if (lane == 0) base = atomicAdd(work_counter, (unsigned long long)group);
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
+      if (work_counter) {
+        if (lane == 0) base = atomicAdd(work_counter, (unsigned long long)group);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+      } else { // one group per warp of a launch of at most one wave
+        base = mine_from;
+        mine_from += uint64_t(gridDim.x) * (kTraceThreads / 32) * group;
+      }
       if (base >= n) break;
     }
     uint64_t i = base + lane;
