@@ -53,6 +53,46 @@ bool boxes_clean(const lrt_bvh_node* n, size_t count)
   return true;
 }
 
+// Turns `count` uploaded nodes into node records in place (device_layout.h).
+// owner: the geometry of each node pair.
+// flags |= 1 for a box with some but not six NaN coordinates, |= 2 for a leaf
+// entry that would read as the empty leaf's word.
+__global__ void __launch_bounds__(256) k_node_records(float4* __restrict__ nodes, uint64_t count,
+                                                      const uint32_t* __restrict__ owner,
+                                                      const DevGeom* __restrict__ geoms,
+                                                      const uint32_t* __restrict__ leafTable,
+                                                      uint32_t* __restrict__ flags)
+{
+  const uint64_t i = uint64_t(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= count) return;
+  const float4 a = nodes[2 * i], b = nodes[2 * i + 1];
+  uint32_t word = __float_as_uint(a.w);
+  if ((word & kLeafBit) && word != kLeafNormal) {
+    const uint32_t g = owner[i >> 1];
+    if (g != ~0u) word = kLeafBit | (leafTable[geoms[g].aabbBase + (word & kStartMask)] & ~kLeafBit);
+    if (word == kLeafNormal) atomicOr(flags, 2u);
+  }
+  const int nans = isnan(a.x) + isnan(a.y) + isnan(a.z) + isnan(b.x) + isnan(b.y) + isnan(b.z);
+  if (nans != 0 && nans != 6) atomicOr(flags, 1u);
+  nodes[2 * i] = make_float4(a.x, b.x, a.y, b.y);
+  nodes[2 * i + 1] = make_float4(a.z, b.z, __uint_as_float(word), b.w);
+}
+
+// The records of the few TLAS nodes, made on the host; their leaf words stay.
+void tlas_records(const std::vector<lrt_bvh_node>& in, bool sideBySide, std::vector<lrt_bvh_node>& out)
+{
+  out = in;
+  if (!sideBySide) return;
+  for (size_t i = 0; i < in.size(); i++) {
+    const lrt_bvh_node& n = in[i];
+    const float box[6] = {n.boxMin[0], n.boxMax[0], n.boxMin[1], n.boxMax[1], n.boxMin[2], n.boxMax[2]};
+    char* o = reinterpret_cast<char*>(&out[i]);
+    std::memcpy(o, box, sizeof(box));
+    std::memcpy(o + 24, &n.leftOffset, 4);
+    std::memcpy(o + 28, &n.escapeIndex, 4);
+  }
+}
+
 template <class T>
 lrt_status upload_vec(lrt_scene* s, DeviceScene* d, const T* src, size_t count, const T** out, const char* name)
 {
@@ -369,6 +409,37 @@ lrt_status trace_host_pipelined(lrt_scene* s, const float* rays, lrt_hit* hits, 
 
 } // namespace
 
+namespace {
+
+// Makes the node records of a scene without bricks from its uploaded BLAS
+// pairs and finds whether their boxes are clean.
+lrt_status node_records(lrt_scene* s, uint64_t count)
+{
+  DeviceScene* d = s->dev;
+  d->pairsClean = true;
+  if (count == 0) return LRT_OK;
+  uint32_t *owner = nullptr, *flags = nullptr, found = 0;
+  const size_t ownerBytes = s->pairGeom.size() * sizeof(uint32_t);
+  cudaError_t e = cudaMalloc(&owner, ownerBytes);
+  if (e == cudaSuccess) e = cudaMalloc(&flags, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemcpy(owner, s->pairGeom.data(), ownerBytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemset(flags, 0, sizeof(uint32_t));
+  if (e == cudaSuccess) {
+    k_node_records<<<unsigned((count + 255) / 256), 256>>>(reinterpret_cast<float4*>(const_cast<DevPair*>(d->S.pairs)),
+                                                           count, owner, d->S.geoms, d->S.primIdCount, flags);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(&found, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+  cudaFree(owner);
+  cudaFree(flags);
+  if (e != cudaSuccess) return cuda_fail(s, e, "node records");
+  if (found & 2u) return fail(s, LRT_ERR_UNSUPPORTED, "a BLAS leaf of 7 primitives starts at 2^28 - 1");
+  d->pairsClean = !(found & 1u);
+  return LRT_OK;
+}
+
+} // namespace
+
 // Device address of the static scratch array of lrt_trace_nearest_noalloc
 // (defined with it at the end of this file), for the current device.
 cudaError_t noalloc_scratch_address(void** p);
@@ -399,11 +470,18 @@ lrt_status device_upload(lrt_scene* s)
     st = upload_vec(s, d, reinterpret_cast<const T*>(vec.data()), vec.size() * sizeof(vec[0]) / sizeof(T), &p, name); \
     S.dst = p;                                                                                        \
   }
-  UP(tlas, h.nodesTLAS, lrt_bvh_node, "TLAS nodes")
-  UP(pairs, pairs, lrt_bvh_node_pair, "BLAS node pairs")
+  uint32_t kinds = 0;
+  for (uint32_t t : h.geomTags)
+    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
+           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
+  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
+  std::vector<lrt_bvh_node> tlas;
+  tlas_records(h.nodesTLAS, S.kind == kKindNoBricks, tlas);
+  UP(tlas, tlas, DevNode, "TLAS nodes")
+  UP(pairs, pairs, DevPair, "BLAS node pairs")
+  UP(primIdCount, h.primIdCount, uint32_t, "leaf table")
   UP(instances, h.instanceData, DevInstance, "instances")
   UP(geoms, geoms, DevGeom, "geometry table")
-  UP(primIdCount, h.primIdCount, uint32_t, "leaf table")
   UP(triSoup, soup, float4, "triangles")
   UP(primIndices, h.primIndices, uint32_t, "primIndices")
   UP(origNodes, h.origNodes, lrt_bvh_node, "origNodes")
@@ -419,17 +497,24 @@ lrt_status device_upload(lrt_scene* s)
     if (h.sdfSBSNodes.empty()) {
       d->pairsOrig = S.pairs; // nothing was pruned
     } else {
-      const lrt_bvh_node_pair* p = nullptr;
-      st = upload_vec(s, d, h.allNodePairs.data(), h.allNodePairs.size(), &p, "unpruned node pairs");
+      const DevPair* p = nullptr;
+      st = upload_vec(s, d, reinterpret_cast<const DevPair*>(h.allNodePairs.data()), h.allNodePairs.size(), &p,
+                      "unpruned node pairs");
       d->pairsOrig = p;
     }
+  }
+  if (S.kind == kKindNoBricks) {
+    if (st == LRT_OK) st = node_records(s, 2 * pairs.size());
+  } else { // the uploaded nodes are the records
+    d->pairsClean = boxes_clean(reinterpret_cast<const lrt_bvh_node*>(pairs.data()), 2 * pairs.size()) &&
+                    boxes_clean(reinterpret_cast<const lrt_bvh_node*>(h.allNodePairs.data()), 2 * h.allNodePairs.size());
   }
   d->sbsHost = sbs;
   d->pairsOrigBytes = (h.sdfSBSNodes.empty() ? pairs.size() : h.allNodePairs.size()) * sizeof(lrt_bvh_node_pair);
   // what a traversal reads per node, leaf, brick and voxel, most shared first
   d->pfCand = {{S.tlas, h.nodesTLAS.size() * sizeof(lrt_bvh_node)},
                {S.pairs, pairs.size() * sizeof(lrt_bvh_node_pair)},
-               {S.primIdCount, h.primIdCount.size() * sizeof(uint32_t)},
+               {S.kind == kKindNoBricks ? nullptr : S.primIdCount, h.primIdCount.size() * sizeof(uint32_t)},
                {S.sbsNodes, h.sdfSBSNodes.size() * sizeof(lrt_sdf_sbs_node)},
                {S.sbsMask, mask.size() * sizeof(uint32_t)},
                {S.triSoup, soup.size() * sizeof(float)},
@@ -438,8 +523,6 @@ lrt_status device_upload(lrt_scene* s)
                {S.svsNodes, h.sdfSVSNodes.size() * sizeof(lrt_sdf_svs_node)},
                {S.sbsDense, dense.size() * sizeof(float)}};
   set_prefetch(d);
-  d->pairsClean = boxes_clean(reinterpret_cast<const lrt_bvh_node*>(pairs.data()), 2 * pairs.size()) &&
-                  boxes_clean(reinterpret_cast<const lrt_bvh_node*>(h.allNodePairs.data()), 2 * h.allNodePairs.size());
   d->cleanBoxes = d->pairsClean && boxes_clean(h.nodesTLAS.data(), h.nodesTLAS.size());
   d->tlasCount = h.nodesTLAS.size();
   d->instCount = h.instanceData.size();
@@ -454,11 +537,6 @@ lrt_status device_upload(lrt_scene* s)
   e = lrt_exact::set_trace_smem(kMaxStack + 1);
   if (e == cudaSuccess) e = lrt_fast::set_trace_smem(kMaxStack + 1);
   int perSm = 0, sms = 0;
-  uint32_t kinds = 0;
-  for (uint32_t t : h.geomTags)
-    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
-           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
-  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
   if (e == cudaSuccess) e = lrt_exact::trace_occupancy(d->stackCap, S.kind, &perSm);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
   if (e == cudaSuccess) e = cudaMalloc(&d->slots, sizeof(StreamSlot) * kMaxStreams);
@@ -514,7 +592,9 @@ lrt_status device_update_instances(lrt_scene* s)
     e = cudaMemcpy(const_cast<void*>(*ptr), src, count * elem, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) st = cuda_fail(s, e, name);
   };
-  put(h.nodesTLAS.data(), h.nodesTLAS.size(), sizeof(lrt_bvh_node), d->tlasCount,
+  std::vector<lrt_bvh_node> tlas;
+  tlas_records(h.nodesTLAS, d->S.kind == kKindNoBricks, tlas);
+  put(tlas.data(), tlas.size(), sizeof(DevNode), d->tlasCount,
       reinterpret_cast<const void**>(&d->S.tlas), "TLAS nodes");
   put(h.instanceData.data(), h.instanceData.size(), sizeof(lrt_instance_data), d->instCount,
       reinterpret_cast<const void**>(&d->S.instances), "instances");

@@ -11,6 +11,15 @@
 //                 corner grid (2.9 KB for 8^3 bricks), so a voxel visit is 8
 //                 loads from 4 adjacent 8-byte pairs instead of 8 index loads
 //                 followed by 8 dependent value loads (BVH2Common.cpp:846-882);
+//   * node records — BLAS and TLAS nodes (two 16-byte words each).  In scenes
+//                 with bricks as the reference has them, {min, child}, {max,
+//                 escape}.  In the others each axis' two slabs lie side by
+//                 side, {min.x, max.x, min.y, max.y}, {min.z, max.z, child,
+//                 escape}, as the packed box test reads them, and a BLAS
+//                 leaf's child word is its leaf-table entry (kLeafBit | count
+//                 << 28 | start) instead of that entry's index, which takes
+//                 one dependent load from every leaf visit (the brick kernels
+//                 were 2% slower with it);
 //   * geoms     — 32 B per geometry with the tag, BLAS offset, leaf-table base
 //                 and SDF ids the traversal needs (one load per BLAS entry).
 // Values are copied bit for bit, so results do not depend on the layout.
@@ -159,12 +168,20 @@ constexpr uint32_t kPrefetchChunk = 4096; // bytes per prefetch instruction
 constexpr uint32_t kKindTriangles = 1, kKindNodes = 2; // triangles; frame-octree and SVS nodes
 constexpr uint32_t kKindBricks = 4, kKindNoBricks = kKindTriangles | kKindNodes, kKindAll = 7;
 
+struct DevNode { // a node record
+  float4 a, b;
+};
+struct DevPair { // a BLAS node pair
+  DevNode left, right;
+};
+static_assert(sizeof(DevPair) == 64, "DevPair is 64 bytes");
+
 struct DevScene {
-  const lrt_bvh_node* tlas;
-  const lrt_bvh_node_pair* pairs;
+  const DevNode* tlas;
+  const DevPair* pairs;
+  const uint32_t* primIdCount; // leaf table (scenes with bricks)
   const DevInstance* instances;
   const DevGeom* geoms;
-  const uint32_t* primIdCount;
   const float4* triSoup;
   const uint32_t* primIndices;
   const lrt_bvh_node* origNodes;

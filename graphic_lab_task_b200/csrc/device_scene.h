@@ -59,7 +59,7 @@ struct DeviceScene {
   int grid = 0; // blocks in one wave of the scene's trace kernel
   StreamSlot* slots = nullptr; // device, kMaxStreams
   std::map<cudaStream_t, int> slotOf;
-  const lrt_bvh_node_pair* pairsOrig = nullptr; // unpruned node pairs (used once SBS values change)
+  const DevPair* pairsOrig = nullptr;           // unpruned node pairs (used once SBS values change)
   uint64_t pairsOrigBytes = 0;
   // the arrays a trace may stream into L2 (DevScene::pfPtr), in priority
   // order, with their sizes; set_prefetch picks those that fit

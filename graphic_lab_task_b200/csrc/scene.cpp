@@ -568,7 +568,7 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
     I.hasSbsNeighbours = c.hasSbsNeighbours;
   }
   const size_t P = geomChecked ? 0 : h.allNodePairs.size();
-  std::vector<uint8_t> pairSeen(P, 0);
+  std::vector<uint32_t> pairGeom(P, ~0u);
   for (size_t g = 0; g < G && !geomChecked; g++) {
     const lrt_geom_data& gd = h.geomData[g];
     const uint32_t tag = h.geomTags[g];
@@ -587,8 +587,8 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
       if (dpt > 4096) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu BLAS deeper than 4096", g);
       const uint64_t abs = uint64_t(gd.bvhOffset) + k;
       if (abs >= P) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu pair %u beyond allNodePairs", g, k);
-      if (pairSeen[abs]) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu pair %u is reached twice", g, k);
-      pairSeen[abs] = 1;
+      if (pairGeom[abs] != ~0u) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu pair %u is reached twice", g, k);
+      pairGeom[abs] = uint32_t(g);
       const lrt_bvh_node* ch[2] = {&h.allNodePairs[abs].left, &h.allNodePairs[abs].right};
       for (int j = 0; j < 2; j++) {
         const uint32_t lo = ch[j]->leftOffset;
@@ -704,6 +704,7 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
   if (I.maxBlasDepth > kMaxStack)
     return fail(s, LRT_ERR_BAD_SCENE, "BLAS depth %u exceeds the %u-entry traversal stack", I.maxBlasDepth, kMaxStack);
   s->geomInfo = I;
+  if (!geomChecked) s->pairGeom = std::move(pairGeom);
   s->validatedGeomVersion = s->geomVersion;
   *info = I;
   return LRT_OK;

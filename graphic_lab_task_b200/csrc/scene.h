@@ -74,6 +74,7 @@ struct lrt_scene {
   uint64_t uploadedGeomVersion = 0;
   uint64_t validatedGeomVersion = 0; // geometry arrays last passed validation at this version
   lrt::SceneInfo geomInfo;           // what that validation found
+  std::vector<uint32_t> pairGeom;    // and the geometry whose BLAS holds each node pair (~0u: none)
   lrt::SceneInfo info;
   lrt::DeviceScene* dev = nullptr;
   int device = -1;

@@ -688,17 +688,27 @@ __device__ __forceinline__ f2 triangle_normal(const DevScene& S, const DevGeom& 
   return encode_normal(normalize(matmul4(S.instances[instId].transformInvTransposed, n, 1.0f)));
 }
 
+// Whether the scene's node records hold each axis' slabs side by side and
+// their leaves' table entries (device_layout.h): those of scenes without
+// bricks do.
+template <class CTX>
+__device__ __forceinline__ bool side_by_side(const DevScene& S)
+{
+  return CTX::kCount ? S.kind == kKindNoBricks : CTX::kKind == kKindNoBricks; // counting kernels serve all kinds
+}
+
 // IntersectAllPrimitivesInLeaf: returns the tag if the hit moved closer.
 // inv = SafeInverse(ray_dir); fast: the ray qualifies for the one-instruction
 // box tests (fast_nodes).
 template <class CTX>
 __device__ __forceinline__ uint32_t leaf(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f3 inv, bool fast,
-                                         float tNear, uint32_t aabbId, uint32_t instId, uint32_t geomId,
+                                         float tNear, uint32_t leafWord, uint32_t instId, uint32_t geomId,
                                          Hit& hit)
 {
   const float tPrev = hit.t;
   c.inc(kCntLeafCalls);
-  const uint32_t packed = __ldg(c.S.primIdCount + g.aabbBase + aabbId);
+  const uint32_t packed =
+      side_by_side<CTX>(c.S) ? leafWord : __ldg(c.S.primIdCount + g.aabbBase + (leafWord & 0x0FFFFFFFu));
   const uint32_t a_start = packed & 0x0FFFFFFFu;
   const uint32_t a_count = (packed & 0x70000000u) >> 28;
   if ((CTX::kKind & kKindTriangles) && g.tag == LRT_TAG_TRIANGLE) {
@@ -714,12 +724,83 @@ __device__ __forceinline__ uint32_t leaf(CTX& c, const DevGeom& g, f3 ray_pos, f
   return (hit.t >= tPrev) ? LRT_TAG_NONE : g.tag;
 }
 
-// Node box test: the literal RayBoxIntersection2 or, when the caller has
-// established the conditions under which it decides the same, ray_box_nodes.
-template <bool FAST>
-__device__ __forceinline__ f2 node_box(f3 o, f3 inv, f3 bmin, f3 bmax)
+__device__ __forceinline__ uint64_t pack2(float x, float y)
 {
-  return FAST ? ray_box_nodes(o, inv, bmin, bmax) : ray_box(o, inv, bmin, bmax);
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& x, float& y)
+{
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+// inv * (b + neg_o) of the two slabs of one axis, two lanes of each packed
+// operation; each rounds like the scalar subtraction and product it replaces
+// (b + (-o) is b - o), and a product of a sum cannot be contracted.
+__device__ __forceinline__ void slab2(float lo, float hi, uint64_t neg_o, uint64_t inv, float& t0, float& t1)
+{
+  uint64_t v = pack2(lo, hi);
+  asm("add.rn.f32x2 %0, %0, %1;\n\tmul.rn.f32x2 %0, %0, %2;" : "+l"(v) : "l"(neg_o), "l"(inv));
+  unpack2(v, t0, t1);
+}
+
+// A ray for node tests: for the packed ones each component twice.
+template <bool PACKED>
+struct NodeRay {
+  uint64_t ox, oy, oz, ix, iy, iz; // -origin, inverse direction
+  __device__ __forceinline__ NodeRay(f3 o, f3 inv)
+      : ox(pack2(-o.x, -o.x)), oy(pack2(-o.y, -o.y)), oz(pack2(-o.z, -o.z)), ix(pack2(inv.x, inv.x)),
+        iy(pack2(inv.y, inv.y)), iz(pack2(inv.z, inv.z))
+  {
+  }
+};
+
+template <>
+struct NodeRay<false> {
+  __device__ __forceinline__ NodeRay(f3, f3) {}
+};
+
+__device__ __forceinline__ f2 node_box_packed(const NodeRay<true>& r, float4 a, float4 b)
+{
+  float lo, hi, lo1, hi1, lo2, hi2;
+  slab2(a.x, a.y, r.ox, r.ix, lo, hi);
+  slab2(a.z, a.w, r.oy, r.iy, lo1, hi1);
+  slab2(b.x, b.y, r.oz, r.iz, lo2, hi2);
+  const float tmin = fmaxf(fminf(lo, hi), fminf(lo1, hi1));
+  const float tmax = fminf(fmaxf(lo, hi), fmaxf(lo1, hi1));
+  return mk2(fmaxf(tmin, fminf(lo2, hi2)), fminf(tmax, fmaxf(lo2, hi2)));
+}
+
+template <class CTX>
+__device__ __forceinline__ uint32_t node_child(const DevScene& S, float4 a, float4 b)
+{
+  return __float_as_uint(side_by_side<CTX>(S) ? b.z : a.w);
+}
+
+// Box test of a node record: the literal RayBoxIntersection2 or, FAST, when
+// the caller has established the conditions under which it decides the same,
+// ray_box_nodes; in kernels without bricks with its subtractions and products
+// packed in pairs, which takes 12 of a pair visit's ~75 instructions away:
+// instanced 4096^2 primary rays 5,577 -> 5,394 us, sorted bounce rays 5,945 ->
+// 5,730, a 200k-triangle mesh at 256^2 102 -> 99.  The brick kernels lose 10%
+// to holding the ray twice (512^3 at 1920x1080 495 -> 541 us).
+template <bool FAST, class CTX>
+constexpr bool kPackedTests = FAST && !CTX::kCount && CTX::kKind == kKindNoBricks;
+
+template <bool FAST, class CTX>
+__device__ __forceinline__ f2 node_box(const DevScene& S, const NodeRay<kPackedTests<FAST, CTX>>& r, f3 o, f3 inv,
+                                       float4 a, float4 b)
+{
+  if constexpr (kPackedTests<FAST, CTX>) {
+    return node_box_packed(r, a, b);
+  } else {
+    f3 bmin = ld3(a), bmax = ld3(b);
+    if (side_by_side<CTX>(S)) {
+      bmin = mk3(a.x, a.z, b.x);
+      bmax = mk3(a.y, a.w, b.y);
+    }
+    return FAST ? ray_box_nodes(o, inv, bmin, bmax) : ray_box(o, inv, bmin, bmax);
+  }
 }
 
 // Rays for which ray_box_nodes decides every node test like ray_box: finite
@@ -737,13 +818,14 @@ __device__ __forceinline__ bool blas_descend(CTX& c, const float4* pairs, uint32
                                              uint32_t cap, f3 ray_pos, f3 inv, float tNear, float tHit, int& top,
                                              uint32_t& leftNodeOffset)
 {
+  const NodeRay<kPackedTests<FAST, CTX>> pr(ray_pos, inv);
   while (top >= 0 && ((leftNodeOffset & kLeafBit) == 0)) {
     c.inc(kCntBlasPairs);
     const float4* p = pairs + 4 * uint64_t(leftNodeOffset);
     const float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
-    const uint32_t n0 = __float_as_uint(l0.w), n1 = __float_as_uint(r0.w);
-    const f2 tm0 = node_box<FAST>(ray_pos, inv, ld3(l0), ld3(l1));
-    const f2 tm1 = node_box<FAST>(ray_pos, inv, ld3(r0), ld3(r1));
+    const uint32_t n0 = node_child<CTX>(c.S, l0, l1), n1 = node_child<CTX>(c.S, r0, r1);
+    const f2 tm0 = node_box<FAST, CTX>(c.S, pr, ray_pos, inv, l0, l1);
+    const f2 tm1 = node_box<FAST, CTX>(c.S, pr, ray_pos, inv, r0, r1);
     const bool h0 = (tm0.x <= tm0.y) && (tm0.y >= tNear) && (tm0.x <= tHit);
     const bool h1 = (tm1.x <= tm1.y) && (tm1.y >= tNear) && (tm1.x <= tHit);
     leftNodeOffset = h0 ? n0 : n1;
@@ -771,13 +853,14 @@ template <bool FAST, class CTX>
 __device__ __forceinline__ void tlas_walk(CTX& c, f3 pos, f3 inv, float tmin, float tHit, uint32_t& nodeIdx,
                                           uint32_t& travFlags, uint32_t& leftOffset)
 {
+  const NodeRay<kPackedTests<FAST, CTX>> pr(pos, inv);
   do {
     c.inc(kCntTlasNodes);
     const float4* np = reinterpret_cast<const float4*>(c.S.tlas + nodeIdx);
     const float4 a = __ldg(np), b = __ldg(np + 1);
-    const f2 bh = node_box<FAST>(pos, inv, ld3(a), ld3(b));
+    const f2 bh = node_box<FAST, CTX>(c.S, pr, pos, inv, a, b);
     const uint32_t intersects = (bh.x <= bh.y) && (bh.y > tmin) && (bh.x < tHit);
-    const uint32_t lo = __float_as_uint(a.w);
+    const uint32_t lo = node_child<CTX>(c.S, a, b);
     travFlags = (lo & kLeafBit) | intersects;
     leftOffset = lo;
     const bool leafOrNot = (travFlags & kLeafBit) != 0 || (travFlags & 1) == 0;
@@ -873,7 +956,7 @@ __device__ __forceinline__ uint32_t walk_leaf(CTX& c, Walk& w, uint32_t* stack, 
     const DevGeom g = c.S.geoms[w.geomId];
     const float tNearSdf = smax(w.tmin, 0.01f); // SDF_BIAS (BVH2Common.cpp:3306-3307)
     const uint32_t tag =
-        leaf(c, g, w.rp, w.rd, w.inv, w.fast, tNearSdf, w.cur & 0x0FFFFFFFu, w.instId, w.geomId, w.hit);
+        leaf(c, g, w.rp, w.rd, w.inv, w.fast, tNearSdf, w.cur, w.instId, w.geomId, w.hit);
     ended = (tag != 0) && (tag != LRT_TAG_TRIANGLE || w.stopOnFirst);
   }
   w.top--;
