@@ -509,6 +509,21 @@ lrt_status device_upload(lrt_scene* s)
     d->pairsClean = boxes_clean(reinterpret_cast<const lrt_bvh_node*>(pairs.data()), 2 * pairs.size()) &&
                     boxes_clean(reinterpret_cast<const lrt_bvh_node*>(h.allNodePairs.data()), 2 * h.allNodePairs.size());
   }
+  std::vector<PruneLeaf> leaves;
+  std::vector<uint32_t> parent;
+  build_prune_tree(h, geoms, sbs, leaves, parent);
+  if (!leaves.empty()) {
+    const PruneLeaf* pl = nullptr;
+    const uint32_t *pp = nullptr, *pa = nullptr;
+    if (st == LRT_OK) st = upload_vec(s, d, leaves.data(), leaves.size(), &pl, "SBS leaf slots");
+    if (st == LRT_OK) st = upload_vec(s, d, parent.data(), parent.size(), &pp, "SBS pair parents");
+    if (st == LRT_OK) st = upload_vec(s, d, parent.data(), parent.size(), &pa, "SBS live-child bits");
+    d->pruneLeaves = pl;
+    d->pruneParent = pp;
+    d->pruneAlive = const_cast<uint32_t*>(pa);
+    d->pruneLeafCount = uint32_t(leaves.size());
+    d->prunePairs = uint32_t(parent.size());
+  }
   d->sbsHost = sbs;
   d->pairsOrigBytes = (h.sdfSBSNodes.empty() ? pairs.size() : h.allNodePairs.size()) * sizeof(lrt_bvh_node_pair);
   // what a traversal reads per node, leaf, brick and voxel, most shared first

@@ -145,6 +145,16 @@ struct DevSbs {
 // the same floats.  A clear bit means the reference does nothing in that
 // voxel but advance the march.
 
+// What the device needs to prune the SBS node pairs again after new values
+// (lrt_sbs_update_values): per leaf of an SBS BLAS the child slot that names
+// it (pair << 1 | side) and the brick's first mask word; per node pair the
+// child slot that leads to it (kPruneRoot for the root of an SBS BLAS,
+// kPruneOther for the pairs of other geometry).
+struct PruneLeaf {
+  uint32_t slot, mask;
+};
+constexpr uint32_t kPruneRoot = 0xFFFFFFFFu, kPruneOther = 0xFFFFFFFEu;
+
 typedef lrt_instance_data DevInstance;
 
 // L2 prefetch of small scenes.  A launch whose rays are few takes as long as

@@ -59,8 +59,14 @@ struct DeviceScene {
   int grid = 0; // blocks in one wave of the scene's trace kernel
   StreamSlot* slots = nullptr; // device, kMaxStreams
   std::map<cudaStream_t, int> slotOf;
-  const DevPair* pairsOrig = nullptr;           // unpruned node pairs (used once SBS values change)
+  const DevPair* pairsOrig = nullptr; // unpruned node pairs
   uint64_t pairsOrigBytes = 0;
+  // the SBS node pairs' tree and one word of live-child bits per pair, for
+  // pruning again after new SBS values (nullptr: the unpruned pairs serve then)
+  const PruneLeaf* pruneLeaves = nullptr;
+  const uint32_t* pruneParent = nullptr;
+  uint32_t* pruneAlive = nullptr;
+  uint32_t pruneLeafCount = 0, prunePairs = 0;
   // the arrays a trace may stream into L2 (DevScene::pfPtr), in priority
   // order, with their sizes; set_prefetch picks those that fit
   std::vector<std::pair<const void*, uint64_t>> pfCand;

@@ -143,6 +143,41 @@ uint64_t prune_sbs_pairs(const HostArrays& h, const std::vector<DevGeom>& geoms,
   return pruned;
 }
 
+void build_prune_tree(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,
+                      std::vector<PruneLeaf>& leaves, std::vector<uint32_t>& parent)
+{
+  leaves.clear();
+  parent.clear();
+  if (h.sdfSBSNodes.empty() || h.allNodePairs.size() >= (1u << 30)) return;
+  for (const DevSbs& sb : sbs)
+    if (sb.maskBase + uint64_t(sb.nodeCount) * sb.maskStride >= 0xFFFFFFFFull) return;
+  parent.assign(h.allNodePairs.size(), kPruneOther);
+  std::vector<uint32_t> todo;
+  for (size_t g = 0; g < geoms.size(); g++) {
+    if (geoms[g].tag != LRT_TAG_SDF_BRICK) continue;
+    const DevSbs& sb = sbs[geoms[g].sdfId];
+    const uint32_t base = geoms[g].bvhOffset, a0 = geoms[g].aabbBase;
+    parent[base] = kPruneRoot;
+    todo.assign(1, base);
+    while (!todo.empty()) {
+      const uint32_t p = todo.back();
+      todo.pop_back();
+      for (uint32_t j = 0; j < 2; j++) {
+        const uint32_t lo = (j ? h.allNodePairs[p].right : h.allNodePairs[p].left).leftOffset;
+        const uint32_t slot = (p << 1) | j;
+        if (!(lo & kLeafBit)) {
+          parent[base + lo] = slot;
+          todo.push_back(base + lo);
+        } else if (lo != kLeafNormal) {
+          const uint32_t primId = h.primIdCount[a0 + (lo & kStartMask)] & kStartMask;
+          if (primId < sb.nodeCount)
+            leaves.push_back({slot, uint32_t(sb.maskBase + uint64_t(primId) * sb.maskStride)});
+        }
+      }
+    }
+  }
+}
+
 // Dense (brick_size+1)^3 corner grids per SBS node; values as
 // load_distance_values returns them (BVH2Common.cpp:846-882).
 void build_sbs_dense(const HostArrays& h, std::vector<DevSbs>& sbs, std::vector<float>& dense)

@@ -14,5 +14,9 @@ void build_sbs_masks(const HostArrays& h, std::vector<DevSbs>& sbs, const std::v
                      std::vector<uint32_t>& mask);
 uint64_t prune_sbs_pairs(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,
                          const std::vector<uint32_t>& mask, std::vector<lrt_bvh_node_pair>& pairs);
+// The tree of the SBS node pairs as k_prune_mark climbs it; empty without SBS
+// geometry, or if its indices do not fit 32 bits.
+void build_prune_tree(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,
+                      std::vector<PruneLeaf>& leaves, std::vector<uint32_t>& parent);
 
 } // namespace lrt
