@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "device_scene.h"
+#include "layout.h"
 #include "trace_api.h"
 
 namespace lrt {
@@ -160,18 +161,6 @@ lrt_status upload_materials(lrt_scene* s)
   if (e != cudaSuccess) return cuda_fail(s, e, "material tables host->device");
   d->matVersion = s->matVersion;
   return LRT_OK;
-}
-
-// Triangle slots of geometry g (its records in the triangle soup): one past
-// the largest leaf range of its leaf table, as build_tri_soup counts them.
-uint64_t triangle_slots(const HostArrays& h, size_t g)
-{
-  uint64_t ntri = 0;
-  for (uint32_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a++) {
-    const uint32_t pk = h.primIdCount[a];
-    ntri = std::max<uint64_t>(ntri, uint64_t(pk & 0x0FFFFFFFu) + ((pk & 0x70000000u) >> 28));
-  }
-  return ntri;
 }
 
 // Copies the textures and the triangles' texture coordinates to the device

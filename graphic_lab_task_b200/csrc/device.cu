@@ -78,6 +78,23 @@ __global__ void __launch_bounds__(256) k_node_records(float4* __restrict__ nodes
   nodes[2 * i + 1] = make_float4(a.z, b.z, __uint_as_float(word), b.w);
 }
 
+// {A, B-A, C-A} per reordered triangle slot of one geometry, from the
+// vertices (float4) and indices; IntersectAllTrianglesInLeaf computes exactly
+// these differences (BVH2Common.cpp:1585-1589).
+__global__ void __launch_bounds__(256) k_tri_soup(const float4* __restrict__ verts, const uint32_t* __restrict__ indices,
+                                                  uint64_t firstVert, uint64_t base, uint64_t count,
+                                                  float4* __restrict__ soup)
+{
+  const uint64_t t = uint64_t(blockIdx.x) * 256 + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t* idx = indices + 3 * (base + t);
+  const float4 A = verts[firstVert + idx[0]], B = verts[firstVert + idx[1]], C = verts[firstVert + idx[2]];
+  float4* o = soup + 3 * (base + t);
+  o[0] = make_float4(A.x, A.y, A.z, 0.0f);
+  o[1] = make_float4(__fsub_rn(B.x, A.x), __fsub_rn(B.y, A.y), __fsub_rn(B.z, A.z), 0.0f);
+  o[2] = make_float4(__fsub_rn(C.x, A.x), __fsub_rn(C.y, A.y), __fsub_rn(C.z, A.z), 0.0f);
+}
+
 // The records of the few TLAS nodes, made on the host; their leaf words stay.
 void tlas_records(const std::vector<lrt_bvh_node>& in, bool sideBySide, std::vector<lrt_bvh_node>& out)
 {
@@ -411,6 +428,42 @@ lrt_status trace_host_pipelined(lrt_scene* s, const float* rays, lrt_hit* hits, 
 
 namespace {
 
+// Builds the triangle soup on the device (48 bytes a triangle, made there from
+// its 12 bytes of indices and the shared vertices).
+lrt_status tri_soup(lrt_scene* s)
+{
+  DeviceScene* d = s->dev;
+  const HostArrays& h = s->h;
+  const uint64_t nslots = h.indices.size() / 3;
+  d->S.triSoup = nullptr;
+  if (nslots == 0) return LRT_OK;
+  void *soup = nullptr, *verts = nullptr, *idx = nullptr;
+  const size_t vertBytes = h.vertPos.size() * sizeof(float), idxBytes = h.indices.size() * sizeof(uint32_t);
+  cudaError_t e = cudaMalloc(&soup, nslots * 48);
+  if (e != cudaSuccess) return cuda_fail(s, e, "triangles");
+  d->allocs.push_back(soup);
+  e = cudaMalloc(&verts, std::max<size_t>(vertBytes, 16));
+  if (e == cudaSuccess) e = cudaMalloc(&idx, idxBytes);
+  if (e == cudaSuccess) e = cudaMemcpy(verts, h.vertPos.data(), vertBytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(idx, h.indices.data(), idxBytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemsetAsync(soup, 0, nslots * 48);
+  for (size_t g = 0; g < h.geomData.size() && e == cudaSuccess; g++) {
+    if (h.geomTags[g] != LRT_TAG_TRIANGLE) continue;
+    const uint64_t base = h.geomData[g].offset[0] / 3;
+    const uint64_t n = base < nslots ? std::min(triangle_slots(h, g), nslots - base) : 0;
+    if (n == 0) continue;
+    k_tri_soup<<<unsigned((n + 255) / 256), 256>>>(static_cast<const float4*>(verts), static_cast<const uint32_t*>(idx),
+                                                   h.geomData[g].offset[1], base, n, static_cast<float4*>(soup));
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  cudaFree(verts);
+  cudaFree(idx);
+  if (e != cudaSuccess) return cuda_fail(s, e, "triangles");
+  d->S.triSoup = static_cast<const float4*>(soup);
+  return LRT_OK;
+}
+
 // Makes the node records of a scene without bricks from its uploaded BLAS
 // pairs and finds whether their boxes are clean.
 lrt_status node_records(lrt_scene* s, uint64_t count)
@@ -454,15 +507,15 @@ lrt_status device_upload(lrt_scene* s)
   const HostArrays& h = s->h;
   DevScene& S = d->S;
   std::vector<DevGeom> geoms;
-  std::vector<float> soup, dense;
+  std::vector<float> dense;
   std::vector<DevSbs> sbs;
   std::vector<uint32_t> mask;
   build_geoms(h, geoms);
-  build_tri_soup(h, soup);
   build_sbs_dense(h, sbs, dense);
   build_sbs_masks(h, sbs, dense, mask);
-  std::vector<lrt_bvh_node_pair> pairs;
-  prune_sbs_pairs(h, geoms, sbs, mask, pairs);
+  HostVec<lrt_bvh_node_pair> pruned;
+  if (!h.sdfSBSNodes.empty()) prune_sbs_pairs(h, geoms, sbs, mask, pruned);
+  const HostVec<lrt_bvh_node_pair>& pairs = h.sdfSBSNodes.empty() ? h.allNodePairs : pruned;
   lrt_status st = LRT_OK;
 #define UP(dst, vec, T, name)                                                                        \
   if (st == LRT_OK) {                                                                                 \
@@ -482,7 +535,7 @@ lrt_status device_upload(lrt_scene* s)
   UP(primIdCount, h.primIdCount, uint32_t, "leaf table")
   UP(instances, h.instanceData, DevInstance, "instances")
   UP(geoms, geoms, DevGeom, "geometry table")
-  UP(triSoup, soup, float4, "triangles")
+  if (st == LRT_OK) st = tri_soup(s);
   UP(primIndices, h.primIndices, uint32_t, "primIndices")
   UP(origNodes, h.origNodes, lrt_bvh_node, "origNodes")
   UP(frameOctreeNodes, h.sdfFrameOctreeNodes, lrt_sdf_frame_octree_node, "frame-octree nodes")
@@ -532,7 +585,7 @@ lrt_status device_upload(lrt_scene* s)
                {S.kind == kKindNoBricks ? nullptr : S.primIdCount, h.primIdCount.size() * sizeof(uint32_t)},
                {S.sbsNodes, h.sdfSBSNodes.size() * sizeof(lrt_sdf_sbs_node)},
                {S.sbsMask, mask.size() * sizeof(uint32_t)},
-               {S.triSoup, soup.size() * sizeof(float)},
+               {S.triSoup, h.indices.size() / 3 * 48},
                {S.origNodes, h.origNodes.size() * sizeof(lrt_bvh_node)},
                {S.frameOctreeNodes, h.sdfFrameOctreeNodes.size() * sizeof(lrt_sdf_frame_octree_node)},
                {S.svsNodes, h.sdfSVSNodes.size() * sizeof(lrt_sdf_svs_node)},

@@ -33,32 +33,14 @@ void build_geoms(const HostArrays& h, std::vector<DevGeom>& out)
   }
 }
 
-// {A, B-A, C-A} per reordered triangle slot; IntersectAllTrianglesInLeaf
-// computes exactly these differences (BVH2Common.cpp:1585-1589).
-void build_tri_soup(const HostArrays& h, std::vector<float>& soup)
+uint64_t triangle_slots(const HostArrays& h, size_t g)
 {
-  const size_t nslots = h.indices.size() / 3;
-  soup.assign(nslots * 12, 0.0f);
-  for (size_t g = 0; g < h.geomData.size(); g++) {
-    if (h.geomTags[g] != LRT_TAG_TRIANGLE) continue;
-    const lrt_geom_data& gd = h.geomData[g];
-    uint64_t ntri = 0;
-    for (uint32_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a++) {
-      const uint32_t pk = h.primIdCount[a];
-      ntri = std::max<uint64_t>(ntri, uint64_t(pk & 0x0FFFFFFFu) + ((pk & 0x70000000u) >> 28));
-    }
-    const uint64_t base = gd.offset[0] / 3;
-    for (uint64_t t = 0; t < ntri && base + t < nslots; t++) {
-      const float* P[3];
-      for (int c = 0; c < 3; c++) P[c] = h.vertPos.data() + 4 * (uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + 3 * t + c]);
-      float* o = soup.data() + 12 * (base + t);
-      for (int k = 0; k < 3; k++) {
-        o[k] = P[0][k];
-        o[4 + k] = P[1][k] - P[0][k];
-        o[8 + k] = P[2][k] - P[0][k];
-      }
-    }
+  uint64_t ntri = 0;
+  for (uint32_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a++) {
+    const uint32_t pk = h.primIdCount[a];
+    ntri = std::max<uint64_t>(ntri, uint64_t(pk & 0x0FFFFFFFu) + ((pk & 0x70000000u) >> 28));
   }
+  return ntri;
 }
 
 // Surface-voxel masks of every brick from its dense corner grid (see
@@ -110,7 +92,7 @@ void build_sbs_masks(const HostArrays& h, std::vector<DevSbs>& sbs, const std::v
 // other child is pruned the reference would visit that child (before or
 // after) without effect.  Returns the number of pruned children.
 uint64_t prune_sbs_pairs(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,
-                         const std::vector<uint32_t>& mask, std::vector<lrt_bvh_node_pair>& pairs)
+                         const std::vector<uint32_t>& mask, HostVec<lrt_bvh_node_pair>& pairs)
 {
   pairs = h.allNodePairs;
   const float qnan = std::numeric_limits<float>::quiet_NaN();

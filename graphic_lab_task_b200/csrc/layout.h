@@ -8,12 +8,14 @@
 namespace lrt {
 
 void build_geoms(const HostArrays& h, std::vector<DevGeom>& out);
-void build_tri_soup(const HostArrays& h, std::vector<float>& soup);
+// Records of triangle geometry g in the triangle soup (one past the largest
+// leaf range of its leaf table).
+uint64_t triangle_slots(const HostArrays& h, size_t g);
 void build_sbs_dense(const HostArrays& h, std::vector<DevSbs>& sbs, std::vector<float>& dense);
 void build_sbs_masks(const HostArrays& h, std::vector<DevSbs>& sbs, const std::vector<float>& dense,
                      std::vector<uint32_t>& mask);
 uint64_t prune_sbs_pairs(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,
-                         const std::vector<uint32_t>& mask, std::vector<lrt_bvh_node_pair>& pairs);
+                         const std::vector<uint32_t>& mask, HostVec<lrt_bvh_node_pair>& pairs);
 // The tree of the SBS node pairs as k_prune_mark climbs it; empty without SBS
 // geometry, or if its indices do not fit 32 bits.
 void build_prune_tree(const HostArrays& h, const std::vector<DevGeom>& geoms, const std::vector<DevSbs>& sbs,

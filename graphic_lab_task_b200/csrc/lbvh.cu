@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cstdio>
 #include <map>
 #include <mutex>
@@ -410,10 +411,41 @@ struct Arena {
 
 namespace {
 
+// The triangles' boxes, with the host's order of comparisons (std::min and
+// std::max keep the first of equal values and ignore a NaN second one).
+__global__ void k_triangle_boxes(const float4* __restrict__ verts, const uint32_t* __restrict__ tris, uint32_t n,
+                                 float* __restrict__ boxes)
+{
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+  for (int c = 0; c < 3; c++) {
+    const float4 v = verts[tris[3 * uint64_t(t) + c]];
+    const float p[3] = {v.x, v.y, v.z};
+    for (int k = 0; k < 3; k++) {
+      lo[k] = p[k] < lo[k] ? p[k] : lo[k];
+      hi[k] = hi[k] < p[k] ? p[k] : hi[k];
+    }
+  }
+  float* b = boxes + 6 * uint64_t(t);
+  for (int k = 0; k < 3; k++) {
+    b[k] = lo[k];
+    b[3 + k] = hi[k];
+  }
+}
+
+// What the tree is built over: n boxes, or n triangles.
+struct BuildInput {
+  const float* boxes6 = nullptr;
+  const float* verts4 = nullptr;
+  const uint32_t* tris = nullptr;
+  uint32_t nverts = 0;
+};
+
 // The build on the current device; with `emit` (maxLeaf > 0) the triangle
 // BLAS emission too.  Outputs: order and, without emission, the inner nodes;
 // with it, the pairs and leaf table (order then being the leaves' box order).
-const char* run(const float* boxes6, uint32_t n, uint32_t maxLeaf, bool emit, std::vector<uint32_t>& order,
+const char* run(const BuildInput& in, uint32_t n, uint32_t maxLeaf, bool emit, std::vector<uint32_t>& order,
                 std::vector<LbvhInner>* innerOut, const std::function<LbvhPairOut*(size_t)>* pairsAt,
                 std::vector<uint32_t>* startCountOut)
 {
@@ -445,7 +477,8 @@ const char* run(const float* boxes6, uint32_t n, uint32_t maxLeaf, bool emit, st
   Arena A;
   auto carve = [&](Arena& a) {
     struct P {
-      float* boxes;
+      float *boxes, *verts;
+      uint32_t* tris;
       uint32_t *bounds, *codes, *codesAlt, *ids, *idsAlt, *parentLeaf, *parentInner, *arrivals, *err;
       LbvhInner* inner;
       void* temp;
@@ -456,6 +489,8 @@ const char* run(const float* boxes6, uint32_t n, uint32_t maxLeaf, bool emit, st
       void* scanTemp;
     } p;
     p.boxes = a.take<float>(6 * size_t(n));
+    p.verts = a.take<float>(4 * size_t(in.nverts));
+    p.tris = a.take<uint32_t>(in.tris ? 3 * size_t(n) : 0);
     p.bounds = a.take<uint32_t>(8);
     p.codes = a.take<uint32_t>(n);
     p.codesAlt = a.take<uint32_t>(n);
@@ -507,8 +542,19 @@ const char* run(const float* boxes6, uint32_t n, uint32_t maxLeaf, bool emit, st
   const auto P = carve(A);
   cudaStream_t st = nullptr;
   LBVH_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
-  LBVH_TRY(cudaMemcpyAsync(P.boxes, boxes6, 6 * sizeof(float) * size_t(n), cudaMemcpyHostToDevice, st),
-           "boxes host->device");
+  if (in.tris) {
+    LBVH_TRY(cudaMemcpyAsync(P.verts, in.verts4, 16 * size_t(in.nverts), cudaMemcpyHostToDevice, st),
+             "vertices host->device");
+    LBVH_TRY(cudaMemcpyAsync(P.tris, in.tris, 12 * size_t(n), cudaMemcpyHostToDevice, st), "triangles host->device");
+    if (e == cudaSuccess) {
+      k_triangle_boxes<<<blocks, kBlock, 0, st>>>(reinterpret_cast<const float4*>(P.verts), P.tris, n, P.boxes);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) what = "triangle box kernel";
+    }
+  } else {
+    LBVH_TRY(cudaMemcpyAsync(P.boxes, in.boxes6, 6 * sizeof(float) * size_t(n), cudaMemcpyHostToDevice, st),
+             "boxes host->device");
+  }
   LBVH_TRY(cudaMemsetAsync(P.arrivals, 0, sizeof(uint32_t) * m, st), "memset");
   LBVH_TRY(cudaMemsetAsync(P.err, 0, sizeof(uint32_t), st), "memset");
   if (e == cudaSuccess) {
@@ -618,14 +664,20 @@ const char* run(const float* boxes6, uint32_t n, uint32_t maxLeaf, bool emit, st
 
 const char* lbvh_build(const float* boxes6, uint32_t n, std::vector<uint32_t>& order, std::vector<LbvhInner>& inner)
 {
-  return run(boxes6, n, 0, false, order, &inner, nullptr, nullptr);
+  BuildInput in;
+  in.boxes6 = boxes6;
+  return run(in, n, 0, false, order, &inner, nullptr, nullptr);
 }
 
-const char* lbvh_build_blas(const float* boxes6, uint32_t n, uint32_t maxLeaf,
+const char* lbvh_build_blas(const float* verts4, uint32_t nverts, const uint32_t* tris, uint32_t n, uint32_t maxLeaf,
                             const std::function<LbvhPairOut*(size_t)>& pairsAt, std::vector<uint32_t>& startCount,
                             std::vector<uint32_t>& order)
 {
-  return run(boxes6, n, std::max(1u, maxLeaf), true, order, nullptr, &pairsAt, &startCount);
+  BuildInput in;
+  in.verts4 = verts4;
+  in.nverts = nverts;
+  in.tris = tris;
+  return run(in, n, std::max(1u, maxLeaf), true, order, nullptr, &pairsAt, &startCount);
 }
 
 } // namespace lrt

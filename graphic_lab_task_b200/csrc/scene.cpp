@@ -249,7 +249,7 @@ lrt_bvh_node dummy_node()
 // packed leftOffset of a leaf.  escapeIndex follows the aligned-array
 // convention of AlignNodes2 (left -> its right sibling, right -> parent's).
 template <class Tree, class LeafWord>
-void emit_pairs(const Tree& B, std::vector<lrt_bvh_node_pair>& out, LeafWord leafWord)
+void emit_pairs(const Tree& B, HostVec<lrt_bvh_node_pair>& out, LeafWord leafWord)
 {
   const BNode& root = B.nodes[0];
   if (root.leaf()) {
@@ -260,7 +260,7 @@ void emit_pairs(const Tree& B, std::vector<lrt_bvh_node_pair>& out, LeafWord lea
     return;
   }
   struct Rec {
-    static uint32_t go(const Tree& B, std::vector<lrt_bvh_node_pair>& out, int32_t node, uint32_t base,
+    static uint32_t go(const Tree& B, HostVec<lrt_bvh_node_pair>& out, int32_t node, uint32_t base,
                        uint32_t parentEsc, LeafWord& lw)
     {
       const BNode& n = B.nodes[node];
@@ -498,6 +498,64 @@ bool need_normal(const lrt_preset& p)
 
 } // namespace
 
+namespace {
+
+constexpr size_t kParallelPairs = 1u << 15;
+
+// The checks of validate's walk over geometry g's BLAS on all cores: from the
+// root breadth first until there are subtrees for every core, then each
+// subtree by itself.  A pair reached twice (by whichever core comes second),
+// an index out of range or a depth over the bound gives false, and validate's
+// own walk then says which.
+bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVec<uint32_t>& pairGeom,
+               uint32_t& maxDepth)
+{
+  typedef std::pair<uint32_t, uint32_t> Item; // pair, depth
+  const uint64_t P = h.allNodePairs.size(), base = h.geomData[g].bvhOffset;
+  // marks the pair and puts its inner children into `out`
+  auto visit = [&](const Item& it, std::vector<Item>& out) {
+    const uint64_t abs = base + it.first;
+    if (it.second > 4096 || abs >= P) return false;
+    if (__atomic_exchange_n(&pairGeom[abs], g, __ATOMIC_RELAXED) != ~0u) return false;
+    const lrt_bvh_node* ch[2] = {&h.allNodePairs[abs].left, &h.allNodePairs[abs].right};
+    for (int j = 0; j < 2; j++) {
+      const uint32_t lo = ch[j]->leftOffset;
+      if (lo & kLeafBit) {
+        if (lo != kLeafNormal && uint64_t(a0) + (lo & kStartMask) >= a1) return false;
+      } else {
+        if (lo <= it.first) return false;
+        out.push_back({lo, it.second + 1});
+      }
+    }
+    return true;
+  };
+  std::vector<Item> level{{0u, 1u}};
+  bool ok = true;
+  uint32_t deepest = 0;
+  while (ok && !level.empty() && level.size() < 512) {
+    std::vector<Item> next;
+    for (const Item& it : level) {
+      deepest = std::max(deepest, it.second);
+      ok = ok && visit(it, next);
+    }
+    level.swap(next);
+  }
+#pragma omp parallel for schedule(dynamic, 1) reduction(max : deepest) reduction(&& : ok)
+  for (size_t i = 0; i < level.size(); i++) {
+    std::vector<Item> todo{level[i]};
+    while (ok && !todo.empty()) {
+      const Item it = todo.back();
+      todo.pop_back();
+      deepest = std::max(deepest, it.second);
+      ok = visit(it, todo);
+    }
+  }
+  maxDepth = deepest;
+  return ok;
+}
+
+} // namespace
+
 // ---------------------------------------------------------------------------
 // Structural validation: every index the kernels follow is in bounds, every
 // tree pointer points forward (so the stackless TLAS loop and the BLAS loop
@@ -568,7 +626,9 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
     I.hasSbsNeighbours = c.hasSbsNeighbours;
   }
   const size_t P = geomChecked ? 0 : h.allNodePairs.size();
-  std::vector<uint32_t> pairGeom(P, ~0u);
+  HostVec<uint32_t> pairGeom(P);
+#pragma omp parallel for schedule(static)
+  for (size_t i = 0; i < P; i++) pairGeom[i] = ~0u;
   for (size_t g = 0; g < G && !geomChecked; g++) {
     const lrt_geom_data& gd = h.geomData[g];
     const uint32_t tag = h.geomTags[g];
@@ -579,7 +639,14 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
     // BLAS: walk the pairs reachable from the root, checking forward pointers
     // and leaf ids, and measure depth.
     uint32_t maxDepth = 0;
-    std::vector<std::pair<uint32_t, uint32_t>> st{{0u, 1u}};
+    // The largest trees are walked by all cores first; only if that finds the
+    // tree sound (it marks every pair it reaches) is the walk below left out.
+    const bool sound = P >= kParallelPairs && walk_blas(h, uint32_t(g), a0, a1, pairGeom, maxDepth);
+    if (P >= kParallelPairs && !sound)
+      for (size_t i = 0; i < P; i++)
+        if (pairGeom[i] == uint32_t(g)) pairGeom[i] = ~0u;
+    std::vector<std::pair<uint32_t, uint32_t>> st;
+    if (!sound) st.push_back({0u, 1u});
     while (!st.empty()) {
       const auto [k, dpt] = st.back();
       st.pop_back();
@@ -609,7 +676,21 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
       I.hasTriangles = true;
       if (gd.type != LRT_TYPE_MESH_TRIANGLE) return fail(s, LRT_ERR_BAD_SCENE, "triangle geometry %zu has type %u", g, gd.type);
       if (gd.offset[0] % 3 != 0) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu index offset not a multiple of 3", g);
+      // all cores first; only a leaf that fails is looked for again, in order
+      bool sound2 = true;
+      const uint64_t nidx = h.indices.size(), nprim = h.primIndices.size(), nvert = h.vertPos.size() / 4;
+#pragma omp parallel for schedule(static) reduction(&& : sound2)
       for (uint32_t a = a0; a < a1; a++) {
+        const uint32_t pk = h.primIdCount[a];
+        const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
+        if (cnt && (uint64_t(gd.offset[0]) + (st0 + cnt) * 3 > nidx || uint64_t(gd.offset[0]) / 3 + st0 + cnt > nprim)) {
+          sound2 = false;
+          continue;
+        }
+        for (uint64_t q = 3 * st0; q < 3 * (st0 + cnt); q++)
+          sound2 = sound2 && uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + q] < nvert;
+      }
+      for (uint32_t a = a0; a < a1 && !sound2; a++) {
         const uint32_t pk = h.primIdCount[a];
         const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
         const uint64_t lastIdx = uint64_t(gd.offset[0]) + (st0 + cnt) * 3;
@@ -879,10 +960,12 @@ lrt_status lrt_add_geom_triangles3f(lrt_scene* s, const float* vpos, size_t nver
   h.geomTags.push_back(LRT_TAG_TRIANGLE);
 
   const size_t nt = nidx / 3;
-  std::vector<Aabb> boxes(nt);
   const float* V = h.vertPos.data() + 4 * oldV;
+  // (the device builder makes the boxes itself)
+  const bool onDevice = (flags & LRT_BUILD_LOW) && nt > s->primsInLeaf;
+  std::vector<Aabb> boxes(onDevice ? 0 : nt);
 #pragma omp parallel for schedule(static)
-  for (size_t t = 0; t < nt; t++) {
+  for (size_t t = 0; t < boxes.size(); t++) {
     boxes[t].reset();
     for (int c = 0; c < 3; c++) {
       const float* p = V + 4 * size_t(tri[3 * t + c]);
@@ -912,14 +995,18 @@ lrt_status lrt_add_geom_triangles3f(lrt_scene* s, const float* vpos, size_t nver
     // also emits the pairs, leaf table and triangle order (lbvh_build_blas:
     // the arrays the host emitter makes from the same tree)
     const char* err = nullptr;
-    if (nt > s->primsInLeaf) {
+    if (onDevice) {
       static_assert(sizeof(LbvhPairOut) == sizeof(lrt_bvh_node_pair), "a pair is 64 bytes");
       const size_t base = h.allNodePairs.size();
       err = lbvh_build_blas(
-          reinterpret_cast<const float*>(boxes.data()), uint32_t(nt), s->primsInLeaf,
+          V, uint32_t(nvert), tri, uint32_t(nt), s->primsInLeaf,
           [&](size_t count) {
             h.allNodePairs.resize(base + count);
-            return reinterpret_cast<LbvhPairOut*>(h.allNodePairs.data() + base);
+            lrt_bvh_node_pair* p = h.allNodePairs.data() + base;
+            // page the new memory in by all cores (64 pairs to a page)
+#pragma omp parallel for schedule(static)
+            for (size_t i = 0; i < count; i += 64) *reinterpret_cast<volatile char*>(p + i) = 0;
+            return reinterpret_cast<LbvhPairOut*>(p);
           },
           startCount, reordered);
       if (err) h.allNodePairs.resize(base);

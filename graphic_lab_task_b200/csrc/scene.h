@@ -7,8 +7,11 @@
 // `dev` (device.cu).
 #pragma once
 #include <cstdint>
-#include <string>
 #include <map>
+#include <memory>
+#include <new>
+#include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/lrt_b200.h"
@@ -18,16 +21,38 @@ namespace lrt {
 
 struct DeviceScene; // device.cu
 
+// A vector whose resize leaves new elements uninitialised: the large arrays are
+// written right after they are sized, by all cores or by a copy from the
+// device, and zero-filling them first takes one core through every page.
+template <class T>
+struct NoInit : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    typedef NoInit<U> other;
+  };
+  template <class U>
+  void construct(U*) noexcept
+  {
+  }
+  template <class U, class... A>
+  void construct(U* p, A&&... a)
+  {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+  }
+};
+template <class T>
+using HostVec = std::vector<T, NoInit<T>>;
+
 struct HostArrays {
   std::vector<lrt_bvh_node> nodesTLAS;
-  std::vector<lrt_bvh_node_pair> allNodePairs;
+  HostVec<lrt_bvh_node_pair> allNodePairs;
   std::vector<lrt_instance_data> instanceData;
   std::vector<lrt_geom_data> geomData;
   std::vector<uint32_t> geomTags;
   std::vector<uint32_t> startEnd; // uint2 pairs, flattened
   std::vector<uint32_t> primIdCount;
-  std::vector<uint32_t> indices;
-  std::vector<float> vertPos; // float4 per vertex, flattened
+  HostVec<uint32_t> indices;
+  HostVec<float> vertPos; // float4 per vertex, flattened
   std::vector<uint32_t> primIndices;
   std::vector<lrt_bvh_node> origNodes;
   std::vector<lrt_sdf_frame_octree_node> sdfFrameOctreeNodes;
@@ -74,7 +99,7 @@ struct lrt_scene {
   uint64_t uploadedGeomVersion = 0;
   uint64_t validatedGeomVersion = 0; // geometry arrays last passed validation at this version
   lrt::SceneInfo geomInfo;           // what that validation found
-  std::vector<uint32_t> pairGeom;    // and the geometry whose BLAS holds each node pair (~0u: none)
+  lrt::HostVec<uint32_t> pairGeom;   // and the geometry whose BLAS holds each node pair (~0u: none)
   lrt::SceneInfo info;
   lrt::DeviceScene* dev = nullptr;
   int device = -1;
