@@ -70,11 +70,10 @@ inline __host__ __device__ uint64_t sched_words(uint64_t tiles)
 // deferred SBS hit colour (object-space hit point, brick node index).
 constexpr uint32_t kNormalWords = 16;
 constexpr uint32_t kColourWord = 12;
-// Dynamic shared memory of a trace kernel with stack_cap stack entries per thread.
-constexpr size_t trace_smem_bytes(uint32_t stack_cap)
-{
-  return size_t(stack_cap + kNormalWords) * kTraceThreads * sizeof(uint32_t);
-}
+// After them, in the brick kernels for many waves, the ray's origin and
+// direction: they are only read when an instance is entered, and out of the
+// march's registers they let 7 blocks per SM run with few spills.
+constexpr uint32_t kRayWord = 16, kRayWords = 6;
 constexpr uint32_t kMaxStackDev = 80; // STACK_SIZE of raytrace_common.h:36
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kMaxVoxelSteps = 4096u; // voxel-march cap per brick (the reference loop is unbounded)
@@ -177,6 +176,15 @@ constexpr uint32_t kPrefetchChunk = 4096; // bytes per prefetch instruction
 // their own.
 constexpr uint32_t kKindTriangles = 1, kKindNodes = 2; // triangles; frame-octree and SVS nodes
 constexpr uint32_t kKindBricks = 4, kKindNoBricks = kKindTriangles | kKindNodes, kKindAll = 7;
+
+// Dynamic shared memory of a trace kernel with stack_cap stack entries per
+// thread; sharedRay: with the words of kRayWord.
+constexpr size_t trace_smem_bytes(uint32_t stack_cap, bool sharedRay = false)
+{
+  return size_t(stack_cap + kNormalWords + (sharedRay ? kRayWords : 0u)) * kTraceThreads * sizeof(uint32_t);
+}
+// What any of them may ask for.
+constexpr size_t kMaxTraceSmem = trace_smem_bytes(kMaxStackDev + 1, true);
 
 struct DevNode { // a node record
   float4 a, b;

@@ -62,6 +62,7 @@ struct Hit {
 // Measured (us; 5 / 6 / 8 blocks of 128 threads = 96 / 80 / 64 registers):
 //   bricks: 512^3 model at 1920x1080 493 / 503 / -, fused render 382 / 402 / -,
 //     64 cameras (51 M rays) 13,319 / 12,546 / -, Lambert step 3,429 / 3,254 / -
+//     (these two with the ray in shared memory run 7 blocks: shared_ray)
 //   no bricks: 4096^2 instanced primary rays - / 5,737 / 5,573, sorted bounce
 //     - / 6,211 / 5,940, a 200k-triangle mesh at 256^2 - / 102 / 108, a voxel
 //     set at 1001x777 (ANALYTIC) - / 290 / 311
@@ -70,8 +71,14 @@ constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
 constexpr int kManyWaves = 12;       // k_trace takes the kernel for many from here on
 constexpr int min_blocks(uint32_t kind, int size)
 {
-  return kind == kKindBricks ? (size == kMany ? 6 : 5) : kind == kKindNoBricks ? (size == kMany ? 8 : 6) : 5;
+  return kind == kKindBricks ? (size == kMany ? 7 : 5) : kind == kKindNoBricks ? (size == kMany ? 8 : 6) : 5;
 }
+
+// The brick kernels for many waves keep the ray in shared memory: at 80
+// registers (6 blocks) with it in registers 64 cameras took 12,556 us and a
+// Lambert step 2,684; from shared memory 12,357 and 2,671, and at 72 (7 blocks)
+// 12,189 and 2,603.  Frames gain nothing (fused render 377 -> 384).
+constexpr bool shared_ray(uint32_t kind) { return kind == kKindBricks; }
 
 // f(std::integral_constant<uint32_t, kind>) for a scene's kernel kind.
 template <class F>
@@ -87,8 +94,9 @@ auto with_kind(uint32_t kind, F f)
 // there); the plain trace kernel instantiates none.  nrec points at this thread's
 // kNormalWords shared-memory words (thread-strided), where a sphere-traced
 // hit leaves what its normal is computed from once the traversal has ended.
-template <bool COUNT, bool RECORD = false, bool SOLVERS = false, uint32_t KIND = kKindAll>
+template <bool COUNT, bool RECORD = false, bool SOLVERS = false, uint32_t KIND = kKindAll, bool SHARED_RAY = false>
 struct Ctx {
+  static constexpr bool kSharedRay = SHARED_RAY; // the ray is in the words of kRayWord
   static constexpr uint32_t kKind = KIND;
   static constexpr bool kCount = COUNT;
   static constexpr bool kRecord = RECORD;
@@ -876,7 +884,7 @@ __device__ __forceinline__ void tlas_walk(CTX& c, f3 pos, f3 inv, float tmin, fl
 // The order of node, leaf and instance visits is that of the reference's
 // nested loops, so every comparison and every hit is the same.
 struct Walk {
-  f3 pos, dir;       // the ray
+  f3 pos, dir;       // the ray (unless kSharedRay: kRayWord)
   float tmin;
   f3 rp, rd, inv;    // the ray in the current instance's space, inv = SafeInverse(rd)
   Hit hit;
@@ -889,13 +897,21 @@ struct Walk {
 // What the ray does next.
 constexpr uint32_t kRayDone = 1, kRayTlas = 2, kRayBlas = 3;
 
-__device__ __forceinline__ void walk_begin(Walk& w, float4 pn, float4 df)
+template <class CTX>
+__device__ __forceinline__ void walk_begin(CTX& c, Walk& w, float4 pn, float4 df)
 {
   float dirW = df.w;
   w.stopOnFirst = (dirW <= 0.0f);
   if (w.stopOnFirst) dirW *= -1.0f;
-  w.pos = mk3(pn.x, pn.y, pn.z);
-  w.dir = mk3(df.x, df.y, df.z);
+  if constexpr (CTX::kSharedRay) {
+    const uint32_t st = blockDim.x;
+    float* rw = c.nrec + kRayWord * st;
+    rw[0] = pn.x, rw[st] = pn.y, rw[2 * st] = pn.z;
+    rw[3 * st] = df.x, rw[4 * st] = df.y, rw[5 * st] = df.z;
+  } else {
+    w.pos = mk3(pn.x, pn.y, pn.z);
+    w.dir = mk3(df.x, df.y, df.z);
+  }
   w.tmin = pn.w;
   w.hit.t = dirW;
   w.hit.primId = 0xFFFFFFFFu;
@@ -912,21 +928,31 @@ template <class CTX>
 __device__ __forceinline__ uint32_t walk_tlas(CTX& c, Walk& w, uint32_t* stack)
 {
   const DevScene& S = c.S;
-  const f3 inv = safe_inverse(w.dir);
-  const bool fast = fast_nodes(S, w.pos, w.dir, inv);
+  f3 pos, dir;
+  if constexpr (CTX::kSharedRay) {
+    const uint32_t st = blockDim.x;
+    const float* rw = c.nrec + kRayWord * st;
+    pos = mk3(rw[0], rw[st], rw[2 * st]);
+    dir = mk3(rw[3 * st], rw[4 * st], rw[5 * st]);
+  } else {
+    pos = w.pos;
+    dir = w.dir;
+  }
+  const f3 inv = safe_inverse(dir);
+  const bool fast = fast_nodes(S, pos, dir, inv);
   uint32_t travFlags = 0, leftOffset = 0;
   if (fast)
-    tlas_walk<true>(c, w.pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
+    tlas_walk<true>(c, pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
   else
-    tlas_walk<false>(c, w.pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
+    tlas_walk<false>(c, pos, inv, w.tmin, w.hit.t, w.nodeIdx, travFlags, leftOffset);
   // without a leaf the walk has reached the end of the escape chain
   if (travFlags != (kLeafBit | 1u)) return kRayDone;
   w.instId = leftOffset & 0x0FFFFFFFu;
   const DevInstance& I = S.instances[w.instId];
   c.inc(kCntInstances);
   w.geomId = I.geomId;
-  w.rp = matmul4(I.transformInv, w.pos, 1.0f);
-  w.rd = matmul4(I.transformInv, w.dir, 0.0f);
+  w.rp = matmul4(I.transformInv, pos, 1.0f);
+  w.rd = matmul4(I.transformInv, dir, 0.0f);
   w.inv = safe_inverse(w.rd);
   w.fast = fast_nodes(S, w.rp, w.rd, w.inv);
   w.top = 0;
@@ -1012,7 +1038,7 @@ __device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap
                           lrt_hit& hit)
 {
   Walk w;
-  walk_begin(w, pn, df);
+  walk_begin(c, w, pn, df);
   while (walk_tlas(c, w, stack) == kRayBlas) {
     uint32_t next;
     do {
@@ -1695,7 +1721,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_trac
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, shape.stackCap));
+  Ctx<false, false, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, shape.stackCap));
   for (;;) {
     unsigned long long tile = 0;
     if (lane == 0) tile = atomicAdd(work_counter, 1ull);
@@ -1739,13 +1765,13 @@ cudaError_t launch_trace_cameras(const DevScene& S, const DevBatchCamera* cams, 
                                  uint32_t* err_word, int blocks, cudaStream_t stream, const DevLights* lights,
                                  uint32_t* image)
 {
-  const size_t smem = trace_smem_bytes(shape.stackCap);
+  const size_t smem = trace_smem_bytes(shape.stackCap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     if (image) {
       cudaError_t e = cudaFuncSetAttribute(k_trace_cameras<true, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(trace_smem_bytes(kMaxStackDev + 1)));
+                                           int(kMaxTraceSmem));
       if (e != cudaSuccess) return e;
       k_trace_cameras<true, K><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
                                                                    err_word, *lights, image);
@@ -1763,7 +1789,7 @@ cudaError_t set_cameras_smem(uint32_t kind)
 {
   return with_kind(kind, [&](auto k) {
     return cudaFuncSetAttribute(k_trace_cameras<false, decltype(k)::value>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(trace_smem_bytes(kMaxStackDev + 1)));
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxTraceSmem));
   });
 }
 
@@ -2058,7 +2084,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_rend
     wc->longest = 0;
     wc->busy = 0;
   }
-  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, stack_cap));
   const f3 L = mk3(light.x, light.y, light.z);
   uint64_t i = 0;
   bool valid = false;
@@ -2113,7 +2139,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
     if (!valid) continue;
     const float dLdI = __ldg(dimage + i);
     if (dLdI == 0.0f) continue;
-    Ctx<false, true, false, KIND> c(S, normal_words(smem_stack, stack_cap));
+    Ctx<false, true, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, stack_cap));
     const float4 pn = __ldg(rays + 2 * i), df = __ldg(rays + 2 * i + 1);
     lrt_hit h;
     trace_one(c, stack, blockDim.x, stack_cap, pn, df, h);
@@ -2176,7 +2202,7 @@ cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const D
     const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
     auto kernel = modes ? k_render_rgba8<true, K> : k_render_rgba8<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+                                         int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
     DevRenderModes one{};
     one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
@@ -2196,7 +2222,7 @@ cudaError_t launch_outline_fill(const DevScene& S, const DevCamera& cam, const D
     constexpr uint32_t K = decltype(kind)::value;
     const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
     cudaError_t e = cudaFuncSetAttribute(k_outline_fill<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+                                         int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
     k_outline_fill<K><<<grid, kTraceThreads, trace_smem_bytes(stack_cap), stream>>>(
         S, cam, lights, M, RM, smp, tm, col, work_counter, err_word, stack_cap, sched_rd, sched_wr);
@@ -2223,7 +2249,7 @@ cudaError_t launch_fill_gbuffer_transparency(const DevScene& S, const DevCamera&
     constexpr uint32_t K = decltype(kind)::value;
     const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
     cudaError_t e = cudaFuncSetAttribute(k_fill_gbuffer_transparency<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+                                         int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
     k_fill_gbuffer_transparency<K><<<grid, kTraceThreads, smem, stream>>>(S, cam, M, transparency, gbuffer, work_counter,
                                                                        err_word, stack_cap, sched_rd, sched_wr);
@@ -2239,13 +2265,13 @@ cudaError_t launch_render_lambert(const DevScene& S, const float4* rays, uint64_
                                   cudaStream_t stream, uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd,
                                   uint32_t* sched_wr)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
+  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     auto kernel = img_w ? k_render_lambert<true, K> : k_render_lambert<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+                                         int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
     kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
                                                   img_h, sched_rd, sched_wr);
@@ -2258,13 +2284,13 @@ cudaError_t launch_adjoint_lambert(const DevScene& S, const float4* rays, uint64
                                    uint32_t* err_word, uint32_t stack_cap, int blocks, cudaStream_t stream,
                                    uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
+  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     auto kernel = img_w ? k_adjoint_lambert<true, K> : k_adjoint_lambert<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(trace_smem_bytes(kMaxStackDev + 1)));
+                                         int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
     kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
                                                   img_w, img_h, sched_rd, sched_wr);
