@@ -30,21 +30,23 @@ struct Counters {
   uint32_t c[LRT_COUNTER_COUNT];
 };
 
-// What the adjoint needs about the final hit when it lies on an indexed SBS
-// brick: the 8 corner values and their indices in the float value array,
-// the voxel-local hit point, the object-space direction and the voxel size.
-struct HitRecord {
-  float t;          // hit.t when recorded (the record is valid iff it equals the final hit.t)
-  float values[8];
-  uint32_t idx[8];
-  f3 p;
-  f3 dir;
-  float d;
-  bool sbs;         // set by octree_brick for the indexed layouts
-  bool early;       // the field was already <= EPS where the ray entered the
-                    // voxel: the hit is that entry point, which does not move
-                    // with the values (no dt/dtheta term)
-};
+// What the adjoint needs about the final hit on an indexed SBS brick beyond
+// the words the deferred normal and colour leave in shared memory: RECORD
+// kernels keep it in the word of the normal's sign.  (In registers, with the
+// corner values and their indices, the record made the adjoint spill 306 bytes
+// per thread: 1,312 -> 1,192 us for 16 views of 512^2.)  Bits 0-1: the sign (1,
+// 0, or 2 for -1); bit 2: early, the field was already <= EPS where the ray
+// entered the voxel, so that the hit does not move with the values; bits 3-14:
+// the voxel in its brick, 4 bits per axis.
+__device__ __forceinline__ float record_word(float sign, bool early)
+{
+  return __uint_as_float((sign < 0.0f ? 2u : sign > 0.0f ? 1u : 0u) | (early ? 4u : 0u));
+}
+__device__ __forceinline__ float record_sign(float w)
+{
+  const uint32_t b = __float_as_uint(w) & 3u;
+  return b == 2u ? -1.0f : float(b);
+}
 
 // The nearest hit while a ray is being traversed: lrt_hit without the words
 // that are only written once the traversal has ended (finish_hit).  u, v are a
@@ -106,15 +108,10 @@ struct Ctx {
   Counters cnt;
   uint32_t err;
   uint32_t triLocal; // a triangle hit's primId before the m_primIndices remap (its triSoup record)
-  HitRecord rec;
   __device__ Ctx(const DevScene& s, float* normal_rec) : S(s), nrec(normal_rec), err(0)
   {
 #pragma unroll
     for (int i = 0; i < LRT_COUNTER_COUNT; i++) cnt.c[i] = 0;
-    if (RECORD) {
-      rec.t = -1.0f;
-      rec.sbs = false;
-    }
   }
   __device__ __forceinline__ void inc(int k, uint32_t v = 1)
   {
@@ -139,7 +136,7 @@ __device__ __forceinline__ f2 deferred_normal(CTX& c, uint32_t instId)
   const DevScene& S = c.S;
   const uint32_t st = blockDim.x;
   const float* w = c.nrec;
-  const float start_sign = w[0];
+  const float start_sign = CTX::kRecord ? record_sign(w[0]) : w[0];
   const f3 q = mk3(w[st], w[2 * st], w[3 * st]);
   f3 norm;
   if (S.flags & kFlagBBoxMode) { // every hit is an early hit in this mode
@@ -424,27 +421,17 @@ __device__ __forceinline__ void local_surface(CTX& c, uint32_t type, f3 ray_dir,
     // The normal is evaluated once the traversal has ended (finish_hit), from
     // what it depends on, kept here: lanes whose hits are found in different
     // iterations of the surrounding loops then compute their normals together.
-    if (S.flags & kFlagNeedNormal) {
+    if (CTX::kRecord || (S.flags & kFlagNeedNormal)) {
       const uint32_t st = blockDim.x;
       // the sample point: start_q itself for the BBOX mode's early hits
       const f3 q = (S.flags & kFlagBBoxMode) ? start_q : start_q + t * ray_dir;
-      c.nrec[0] = start_sign;
+      c.nrec[0] = CTX::kRecord ? record_word(start_sign, early_hit) : start_sign;
       c.nrec[st] = q.x;
       c.nrec[2 * st] = q.y;
       c.nrec[3 * st] = q.z;
 #pragma unroll
       for (int i = 0; i < 8; i++) c.nrec[(4 + i) * st] = values[i];
       c.inc(kCntNormals);
-    }
-    if (CTX::kRecord) {
-      c.rec.t = tReal;
-#pragma unroll
-      for (int i = 0; i < 8; i++) c.rec.values[i] = values[i];
-      c.rec.p = start_q + t * ray_dir;
-      c.rec.dir = ray_dir;
-      c.rec.d = d;
-      c.rec.sbs = false; // octree_brick marks its own hits
-      c.rec.early = early_hit;
     }
     hit.t = tReal;
     hit.primId = (S.flags & kFlagStIterations) ? iter : primId;
@@ -594,16 +581,8 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
     if (found) {
       local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, 0.0f, qFar, fNearFar, start_q, start_sign,
                     start_dist, hit);
-      if (CTX::kRecord && hit.t < old_t && sb.colorLayout) {
-        // indices of the 8 corner values in the float array (indexed layouts)
-        const uint32_t V = sb.vsize, P = sb.pad;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const uint32_t vId = ((vx + ((i & 4) >> 2) + P) * V + (vy + ((i & 2) >> 1) + P)) * V + (vz + (i & 1) + P);
-          c.rec.idx[i] = __ldg(S.sbsData + node.z + vId);
-        }
-        c.rec.sbs = true;
-      }
+      if (CTX::kRecord && hit.t < old_t)
+        c.nrec[0] = __uint_as_float(__float_as_uint(c.nrec[0]) | (vx << 3) | (vy << 7) | (vz << 11));
     }
   }
   if (hit.t < old_t && sb.colorLayout) {
@@ -2144,11 +2123,21 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
     lrt_hit h;
     trace_one(c, stack, blockDim.x, stack_cap, pn, df, h);
     err |= c.err;
-    if (h.primId == 0xFFFFFFFFu || !c.rec.sbs || c.rec.t != h.t) continue;
+    if (h.primId == 0xFFFFFFFFu) continue;
+    const DevGeom& geom = S.geoms[h.geomId & 0x00FFFFFFu];
+    if (geom.tag != LRT_TAG_SDF_BRICK || !S.sbs[geom.sdfId].colorLayout) continue;
     if (lambert(h, mk3(df.x, df.y, df.z), L) <= 0.0f) continue; // max(0, .) is flat there
-    const HitRecord& r = c.rec;
+    // the hit's record: corner values, voxel-local point, voxel and brick
+    const uint32_t st = blockDim.x;
+    const float* w = c.nrec;
+    const uint32_t rec = __float_as_uint(w[0]);
+    const bool early = rec & 4u;
+    const f3 p = mk3(w[st], w[2 * st], w[3 * st]);
+    float values[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) values[k] = w[(4 + k) * st];
+    const uint32_t nodeId = __float_as_uint(w[(kColourWord + 3) * st]);
     const float* M = S.instances[h.instId].transformInvTransposed;
-    const f3 p = r.p;
     // trilinear gradient and mixed second derivatives at p
     f3 g = mk3(0, 0, 0);
     float hxy = 0, hxz = 0, hyz = 0;
@@ -2156,7 +2145,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
     for (int k = 0; k < 8; k++) {
       const float sx = (k & 4) ? 1.0f : -1.0f, sy = (k & 2) ? 1.0f : -1.0f, sz = (k & 1) ? 1.0f : -1.0f;
       const float wx = (k & 4) ? p.x : 1.0f - p.x, wy = (k & 2) ? p.y : 1.0f - p.y, wz = (k & 1) ? p.z : 1.0f - p.z;
-      const float v = r.values[k];
+      const float v = values[k];
       g = g + v * mk3(sx * wy * wz, wx * sy * wz, wx * wy * sz);
       hxy += v * sx * sy * wz;
       hxz += v * sx * wy * sz;
@@ -2169,19 +2158,24 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
     // u = M^T q (M column-major: M^T q has components dot(column_k, q))
     const f3 u = mk3(M[0] * q.x + M[1] * q.y + M[2] * q.z, M[4] * q.x + M[5] * q.y + M[6] * q.z,
                      M[8] * q.x + M[9] * q.y + M[10] * q.z);
-    const f3 dir = r.dir;
+    const f3 dir = matmul4(S.instances[h.instId].transformInv, mk3(df.x, df.y, df.z), 0.0f);
     const f3 Hd = mk3(hxy * dir.y + hxz * dir.z, hxy * dir.x + hyz * dir.z, hxz * dir.x + hyz * dir.y);
     const float gd = dot(g, dir);
-    if (gd == 0.0f && !r.early) continue;
-    const float uHd = r.early ? 0.0f : dot(u, Hd); // early hits: the hit point is fixed
+    if (gd == 0.0f && !early) continue;
+    // the 8 corners' indices in the float array (x-major grid of the padded brick)
+    const DevSbs& sb = S.sbs[geom.sdfId];
+    const uint32_t V = sb.vsize, P = sb.pad;
+    const uint32_t* corner = S.sbsData + S.sbsNodes[nodeId].data_offset +
+                             (((rec >> 3) & 15u) + P) * V * V + (((rec >> 7) & 15u) + P) * V + ((rec >> 11) & 15u) + P;
+    const float uHd = early ? 0.0f : dot(u, Hd); // early hits: the hit point is fixed
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const float sx = (k & 4) ? 1.0f : -1.0f, sy = (k & 2) ? 1.0f : -1.0f, sz = (k & 1) ? 1.0f : -1.0f;
       const float wx = (k & 4) ? p.x : 1.0f - p.x, wy = (k & 2) ? p.y : 1.0f - p.y, wz = (k & 1) ? p.z : 1.0f - p.z;
       const float w = wx * wy * wz;
       const f3 dw = mk3(sx * wy * wz, wx * sy * wz, wx * wy * sz);
-      const float dI = r.early ? dot(u, dw) : dot(u, dw) - uHd * w / gd;
-      atomicAdd(grad + r.idx[k], dLdI * dI);
+      const float dI = early ? dot(u, dw) : dot(u, dw) - uHd * w / gd;
+      atomicAdd(grad + __ldg(corner + ((k & 4) ? V * V : 0) + ((k & 2) ? V : 0) + (k & 1)), dLdI * dI);
     }
   }
   if (err) atomicOr(err_word, err);
