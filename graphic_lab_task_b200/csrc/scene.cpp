@@ -516,7 +516,8 @@ bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVe
   auto visit = [&](const Item& it, std::vector<Item>& out) {
     const uint64_t abs = base + it.first;
     if (it.second > 4096 || abs >= P) return false;
-    if (__atomic_exchange_n(&pairGeom[abs], g, __ATOMIC_RELAXED) != ~0u) return false;
+    uint32_t none = ~0u; // (a pair of another geometry keeps its owner)
+    if (!__atomic_compare_exchange_n(&pairGeom[abs], &none, g, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED)) return false;
     const lrt_bvh_node* ch[2] = {&h.allNodePairs[abs].left, &h.allNodePairs[abs].right};
     for (int j = 0; j < 2; j++) {
       const uint32_t lo = ch[j]->leftOffset;

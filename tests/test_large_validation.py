@@ -22,7 +22,7 @@ def arrays():
 
 
 @pytest.mark.parametrize("what,message", [
-    ("duplicate", "reached twice"), ("backward", "not a later pair"), ("beyond", "beyond allNodePairs"),
+    ("duplicate", "reached twice"), ("shared", "reached twice"), ("backward", "not a later pair"), ("beyond", "beyond allNodePairs"),
     ("leaf", "outside its"), ("vertex", "vertex beyond vertPos"), ("prims", "triangles beyond indices")])
 def test_faults_are_named(arrays, what, message):
     a = {k: v.copy() for k, v in arrays.items()}
@@ -33,6 +33,9 @@ def test_faults_are_named(arrays, what, message):
     if what == "duplicate":
         first = base + int(inner[len(inner) // 2])
         pairs["left"]["leftOffset"][first] = max(int(pairs["left"]["leftOffset"][first]), k - base + 1)
+    elif what == "shared":  # the small mesh's tree runs into the large one's
+        small = np.nonzero(pairs["left"]["leftOffset"][:base] < 0x80000000)[0]
+        pairs["left"]["leftOffset"][int(small[-1])] = k
     elif what == "backward":
         pairs["left"]["leftOffset"][k] = k - base
     elif what == "beyond":
