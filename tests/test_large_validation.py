@@ -35,7 +35,8 @@ def test_faults_are_named(arrays, what, message):
         pairs["left"]["leftOffset"][first] = max(int(pairs["left"]["leftOffset"][first]), k - base + 1)
     elif what == "shared":  # the small mesh's tree runs into the large one's
         small = np.nonzero(pairs["left"]["leftOffset"][:base] < 0x80000000)[0]
-        pairs["left"]["leftOffset"][int(small[-1])] = k
+        both = (pairs["left"]["leftOffset"][base:] >= 0x80000000) & (pairs["right"]["leftOffset"][base:] >= 0x80000000)
+        pairs["left"]["leftOffset"][int(small[-1])] = base + int(np.nonzero(both)[0][0])
     elif what == "backward":
         pairs["left"]["leftOffset"][k] = k - base
     elif what == "beyond":
