@@ -271,7 +271,8 @@ lrt_status finish(lrt_scene* s, cudaStream_t stream, StreamSlot* slot, bool coun
   return LRT_OK;
 }
 
-// Host-pointer trace of fewer rays than the pipeline takes: the rays are
+// Host-pointer trace of ordinary memory, of fewer rays than the pipeline
+// takes: the rays are
 // copied into page-locked memory, from which the kernel reads them and into
 // which it writes the hits and its error word, so that the call is one launch
 // and one synchronisation.  Device staging took two pageable copies, a memset
@@ -295,6 +296,19 @@ bool host_stage(DeviceScene* d, uint64_t n)
   d->stage = static_cast<unsigned char*>(p);
   d->stageCap = cap;
   return true;
+}
+
+// Ordinary memory, which the caller's thread may read and write at once: a
+// page-locked, managed or device buffer may have work on the stream still to
+// come before it holds the rays, and is copied in stream order.
+bool pageable(const void* p)
+{
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError(); // not sticky: clear it
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
 }
 
 lrt_status trace_host_staged(lrt_scene* s, const float* rays, lrt_hit* hits, uint64_t n, cudaStream_t stream,
@@ -737,7 +751,7 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
       return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot, 8, uint32_t((n + 7) / 8));
     return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot);
   }
-  if (n < kPipeMinRays && !(flags & LRT_TRACE_COUNT_WORK) && host_stage(d, n))
+  if (n < kPipeMinRays && !(flags & LRT_TRACE_COUNT_WORK) && pageable(rays) && pageable(hits) && host_stage(d, n))
     return trace_host_staged(s, rays, hits, n, stream, flags, slot);
   if (n > d->cap) {
     if (d->rays) cudaFree(d->rays);

@@ -37,6 +37,28 @@ def test_staged_sizes_match_device_trace(cuda):
             assert 0.02 < (want["primId"] != MISS).mean() < 1.0
 
 
+def test_page_locked_rays_are_read_in_stream_order(cuda):
+    """Rays that an earlier copy on the stream brings into page-locked memory
+    are traced as they are once that copy has run."""
+    torch = cuda
+    sc = SceneRT()
+    sc.AddInstance(sc.AddGeom_Triangles3f(*wl.noisy_sphere(40, seed=3)), wl.IDENTITY)
+    sc.CommitScene()
+    n = 64 * 64
+    rays = wl.eye_rays_host(wl.camera((0.1, 0.2, 3), width=64, height=64))
+    want = sc.RayQuery_NearestHitBatch(rays)
+    src = torch.from_numpy(rays).cuda()
+    busy = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    host = torch.zeros(n * 8, dtype=torch.float32).pin_memory()
+    hits = torch.zeros(n * 8, dtype=torch.float32).pin_memory()
+    for _ in range(20):
+        busy.add_(1)  # the copy below is still to come when the call is made
+    host.copy_(src.view(-1), non_blocking=True)
+    sc.trace_host(host.data_ptr(), hits.data_ptr(), n)
+    got = hits.numpy().view(HIT_DTYPE).reshape(-1)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+
+
 def test_staged_error_is_reported_once(cuda):
     sc = SceneRT()
     sc.AddInstance(sc.AddGeom_SdfSBS(*wl.sbs_from_spheres(wl.spheres(8, seed=2), grid_res=32)), wl.IDENTITY)
