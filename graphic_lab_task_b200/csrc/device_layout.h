@@ -48,11 +48,10 @@ constexpr uint32_t kSchedWarps = 4;  // header word: warps that reported their b
 constexpr uint32_t kSchedBusy = 6;   // header words 6-7: the sum of those busy times
 constexpr uint32_t kSchedClasses = 3;
 // When the previous launch was tail-bound (its longest tile took longer than
-// its warps were busy on average), each tile of cost class 0 goes out as
-// kSplitParts work items, each traced by one warp on 32 / kSplitParts of the
-// tile's lanes (rows of the 8x4 tile): those tiles are the ones whose rays
-// diverge most, and a warp serialises its lanes' divergent paths.
-constexpr uint32_t kSplitParts = 2;
+// its warps were busy on average), each tile of cost class 0 goes out in parts
+// (split_log2), each traced by one warp on its share of the tile's lanes:
+// those tiles are the ones whose rays diverge most, and a warp serialises its
+// lanes' divergent paths.
 inline __host__ __device__ uint64_t sched_acc_offset(uint64_t tiles) // in words, 8-byte aligned
 {
   return (kSchedHeader + (tiles + 31) / 32 + 1) & ~1ull;

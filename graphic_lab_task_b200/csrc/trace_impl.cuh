@@ -69,11 +69,16 @@ struct Hit {
 //     - / 6,211 / 5,940, a 200k-triangle mesh at 256^2 - / 102 / 108, a voxel
 //     set at 1001x777 (ANALYTIC) - / 290 / 311
 //   all kinds: mixed scene at 1280x720 556 / 577 / 672 (7 blocks)
+//     and its render of all modes, LAMBERT with a transparent mesh, 1,669 /
+//     1,869 / 1,833 / 1,901 in 4 / 5 / 6 / 7 blocks (128 registers and up)
 constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
+constexpr int kModes = 2;            // the render of all modes, samples and transparency
 constexpr int kManyWaves = 12;       // k_trace takes the kernel for many from here on
 constexpr int min_blocks(uint32_t kind, int size)
 {
-  return kind == kKindBricks ? (size == kMany ? 7 : 5) : kind == kKindNoBricks ? (size == kMany ? 8 : 6) : 5;
+  if (kind == kKindBricks) return size == kMany ? 7 : 5;
+  if (kind == kKindNoBricks) return size == kMany ? 8 : 6;
+  return size == kModes ? 4 : 5;
 }
 
 // The brick kernels for many waves keep the ray in shared memory: at 80
@@ -1037,8 +1042,8 @@ __device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap
 // finished, then every other tile in natural order (a bitmap skips the
 // listed ones).  If the previous launch was tail-bound (its longest tile
 // took longer than its warps' mean busy time), a class-0 tile goes out as
-// kSplitParts work items, each traced by one warp on its own rows of the
-// tile; the parts' costs add up in the tile's accumulator and the last part
+// 2, 4 or 8 work items, each traced by one warp on its own rows (or half
+// rows) of the tile; the parts' costs add up in the tile's accumulator and the last part
 // to finish records the tile.  Only which warp traces which ray, and when,
 // depends on it.
 // rd == nullptr: natural order; wr == nullptr: nothing recorded.  Buffer
@@ -1047,7 +1052,8 @@ __device__ void trace_one(CTX& c, uint32_t* stack, uint32_t stride, uint32_t cap
 // registers.
 //
 // A work item is a tile index with, for the part of a split tile, bit 31 set
-// and the part in bits 24..30 (tile counts stay below 2^24).
+// log2 of its parts in bits 28..29 and the part in bits 24..27 (tile counts
+// stay below 2^24).
 struct WarpClock {
   long long start;  // clock64 when the warp took its current item
   uint32_t item;    // that item, ~0u before the first
@@ -1061,10 +1067,10 @@ constexpr uint32_t kItemTileMask = 0x00FFFFFFu;
 __device__ __forceinline__ uint32_t item_tile(uint32_t item) { return item & kItemTileMask; }
 
 // Whether `lane` traces its pixel of the item's tile: every lane for a whole
-// tile, rows part * (32 / kSplitParts) ... of it for a part.
+// tile, its part's share of them for a part.
 __device__ __forceinline__ bool item_has_lane(uint32_t item, uint32_t lane)
 {
-  return !(item & kItemSplit) || lane / (32u / kSplitParts) == ((item >> 24) & 0x7Fu);
+  return !(item & kItemSplit) || lane >> (5u - ((item >> 28) & 3u)) == ((item >> 24) & 0xFu);
 }
 
 // lane 0: records that a tile took `cost` (longest, class list, bitmap).
@@ -1087,13 +1093,36 @@ __device__ __forceinline__ void sched_record(const uint32_t* __restrict__ rd, ui
   }
 }
 
+// In how many parts (log2) the previous launch's class-0 tiles go out, by how
+// far its longest tile outlasted its warps' mean busy time: whole tiles if it
+// did not, else 2, and in scenes without bricks from 2 times on 4 and from 4
+// times on 8 (one row is the least that keeps a part's pixels together).
+// Parts repeat the node loads that a whole tile shares, which a launch that is
+// hardly tail-bound pays for: in 2 / 4 / 8 parts an animated 256-instance frame
+// took 457 / 500 / 588 us, a 200k-triangle mesh at 256^2 in image order 194 /
+// 175 / 128, a voxel set at 1001x777 231 / 193 / 196.  Bricks share most (512^3
+// at 1920x1080 393 / 418 us in 2 / 4 parts), and mixed scenes lose when the
+// schedule comes from another view (1,742 -> 1,913 us in up to 8).
+template <uint32_t KIND>
+__device__ __forceinline__ uint32_t split_log2(const uint32_t* __restrict__ rd)
+{
+  if (!rd) return 0u;
+  const uint64_t span = uint64_t(__ldg(rd)) * __ldg(rd + kSchedWarps);
+  const uint64_t busy = __ldg(reinterpret_cast<const unsigned long long*>(rd + kSchedBusy));
+  if (span <= busy) return 0u;
+  if (KIND != kKindNoBricks) return 1u;
+  return span > 4 * busy ? 3u : span > 2 * busy ? 2u : 1u;
+}
+
 // lane 0, after the warp has finished its current item (if any): records
 // that item's duration and returns the next item of `tiles`, ~0u when none
 // is left.
+template <uint32_t KIND>
 __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, uint32_t* wr, uint32_t tiles,
                                                unsigned long long* counter, WarpClock& wc)
 {
   const uint64_t lists = sched_lists_offset(tiles);
+  const uint32_t lg = split_log2<KIND>(rd), parts = 1u << lg;
   if (wr && wc.item != ~0u) {
     const long long dt = (clock64() - wc.start) >> 4;
     uint32_t cost = uint32_t(dt < 0xFFFFFFFFll ? dt : 0xFFFFFFFFll);
@@ -1101,7 +1130,7 @@ __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, 
     if (wc.item & kItemSplit) { // parts add up; the last one records the tile
       unsigned long long* acc = reinterpret_cast<unsigned long long*>(wr + sched_acc_offset(tiles));
       const unsigned long long prev = atomicAdd(acc + wc.pos, (1ull << 40) | cost);
-      record = (prev >> 40) + 1 == kSplitParts;
+      record = (prev >> 40) + 1 == parts;
       const unsigned long long sum = (prev & ((1ull << 40) - 1)) + cost;
       cost = uint32_t(sum < 0xFFFFFFFFull ? sum : 0xFFFFFFFFull);
     }
@@ -1109,29 +1138,23 @@ __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, 
     if (record) sched_record(rd, wr, tiles, item_tile(wc.item), cost, wc);
   }
   static_assert(kSchedClasses == 3, "three cost classes");
-  static_assert(kSplitParts >= 1 && kSplitParts <= 32 && (32 % kSplitParts) == 0, "parts of a 32-lane tile");
   uint32_t n[3] = {0, 0, 0};
   if (rd)
     for (int c = 0; c < 3; c++) n[c] = min(__ldg(rd + 1 + c), tiles);
   const uint64_t nAll = uint64_t(n[0]) + n[1] + n[2];
-  // class-0 tiles go out in kSplitParts parts if the previous launch was
-  // tail-bound: longest * warps > sum of the warps' busy times
-  const bool tailBound =
-      rd && uint64_t(__ldg(rd)) * __ldg(rd + kSchedWarps) >
-                __ldg(reinterpret_cast<const unsigned long long*>(rd + kSchedBusy));
-  const uint64_t nSplit = tailBound ? n[0] : 0;
-  const uint64_t nItems = nSplit * kSplitParts + (nAll - nSplit);
+  const uint64_t nSplit = lg ? n[0] : 0;
+  const uint64_t nItems = nSplit * parts + (nAll - nSplit);
   for (;;) {
     const unsigned long long k = atomicAdd(counter, 1ull);
     uint32_t item;
     if (k < nItems) {
-      const bool split = k < nSplit * kSplitParts;
-      const uint64_t j = split ? k / kSplitParts : k - nSplit * (kSplitParts - 1);
+      const bool split = k < nSplit * parts;
+      const uint64_t j = split ? k / parts : k - nSplit * (parts - 1);
       const int cls = j < n[0] ? 0 : j < uint64_t(n[0]) + n[1] ? 1 : 2;
       const uint64_t jj = cls == 0 ? j : cls == 1 ? j - n[0] : j - n[0] - n[1];
       const uint32_t tile = __ldg(rd + lists + cls * tiles + jj);
       if (tile >= tiles) continue;
-      item = (split && kSplitParts > 1) ? tile | kItemSplit | (uint32_t(k % kSplitParts) << 24) : tile;
+      item = split ? tile | kItemSplit | (lg << 28) | (uint32_t(k & (parts - 1)) << 24) : tile;
       wc.pos = uint32_t(j);
     } else {
       if (k - nItems >= tiles) { // none left: report this warp's busy time
@@ -1211,7 +1234,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_trace
       __syncwarp();
       uint32_t item = 0;
       if (lane == 0)
-        item = sched_next(sched_rd, sched_wr, uint32_t(tilesX * ((img_h + kImgTileH - 1) / kImgTileH)), work_counter,
+        item = sched_next<KIND>(sched_rd, sched_wr, uint32_t(tilesX * ((img_h + kImgTileH - 1) / kImgTileH)), work_counter,
                           wclock[threadIdx.x >> 5]);
       item = __shfl_sync(0xFFFFFFFFu, item, 0);
       if (item == ~0u) break;
@@ -1794,7 +1817,7 @@ __device__ __forceinline__ float lambert(const lrt_hit& h, f3 dir, f3 L)
 // SDF normals decoded from the hit) and Tonemap (:536-542) into RGBA8.  A warp
 // takes 8x4-pixel tiles from a global counter.
 template <bool MODES, uint32_t KIND>
-__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, MODES ? kModes : kFrame)) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
                                                                 uint32_t* __restrict__ image,
                                                                 unsigned long long* __restrict__ work_counter,
                                                                 uint32_t* __restrict__ err_word, uint32_t stack_cap,
@@ -1816,7 +1839,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_ren
   for (;;) {
     uint32_t item = 0;
     __syncwarp();
-    if (lane == 0) item = sched_next(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
+    if (lane == 0) item = sched_next<KIND>(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
     item = __shfl_sync(0xFFFFFFFFu, item, 0);
     if (item == ~0u) break;
     const uint32_t tile = item_tile(item);
@@ -1900,7 +1923,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_out
   for (;;) {
     uint32_t item = 0;
     __syncwarp();
-    if (lane == 0) item = sched_next(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
+    if (lane == 0) item = sched_next<KIND>(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
     item = __shfl_sync(0xFFFFFFFFu, item, 0);
     if (item == ~0u) break;
     const uint32_t tile = item_tile(item);
@@ -1985,7 +2008,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_fil
   for (;;) {
     uint32_t item = 0;
     __syncwarp();
-    if (lane == 0) item = sched_next(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
+    if (lane == 0) item = sched_next<KIND>(sched_rd, sched_wr, ntiles, work_counter, wclock[threadIdx.x >> 5]);
     item = __shfl_sync(0xFFFFFFFFu, item, 0);
     if (item == ~0u) break;
     const uint32_t tile = item_tile(item);
@@ -2012,7 +2035,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_fil
 // row-major pixel order and the warp takes its next 8x4-pixel tile from the
 // stream's tile schedule (as k_trace does); otherwise the next 32 rays of n.
 // `valid` is false for the lanes of a tile past the image's edge or past n.
-template <bool IMG>
+template <bool IMG, uint32_t KIND>
 __device__ __forceinline__ bool next_ray(uint64_t n, uint32_t img_w, uint32_t img_h, unsigned long long* counter,
                                          const uint32_t* sched_rd, uint32_t* sched_wr, WarpClock* wc, uint64_t& i,
                                          bool& valid)
@@ -2022,7 +2045,7 @@ __device__ __forceinline__ bool next_ray(uint64_t n, uint32_t img_w, uint32_t im
     const uint32_t tilesX = (img_w + kImgTileW - 1) / kImgTileW;
     __syncwarp();
     uint32_t item = 0;
-    if (lane == 0) item = sched_next(sched_rd, sched_wr, tilesX * ((img_h + kImgTileH - 1) / kImgTileH), counter, *wc);
+    if (lane == 0) item = sched_next<KIND>(sched_rd, sched_wr, tilesX * ((img_h + kImgTileH - 1) / kImgTileH), counter, *wc);
     item = __shfl_sync(0xFFFFFFFFu, item, 0);
     if (item == ~0u) return false;
     const uint32_t tile = item_tile(item);
@@ -2067,7 +2090,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_rend
   const f3 L = mk3(light.x, light.y, light.z);
   uint64_t i = 0;
   bool valid = false;
-  while (next_ray<IMG>(n, img_w, img_h, work_counter, sched_rd, sched_wr, wc, i, valid)) {
+  while (next_ray<IMG, KIND>(n, img_w, img_h, work_counter, sched_rd, sched_wr, wc, i, valid)) {
     if (valid) {
       const float4 pn = __ldg(rays + 2 * i), df = __ldg(rays + 2 * i + 1);
       lrt_hit h;
@@ -2114,7 +2137,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
   uint32_t err = 0;
   uint64_t i = 0;
   bool valid = false;
-  while (next_ray<IMG>(n, img_w, img_h, work_counter, sched_rd, sched_wr, wc, i, valid)) {
+  while (next_ray<IMG, KIND>(n, img_w, img_h, work_counter, sched_rd, sched_wr, wc, i, valid)) {
     if (!valid) continue;
     const float dLdI = __ldg(dimage + i);
     if (dLdI == 0.0f) continue;
@@ -2193,7 +2216,7 @@ cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const D
   const bool modes = rm && (rm->mode != LRT_RENDER_MODE_LAMBERT_NO_TEX || rm->samples != 1 || rm->transparency);
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
+    const int grid = std::min(blocks, min_blocks(K, modes ? kModes : kFrame) * int(S.sms));
     auto kernel = modes ? k_render_rgba8<true, K> : k_render_rgba8<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));

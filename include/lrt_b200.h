@@ -369,8 +369,8 @@ lrt_status lrt_trace_sync(lrt_scene* scene, void* stream, int32_t read_counters)
  * stream starts with the tiles that took at least 1/2, then 1/4, then 1/8 of
  * the longest (the rest follow in row order), so that a few slow tiles do
  * not finish last; when the longest tile took longer than the warps were
- * busy on average, the tiles of the first group are each traced by two warps
- * (two rows of the tile each).  The order never changes a result; the first
+ * busy on average, the tiles of the first group are each traced by 2 to 8 warps
+ * (its pixels shared among them).  The order never changes a result; the first
  * launch of a size on a stream allocates that stream's two schedule buffers
  * (about 36 bytes + 20.1 bytes per tile each).  lrt_render_rgba8,
  * lrt_fill_gbuffer_transparency and the _image forms of the Lambert passes

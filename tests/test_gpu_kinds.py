@@ -79,3 +79,27 @@ def test_reach_test_keeps_every_hit(cuda, surface, noise, distance):
     assert bit_equal(got, want).all(), hit_summary(got, want)
     assert (want["primId"] != MISS).mean() > 0.05
     sc.close()
+
+
+@pytest.mark.parametrize("kind", ["triangles", "nodes", "bricks", "all"])
+@pytest.mark.parametrize("width,height", [(61, 43), (333, 251)])
+def test_split_tiles_of_repeated_frames_match_oracle(cuda, kind, width, height):
+    """Tail-bound frames hand their slowest tiles out in 2, 4 or 8 parts from
+    the third launch on: every pixel of every repeat, and of the fused
+    Lambert image, stays what it was."""
+    torch = cuda
+    sc = _scene(KINDS[kind])
+    rays = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=width, height=height))
+    want = po.port_trace(sc.export_arrays(), rays)
+    for repeat in (3, 4, 7):
+        got = _trace(torch, sc, rays, width, height, False, repeat)
+        assert bit_equal(got, want).all(), (repeat, hit_summary(got, want))
+    r = torch.from_numpy(rays).cuda()
+    image = torch.zeros(len(rays), dtype=torch.float32, device="cuda")
+    shade = po.port_render_lambert(sc.export_arrays(), rays, wl.LIGHT)
+    for _ in range(5):
+        image.zero_()
+        sc.render_lambert(r.data_ptr(), len(rays), wl.LIGHT, image.data_ptr(), image_size=(width, height))
+        sc.sync()
+        assert np.array_equal(image.cpu().numpy(), shade)
+    sc.close()
