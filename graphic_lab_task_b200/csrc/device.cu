@@ -740,7 +740,7 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
     // image-order kernel as an image 8 rays wide, whose 8x4 tiles are the same
     // 32 consecutive rays: the groups are then handed out in the stream's
     // schedule for this ray count (slowest groups first, the slowest split
-    // over two warps when the previous launch was tail-bound).  Traces of
+    // over 2 to 8 warps when the previous launch was tail-bound).  Traces of
     // changing counts keep plain row order and allocate no schedule.
     uint64_t& last = d->lastRays[stream];
     const bool repeat = last == n;
