@@ -80,19 +80,27 @@ __global__ void __launch_bounds__(256) k_node_records(float4* __restrict__ nodes
 
 // {A, B-A, C-A} per reordered triangle slot of one geometry, from the
 // vertices (float4) and indices; IntersectAllTrianglesInLeaf computes exactly
-// these differences (BVH2Common.cpp:1585-1589).
+// these differences (BVH2Common.cpp:1585-1589).  One thread per entry of the
+// geometry's leaf table: the slots that its leaves cover are the ones whose
+// indices validate has checked, and no others are followed (a table may leave
+// gaps, and an entry of no triangles may start anywhere).
 __global__ void __launch_bounds__(256) k_tri_soup(const float4* __restrict__ verts, const uint32_t* __restrict__ indices,
-                                                  uint64_t firstVert, uint64_t base, uint64_t count,
-                                                  float4* __restrict__ soup)
+                                                  const uint32_t* __restrict__ leaves, uint32_t nleaves, uint32_t triBase,
+                                                  uint32_t firstVert, float4* __restrict__ soup)
 {
-  const uint64_t t = uint64_t(blockIdx.x) * 256 + threadIdx.x;
-  if (t >= count) return;
-  const uint32_t* idx = indices + 3 * (base + t);
-  const float4 A = verts[firstVert + idx[0]], B = verts[firstVert + idx[1]], C = verts[firstVert + idx[2]];
-  float4* o = soup + 3 * (base + t);
-  o[0] = make_float4(A.x, A.y, A.z, 0.0f);
-  o[1] = make_float4(__fsub_rn(B.x, A.x), __fsub_rn(B.y, A.y), __fsub_rn(B.z, A.z), 0.0f);
-  o[2] = make_float4(__fsub_rn(C.x, A.x), __fsub_rn(C.y, A.y), __fsub_rn(C.z, A.z), 0.0f);
+  const uint64_t a = uint64_t(blockIdx.x) * 256 + threadIdx.x;
+  if (a >= nleaves) return;
+  const uint32_t entry = leaves[a];
+  const uint64_t first = uint64_t(triBase) + (entry & kStartMask), end = first + ((entry & kSizeMask) >> 28);
+  for (uint64_t t = first; t < end; t++) {
+    const uint32_t* idx = indices + 3 * t;
+    const float4 A = verts[uint64_t(firstVert) + idx[0]], B = verts[uint64_t(firstVert) + idx[1]],
+                 C = verts[uint64_t(firstVert) + idx[2]];
+    float4* o = soup + 3 * t;
+    o[0] = make_float4(A.x, A.y, A.z, 0.0f);
+    o[1] = make_float4(__fsub_rn(B.x, A.x), __fsub_rn(B.y, A.y), __fsub_rn(B.z, A.z), 0.0f);
+    o[2] = make_float4(__fsub_rn(C.x, A.x), __fsub_rn(C.y, A.y), __fsub_rn(C.z, A.z), 0.0f);
+  }
 }
 
 // The records of the few TLAS nodes, made on the host; their leaf words stay.
@@ -463,11 +471,11 @@ lrt_status tri_soup(lrt_scene* s)
   if (e == cudaSuccess) e = cudaMemsetAsync(soup, 0, nslots * 48);
   for (size_t g = 0; g < h.geomData.size() && e == cudaSuccess; g++) {
     if (h.geomTags[g] != LRT_TAG_TRIANGLE) continue;
-    const uint64_t base = h.geomData[g].offset[0] / 3;
-    const uint64_t n = base < nslots ? std::min(triangle_slots(h, g), nslots - base) : 0;
+    const uint32_t a0 = h.startEnd[2 * g], n = h.startEnd[2 * g + 1] - a0;
     if (n == 0) continue;
-    k_tri_soup<<<unsigned((n + 255) / 256), 256>>>(static_cast<const float4*>(verts), static_cast<const uint32_t*>(idx),
-                                                   h.geomData[g].offset[1], base, n, static_cast<float4*>(soup));
+    k_tri_soup<<<unsigned((uint64_t(n) + 255) / 256), 256>>>(
+        static_cast<const float4*>(verts), static_cast<const uint32_t*>(idx), d->S.primIdCount + a0, n,
+        h.geomData[g].offset[0] / 3, h.geomData[g].offset[1], static_cast<float4*>(soup));
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);

@@ -37,8 +37,8 @@ uint64_t triangle_slots(const HostArrays& h, size_t g)
 {
   uint64_t ntri = 0;
   for (uint32_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a++) {
-    const uint32_t pk = h.primIdCount[a];
-    ntri = std::max<uint64_t>(ntri, uint64_t(pk & 0x0FFFFFFFu) + ((pk & 0x70000000u) >> 28));
+    const uint32_t pk = h.primIdCount[a], cnt = (pk & kSizeMask) >> 28;
+    if (cnt) ntri = std::max<uint64_t>(ntri, uint64_t(pk & kStartMask) + cnt);
   }
   return ntri;
 }

@@ -1,0 +1,51 @@
+"""Uploaded leaf tables that leave triangle slots uncovered, against the
+oracle bit for bit."""
+import numpy as np
+import pytest
+
+import pyoracle as po
+from graphic_lab_task_b200 import SceneRT, workloads as wl
+from helpers import MISS, bit_equal, hit_summary
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("meshes", [1, 3])
+@pytest.mark.parametrize("gap", [1, 300])
+def test_uncovered_slots_are_not_followed(cuda, meshes, gap):
+    """Every mesh's leaf ranges leave `gap` triangles uncovered whose indices
+    are far out of range, and its table ends with entries of no triangles that
+    start anywhere."""
+    sc = SceneRT()
+    for k in range(meshes):
+        sc.AddInstance(sc.AddGeom_Triangles3f(*wl.noisy_sphere(12 + k, seed=k)), wl.similarity(0.6, (1.1 * k - 1, 0, 0)))
+    sc.CommitScene(host_only=True)
+    a = {k: v.copy() for k, v in sc.export_arrays().items()}
+    ends = a["startEnd"].reshape(-1, 2)
+    parts = {"indices": [], "primIndices": [], "primIdCount": []}
+    bounds = [int(o) for o in a["geomData"]["offset"][:, 0]] + [len(a["indices"])]
+    for g in range(meshes):
+        leaves = a["primIdCount"][ends[g, 0]:ends[g, 1]]
+        start = leaves & 0x0FFFFFFF
+        cut = int(np.sort(start)[len(start) // 2])  # a leaf starts here
+        leaves = np.where(start >= cut, leaves + gap, leaves).astype(np.uint32)
+        empty = np.array([0x0FFFFFF0, 0x80000000 | 0x0FFFFFFF], np.uint32)
+        idx = a["indices"][bounds[g]:bounds[g + 1]]
+        prim = a["primIndices"][bounds[g] // 3:bounds[g + 1] // 3]
+        bad = np.full(3 * gap, 0xFFFFFFF0, np.uint32)
+        a["geomData"]["offset"][g, 0] = sum(len(x) for x in parts["indices"])
+        parts["indices"] += [idx[:3 * cut], bad, idx[3 * cut:]]
+        parts["primIndices"] += [prim[:cut], bad[:gap], prim[cut:]]
+        ends[g] = [sum(len(x) for x in parts["primIdCount"])] * 2
+        parts["primIdCount"] += [leaves, empty]
+        ends[g, 1] += len(leaves) + 2
+    a["startEnd"] = ends.reshape(a["startEnd"].shape)
+    a.update({k: np.concatenate(v) for k, v in parts.items()})
+    rays = wl.eye_rays_host(wl.camera((0.3, 0.4, 3.5), width=90, height=70))
+    want = po.port_trace(a, rays)
+    sc = SceneRT()
+    sc.upload_arrays(a)
+    got = sc.RayQuery_NearestHitBatch(rays)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+    assert (want["primId"] != MISS).mean() > 0.03
+    sc.close()
