@@ -535,9 +535,18 @@ lrt_status device_upload(lrt_scene* s)
   build_geoms(h, geoms);
   build_sbs_dense(h, sbs, dense);
   build_sbs_masks(h, sbs, dense, mask);
+  uint32_t kinds = 0;
+  for (uint32_t t : h.geomTags)
+    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
+           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
+  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
+  // Only a brick geometry's pairs are pruned.  (SBS arrays that no geometry
+  // names change nothing: the scene's pairs become node records then, of which
+  // there is one copy.)
+  const bool prune = (S.kind & kKindBricks) != 0;
   HostVec<lrt_bvh_node_pair> pruned;
-  if (!h.sdfSBSNodes.empty()) prune_sbs_pairs(h, geoms, sbs, mask, pruned);
-  const HostVec<lrt_bvh_node_pair>& pairs = h.sdfSBSNodes.empty() ? h.allNodePairs : pruned;
+  if (prune) prune_sbs_pairs(h, geoms, sbs, mask, pruned);
+  const HostVec<lrt_bvh_node_pair>& pairs = prune ? pruned : h.allNodePairs;
   lrt_status st = LRT_OK;
 #define UP(dst, vec, T, name)                                                                        \
   if (st == LRT_OK) {                                                                                 \
@@ -545,11 +554,6 @@ lrt_status device_upload(lrt_scene* s)
     st = upload_vec(s, d, reinterpret_cast<const T*>(vec.data()), vec.size() * sizeof(vec[0]) / sizeof(T), &p, name); \
     S.dst = p;                                                                                        \
   }
-  uint32_t kinds = 0;
-  for (uint32_t t : h.geomTags)
-    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
-           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
-  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
   std::vector<lrt_bvh_node> tlas;
   tlas_records(h.nodesTLAS, S.kind == kKindNoBricks, tlas);
   UP(tlas, tlas, DevNode, "TLAS nodes")
@@ -569,8 +573,8 @@ lrt_status device_upload(lrt_scene* s)
   UP(sbsMask, mask, uint32_t, "SBS surface-voxel masks")
   UP(sbs, sbs, DevSbs, "SBS table")
   if (st == LRT_OK) {
-    if (h.sdfSBSNodes.empty()) {
-      d->pairsOrig = S.pairs; // nothing was pruned
+    if (!prune) {
+      d->pairsOrig = S.pairs;
     } else {
       const DevPair* p = nullptr;
       st = upload_vec(s, d, reinterpret_cast<const DevPair*>(h.allNodePairs.data()), h.allNodePairs.size(), &p,
@@ -600,7 +604,7 @@ lrt_status device_upload(lrt_scene* s)
     d->prunePairs = uint32_t(parent.size());
   }
   d->sbsHost = sbs;
-  d->pairsOrigBytes = (h.sdfSBSNodes.empty() ? pairs.size() : h.allNodePairs.size()) * sizeof(lrt_bvh_node_pair);
+  d->pairsOrigBytes = h.allNodePairs.size() * sizeof(lrt_bvh_node_pair);
   // what a traversal reads per node, leaf, brick and voxel, most shared first
   d->pfCand = {{S.tlas, h.nodesTLAS.size() * sizeof(lrt_bvh_node)},
                {S.pairs, pairs.size() * sizeof(lrt_bvh_node_pair)},
