@@ -38,18 +38,19 @@ constexpr uint32_t kImgTileW = 8, kImgTileH = 4;
 
 // Tile schedule of the image-order launches (one per stream and image size,
 // two buffers used alternately): a header {longest tile cost, count of each
-// of the kSchedClasses cost classes, warps of the launch, unused, 64-bit sum
-// of the warps' busy times}, a bitmap of the listed tiles, one 64-bit cost
+// of the kSchedClasses cost classes, warps of the launch, split level, 64-bit
+// sum of the warps' busy times}, a bitmap of the listed tiles, one 64-bit cost
 // accumulator per listed tile (the parts of a split tile add up there), then
 // one list of `tiles` entries per class.  Everything before the lists is
 // cleared before the launch that writes the buffer.  Costs are clock64 / 16.
 constexpr uint32_t kSchedHeader = 8;
 constexpr uint32_t kSchedWarps = 4;  // header word: warps that reported their busy time
+constexpr uint32_t kSchedLevel = 5;  // header word: log2 of the parts that the launch split tiles into
 constexpr uint32_t kSchedBusy = 6;   // header words 6-7: the sum of those busy times
 constexpr uint32_t kSchedClasses = 3;
 // When the previous launch was tail-bound (its longest tile took longer than
 // its warps were busy on average), each tile of cost class 0 goes out in parts
-// (split_log2), each traced by one warp on its share of the tile's lanes:
+// (split_level), each traced by one warp on its share of the tile's lanes:
 // those tiles are the ones whose rays diverge most, and a warp serialises its
 // lanes' divergent paths.
 inline __host__ __device__ uint64_t sched_acc_offset(uint64_t tiles) // in words, 8-byte aligned

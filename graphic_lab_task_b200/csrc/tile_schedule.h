@@ -11,15 +11,15 @@ namespace lrt {
 
 // Longest-first order of the tiles of an image-order launch.  Each launch
 // times its tiles on lane 0 and sorts the slow ones into three classes by
-// their cost against the previous launch's longest tile (at least 1/2, 1/4,
-// 1/8 of it); the next launch of the same image size on the same stream
+// their cost against the previous launch's longest tile (at least 5/8, 3/8,
+// 3/16 of it); the next launch of the same image size on the same stream
 // (rd) hands out class 0, then 1, then 2, each in the order the tiles
 // finished, then every other tile in natural order (a bitmap skips the
 // listed ones).  If the previous launch was tail-bound (its longest tile
 // took longer than its warps' mean busy time), a class-0 tile goes out as
 // 2, 4 or 8 work items, each traced by one warp on its own rows (or half
-// rows) of the tile; the parts' costs add up in the tile's accumulator and the last part
-// to finish records the tile.  Only which warp traces which ray, and when,
+// rows) of the tile; the parts' costs add up in the tile's accumulator and the
+// last part to finish records the tile.  Only which warp traces which ray, and when,
 // depends on it.
 // rd == nullptr: natural order; wr == nullptr: nothing recorded.  Buffer
 // layout: sched_words and the offsets beside it (device_layout.h).  The
@@ -33,6 +33,7 @@ struct WarpClock {
   long long start;  // clock64 when the warp took its current item
   uint32_t item;    // that item, ~0u before the first
   uint32_t longest; // longest tile this warp has reported
+  uint32_t level;   // log2 of the parts that this launch splits tiles into
   uint32_t pos;     // a split item's position in the concatenated class lists
   unsigned long long busy; // sum of the costs of the items this warp traced
 };
@@ -49,8 +50,9 @@ __device__ __forceinline__ bool item_has_lane(uint32_t item, uint32_t lane)
 }
 
 // lane 0: records that a tile took `cost` (longest, class list, bitmap).
+// `listed`, no less than that for a split tile, is what its class goes by.
 __device__ __forceinline__ void sched_record(const uint32_t* __restrict__ rd, uint32_t* wr, uint32_t tiles,
-                                             uint32_t tile, uint32_t cost, WarpClock& wc)
+                                             uint32_t tile, uint32_t cost, uint32_t listed, WarpClock& wc)
 {
   const uint64_t lists = sched_lists_offset(tiles);
   if (cost > wc.longest) {
@@ -59,7 +61,7 @@ __device__ __forceinline__ void sched_record(const uint32_t* __restrict__ rd, ui
   }
   const uint32_t mx = rd ? __ldg(rd) : 0u;
   if (mx) {
-    const int cls = cost >= mx / 2 ? 0 : cost >= mx / 4 ? 1 : cost >= mx / 8 ? 2 : 3;
+    const int cls = listed >= mx / 8 * 5 ? 0 : listed >= mx / 8 * 3 ? 1 : listed >= mx / 16 * 3 ? 2 : 3;
     if (cls < 3) {
       const uint32_t slot = atomicAdd(wr + 1 + cls, 1u);
       if (slot < tiles) wr[lists + cls * tiles + slot] = tile;
@@ -68,25 +70,64 @@ __device__ __forceinline__ void sched_record(const uint32_t* __restrict__ rd, ui
   }
 }
 
-// In how many parts (log2) the previous launch's class-0 tiles go out, by how
-// far its longest tile outlasted its warps' mean busy time: whole tiles if it
-// did not, else 2, and in scenes without bricks from 2 times on 4 and from 4
-// times on 8 (one row is the least that keeps a part's pixels together).
-// Parts repeat the node loads that a whole tile shares, which a launch that is
-// hardly tail-bound pays for: in 2 / 4 / 8 parts an animated 256-instance frame
-// took 457 / 500 / 588 us, a 200k-triangle mesh at 256^2 in image order 194 /
-// 175 / 128, a voxel set at 1001x777 231 / 193 / 196.  Bricks share most (512^3
-// at 1920x1080 393 / 418 us in 2 / 4 parts), and mixed scenes lose when the
-// schedule comes from another view (1,742 -> 1,913 us in up to 8).
+// What a tile traced in 2^lg parts would have cost whole, from the sum of its
+// parts: they repeat the node loads that a whole tile shares, so that the sum
+// grows with the level, by about 1.5 for each (the longest tile's in 2 / 4 / 8
+// parts against whole: a 200k-triangle mesh at 256^2 1.4 / 1.7 / 2.1, at
+// 1920x1080 1.4 / 2.3 / 3.2, voxel sets 1.6 / 2.5 / 4.1 and 1.7 / 3.2 / 5.2,
+// 256 instances 1.4 / 2.1 / 2.8, 512^3 bricks 1.6 / 2.7 / 3.6).  Split levels
+// and the bounds of the classes are of whole tiles' costs: from the plain sums
+// a split tile looked longer than it was and was split further, while the
+// tiles that became slow beside it as the camera moved stayed below its class.
+__device__ __forceinline__ uint32_t whole_cost(uint64_t sum, uint32_t lg)
+{
+  const float whole = float(sum) * (lg == 1 ? 0.6667f : lg == 2 ? 0.4444f : 0.2963f);
+  return whole < 4e9f ? uint32_t(whole) : 4000000000u;
+}
+
+// What a split tile's class goes by: enough of the sum to keep it in class 0
+// (5/8 of the longest) if its parts share nothing, so that a tile whose parts
+// are cheap is not whole again in every other launch.  (The whole sum in 2
+// parts: multi-layer renders of 256^3 bricks at 1920x1080 5,070 -> 5,700 us; 1.25
+// of the whole cost for all: repeated rows of 256 instances 185 -> 206.)
+__device__ __forceinline__ uint32_t listed_cost(uint64_t sum, uint32_t lg)
+{
+  const float cost = float(sum) * (lg == 1 ? 0.8f : lg == 2 ? 0.72f : 0.64f);
+  return cost < 4e9f ? uint32_t(cost) : 4000000000u;
+}
+
+// In how many parts (log2) the class-0 tiles of a launch go out, from the
+// longest tile of the launch before, its warps, their busy time and its level:
+// whole if that tile took no longer than the warps' mean busy time, else 2, and
+// from 2 times on 4 and from 3 times on 8 parts (half rows), as far as `most`.
+// A level is left at half the cost from which it is taken, so that repeated
+// launches settle: the sum's factor differs by half between scenes.
+// Measured in 2 / 4 / 8 parts (us; longest tile in mean busy times): 1.5, 256
+// moving instances 484 / 534 / 558 (whole 575); 1.5, voxel set at 1920x1080
+// 272 / 275 / 302 (278); 2.7, voxel set at 1001x777 284 / 263 / 249 (312);
+// 3.0, mesh at 1920x1080 in rows 307 / 288 / 319 (349); 3.6, 256 instances
+// 251 / 218 / 230 (316); 3.8, mesh at 1920x1080 321 / 270 / 231 (364); 17, mesh
+// at 256^2 198 / 183 / 166 (204).
+inline __host__ __device__ uint32_t split_level(uint32_t was, uint64_t longest, uint64_t warps, uint64_t busy,
+                                                uint32_t most)
+{
+  const uint64_t span = longest * warps;
+  uint32_t lg = 0;
+  while (lg < most && 2 * span > (lg < was ? 1 : 2) * (lg + 1) * busy) lg++;
+  return lg;
+}
+
+// The most parts (log2), by the scene's geometry kind: bricks share most of
+// their loads (512^3 at 1920x1080, camera moving, 451 / 458 / 469 us in 2 / 4 /
+// 8 parts), and mixed scenes lose when the schedule comes from another view
+// (1280x720, two views in turn, 563 / 642 / 643 us).
 template <uint32_t KIND>
 __device__ __forceinline__ uint32_t split_log2(const uint32_t* __restrict__ rd)
 {
   if (!rd) return 0u;
-  const uint64_t span = uint64_t(__ldg(rd)) * __ldg(rd + kSchedWarps);
-  const uint64_t busy = __ldg(reinterpret_cast<const unsigned long long*>(rd + kSchedBusy));
-  if (span <= busy) return 0u;
-  if (KIND != kKindNoBricks) return 1u;
-  return span > 4 * busy ? 3u : span > 2 * busy ? 2u : 1u;
+  return split_level(__ldg(rd + kSchedLevel), __ldg(rd), __ldg(rd + kSchedWarps),
+                     __ldg(reinterpret_cast<const unsigned long long*>(rd + kSchedBusy)),
+                     KIND == kKindNoBricks ? 3u : 1u);
 }
 
 // lane 0, after the warp has finished its current item (if any): records
@@ -97,20 +138,23 @@ __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, 
                                                unsigned long long* counter, WarpClock& wc)
 {
   const uint64_t lists = sched_lists_offset(tiles);
-  const uint32_t lg = split_log2<KIND>(rd), parts = 1u << lg;
+  if (wc.item == ~0u) wc.level = split_log2<KIND>(rd); // the warp's first item
+  const uint32_t lg = wc.level, parts = 1u << lg;
   if (wr && wc.item != ~0u) {
     const long long dt = (clock64() - wc.start) >> 4;
     uint32_t cost = uint32_t(dt < 0xFFFFFFFFll ? dt : 0xFFFFFFFFll);
+    uint32_t listed = cost;
     bool record = true;
     wc.busy += cost;
     if (wc.item & kItemSplit) { // parts add up; the last one records the tile
       unsigned long long* acc = reinterpret_cast<unsigned long long*>(wr + sched_acc_offset(tiles));
       const unsigned long long prev = atomicAdd(acc + wc.pos, (1ull << 40) | cost);
       record = (prev >> 40) + 1 == parts;
-      const unsigned long long sum = (prev & ((1ull << 40) - 1)) + cost;
-      cost = uint32_t(sum < 0xFFFFFFFFull ? sum : 0xFFFFFFFFull);
+      const uint64_t sum = (prev & ((1ull << 40) - 1)) + cost;
+      cost = whole_cost(sum, lg);
+      listed = listed_cost(sum, lg);
     }
-    if (record) sched_record(rd, wr, tiles, item_tile(wc.item), cost, wc);
+    if (record) sched_record(rd, wr, tiles, item_tile(wc.item), cost, listed, wc);
   }
   static_assert(kSchedClasses == 3, "three cost classes");
   uint32_t n[3] = {0, 0, 0};
@@ -136,6 +180,7 @@ __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, 
         if (wr) {
           atomicAdd(reinterpret_cast<unsigned long long*>(wr + kSchedBusy), wc.busy);
           atomicAdd(wr + kSchedWarps, 1u);
+          wr[kSchedLevel] = lg; // (every warp's)
         }
         return wc.item = ~0u;
       }

@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+using std::max;
 using std::min;
 static long long g_clock;
 static long long clock64() { return g_clock; }
@@ -105,23 +106,95 @@ static uint32_t slow_tiles(uint32_t tile, uint32_t lanes)
   return std::max(1u, whole * uint32_t(__builtin_popcount(lanes)) / 32);
 }
 
+// Repeats of one launch: every tile is traced once whatever the level, and the
+// level settles.  Returns it.
 template <uint32_t KIND>
-static void launches(uint32_t tiles, uint32_t warps)
+static uint32_t launches(uint32_t tiles, uint32_t warps, const std::function<uint32_t(uint32_t, uint32_t)>& cost,
+                         long long* spans = nullptr)
 {
   std::vector<uint32_t> prev;
-  for (int k = 0; k < 6; k++) {
-    Launch L = run<KIND>(tiles, warps, prev.empty() ? nullptr : prev.data(), slow_tiles);
+  uint32_t level = 0;
+  for (int k = 0; k < 20; k++) {
+    Launch L = run<KIND>(tiles, warps, prev.empty() ? nullptr : prev.data(), cost);
+    if (k > 8) expect(L.wr[kSchedLevel] == level, "the split level does not settle", L.wr[kSchedLevel], level);
+    level = L.wr[kSchedLevel];
+    const uint32_t most = *std::max_element(L.items.begin(), L.items.end());
+    expect(most <= 1u << level, "more parts than the level's", most, 1u << level);
+    if (spans && (k == 0 || k == 19)) spans[k != 0] = L.span;
     prev = L.wr;
   }
+  return level;
+}
+
+// A launch that starts from a planted level, all tiles listed in class 0.
+template <uint32_t KIND>
+static void planted(uint32_t tiles, uint32_t warps, uint32_t was, uint32_t longest, uint64_t busy, uint32_t want)
+{
+  std::vector<uint32_t> rd(sched_words(tiles), 0u);
+  rd[0] = longest;
+  rd[1] = tiles;
+  rd[kSchedWarps] = warps;
+  rd[kSchedLevel] = was;
+  std::memcpy(&rd[kSchedBusy], &busy, 8);
+  for (uint32_t t = 0; t < tiles; t++) {
+    rd[sched_lists_offset(tiles) + t] = tiles - 1 - t;
+    rd[kSchedHeader + t / 32] |= 1u << (t % 32);
+  }
+  Launch L = run<KIND>(tiles, warps, rd.data(), slow_tiles);
+  expect(L.wr[kSchedLevel] == want, "level after a planted schedule", L.wr[kSchedLevel], want);
+  for (uint32_t t = 0; t < tiles; t++) expect(L.items[t] == 1u << want, "parts of a planted tile", L.items[t], want);
 }
 
 int main()
 {
   for (uint32_t tiles : {1u, 31u, 32u, 300u, 2048u})
     for (uint32_t warps : {1u, 7u, 64u, 600u}) {
-      launches<kKindNoBricks>(tiles, warps);
-      launches<kKindBricks>(tiles, warps);
-      launches<kKindAll>(tiles, warps);
+      launches<kKindNoBricks>(tiles, warps, slow_tiles);
+      launches<kKindBricks>(tiles, warps, slow_tiles);
+      launches<kKindAll>(tiles, warps, slow_tiles);
     }
+  // the slowest tiles take little more than the mean busy time, and their
+  // parts repeat much of what a whole tile shares: from the sums the level
+  // would grow to the most
+  auto shared = [](uint32_t tile, uint32_t lanes) {
+    const uint32_t n = uint32_t(__builtin_popcount(lanes));
+    return tile % 50 == 0 ? 270 + 17 * n : 100u;
+  };
+  long long span[2];
+  uint32_t lg = launches<kKindNoBricks>(2000, 400, shared, span);
+  expect(lg == 1 && span[1] < span[0], "launch whose parts share most of their time", lg, span[1]);
+  lg = launches<kKindNoBricks>(2000, 20, shared, span);
+  expect(lg == 0, "balanced launch", lg);
+  lg = launches<kKindNoBricks>(2048, 2048, slow_tiles, span);
+  expect(lg == 3 && 4 * span[1] < span[0], "launch as long as its slowest tiles", lg, span[1]);
+  // tiles that become slow are split like those that were: the same number
+  // of other tiles is slow in every launch
+  std::vector<uint32_t> prev;
+  for (int k = 0; k < 8; k++) {
+    auto moving = [k](uint32_t tile, uint32_t lanes) {
+      const bool slow = tile % 97 == 5 || tile % 97 == 40 + uint32_t(k) || tile % 97 == 41 + uint32_t(k);
+      return (slow ? 3200u : 64u) * uint32_t(__builtin_popcount(lanes)) / 32 + (slow ? 500u : 0u);
+    };
+    Launch L = run<kKindNoBricks>(970, 500, prev.empty() ? nullptr : prev.data(), moving);
+    if (k > 2) expect(L.items[41 + k] == 1 && L.items[40 + k] == 8, "tile that was slow is not split", k, L.items[40 + k]);
+    prev = L.wr;
+  }
+  // a mean busy time of 100: a level is taken above once, twice and three
+  // times it and left at half of that
+  for (uint32_t was = 0; was < 4; was++) {
+    planted<kKindNoBricks>(100, 10, was, 301, 1000, 3);
+    planted<kKindNoBricks>(100, 10, was, 300, 1000, was == 3 ? 3 : 2);
+    planted<kKindNoBricks>(100, 10, was, 201, 1000, was == 3 ? 3 : 2);
+    planted<kKindNoBricks>(100, 10, was, 150, 1000, was > 1 ? 2 : 1);
+    planted<kKindNoBricks>(100, 10, was, 101, 1000, was > 1 ? 2 : 1);
+    planted<kKindNoBricks>(100, 10, was, 100, 1000, was > 0 ? 1 : 0);
+    planted<kKindNoBricks>(100, 10, was, 51, 1000, was > 0 ? 1 : 0);
+    planted<kKindNoBricks>(100, 10, was, 50, 1000, 0);
+  }
+  for (uint32_t was = 0; was < 2; was++) {
+    planted<kKindAll>(33, 10, was, 900, 1000, 1);
+    planted<kKindBricks>(33, 10, was, 900, 1000, 1);
+    planted<kKindBricks>(33, 10, was, 50, 1000, 0);
+  }
   return failed != 0;
 }

@@ -84,9 +84,9 @@ def test_reach_test_keeps_every_hit(cuda, surface, noise, distance):
 @pytest.mark.parametrize("kind", ["triangles", "nodes", "bricks", "all"])
 @pytest.mark.parametrize("width,height", [(61, 43), (333, 251)])
 def test_split_tiles_of_repeated_frames_match_oracle(cuda, kind, width, height):
-    """Tail-bound frames hand their slowest tiles out in 2, 4 or 8 parts from
-    the third launch on: every pixel of every repeat, and of the fused
-    Lambert image, stays what it was."""
+    """Repeated small frames, whose slowest tiles go out in the parts that the
+    launch before makes of them (planted levels: test_gpu_schedule.py): every
+    pixel of every repeat, and of the fused Lambert image, stays what it was."""
     torch = cuda
     sc = _scene(KINDS[kind])
     rays = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=width, height=height))
