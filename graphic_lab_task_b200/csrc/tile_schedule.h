@@ -26,9 +26,10 @@ namespace lrt {
 // per-warp state lives in shared memory so that the traversal keeps its
 // registers.
 //
-// A work item is a tile index with, for the part of a split tile, bit 31 set
-// log2 of its parts in bits 28..29 and the part in bits 24..27 (tile counts
-// stay below 2^24).
+// A work item is a tile index (below 2^31: more tiles than fit any memory) or
+// the part of a split tile: bit 31, log2 of the parts in bits 28..29, the part
+// in bits 24..27 and the tile below them, so that launches of more than 2^24
+// tiles split none.
 struct WarpClock {
   long long start;  // clock64 when the warp took its current item
   uint32_t item;    // that item, ~0u before the first
@@ -40,7 +41,10 @@ struct WarpClock {
 constexpr uint32_t kItemSplit = 0x80000000u;
 constexpr uint32_t kItemTileMask = 0x00FFFFFFu;
 
-__device__ __forceinline__ uint32_t item_tile(uint32_t item) { return item & kItemTileMask; }
+__device__ __forceinline__ uint32_t item_tile(uint32_t item)
+{
+  return item & kItemSplit ? item & kItemTileMask : item;
+}
 
 // Whether `lane` traces its pixel of the item's tile: every lane for a whole
 // tile, its part's share of them for a part.
@@ -122,9 +126,9 @@ inline __host__ __device__ uint32_t split_level(uint32_t was, uint64_t longest, 
 // 8 parts), and mixed scenes lose when the schedule comes from another view
 // (1280x720, two views in turn, 563 / 642 / 643 us).
 template <uint32_t KIND>
-__device__ __forceinline__ uint32_t split_log2(const uint32_t* __restrict__ rd)
+__device__ __forceinline__ uint32_t split_log2(const uint32_t* __restrict__ rd, uint32_t tiles)
 {
-  if (!rd) return 0u;
+  if (!rd || tiles > kItemTileMask + 1) return 0u;
   return split_level(__ldg(rd + kSchedLevel), __ldg(rd), __ldg(rd + kSchedWarps),
                      __ldg(reinterpret_cast<const unsigned long long*>(rd + kSchedBusy)),
                      KIND == kKindNoBricks ? 3u : 1u);
@@ -138,7 +142,7 @@ __device__ __forceinline__ uint32_t sched_next(const uint32_t* __restrict__ rd, 
                                                unsigned long long* counter, WarpClock& wc)
 {
   const uint64_t lists = sched_lists_offset(tiles);
-  if (wc.item == ~0u) wc.level = split_log2<KIND>(rd); // the warp's first item
+  if (wc.item == ~0u) wc.level = split_log2<KIND>(rd, tiles); // the warp's first item
   const uint32_t lg = wc.level, parts = 1u << lg;
   if (wr && wc.item != ~0u) {
     const long long dt = (clock64() - wc.start) >> 4;

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <queue>
@@ -38,6 +39,7 @@ static int failed = 0;
 static void expect(bool ok, const char* what, long long a = 0, long long b = 0)
 {
   if (ok) return;
+  if (failed > 40) std::exit(1);
   std::printf("%s (%lld, %lld)\n", what, a, b);
   failed++;
 }
@@ -195,6 +197,38 @@ int main()
     planted<kKindAll>(33, 10, was, 900, 1000, 1);
     planted<kKindBricks>(33, 10, was, 900, 1000, 1);
     planted<kKindBricks>(33, 10, was, 50, 1000, 0);
+  }
+  // more tiles than a part's item can number
+  std::vector<uint32_t> head(kSchedHeader, 0u);
+  head[0] = 1000;
+  head[kSchedWarps] = head[kSchedBusy] = 1;
+  const uint32_t many = (1u << 24) + 40;
+  std::vector<uint32_t> rd(sched_words(many), 0u);
+  std::copy(head.begin(), head.end(), rd.begin());
+  rd[1] = 2; // two of them listed
+  rd[sched_lists_offset(many)] = 7;
+  rd[sched_lists_offset(many) + 1] = many - 1;
+  rd[kSchedHeader] = 1u << 7;
+  rd[kSchedHeader + (many - 1) / 32] = 1u << (many - 1) % 32;
+  for (uint32_t first : {0u, (1u << 24) - 2}) {
+    WarpClock wc;
+    std::memset(&wc, 0, sizeof(wc));
+    wc.item = ~0u;
+    unsigned long long counter = first;
+    std::vector<uint32_t> got;
+    for (int k = 0; k < 60 && (k == 0 || wc.item != ~0u); k++) {
+      const uint32_t item = sched_next<kKindNoBricks>(rd.data(), nullptr, many, &counter, wc);
+      if (item == ~0u) break;
+      expect(item_has_lane(item, 0) && item_has_lane(item, 31), "a tile of a launch of many tiles is split", item);
+      got.push_back(item_tile(item));
+    }
+    std::vector<uint32_t> want;
+    if (first == 0)
+      want = {7, many - 1, 0, 1, 2, 3, 4, 5, 6, 8, 9}; // the listed ones first
+    else
+      for (uint32_t t = first - 2; t < many - 1; t++) want.push_back(t);
+    got.resize(std::min(got.size(), want.size()));
+    expect(got == want, "tiles of a launch of many tiles", got.empty() ? 0 : got.back(), want.back());
   }
   return failed != 0;
 }

@@ -90,3 +90,26 @@ def test_planted_levels_match_oracle(cuda, buffers, kind, most, width, height):
                 assert np.array_equal(image.cpu().numpy(), shade), level
     assert (want["primId"] != MISS).mean() > 0.02
     sc.close()
+
+
+def test_image_of_many_tiles(cuda):
+    """More than 2^24 tiles: a column of rays that miss but for its last rows,
+    in natural and in scheduled launches."""
+    torch = cuda
+    sc = _scene("triangles")
+    tail = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=40, height=30))
+    want = po.port_trace(sc.export_arrays(), tail)
+    height = 4 * ((1 << 24) + 3) + 1
+    rays = torch.empty((height, 8), dtype=torch.float32, device="cuda")
+    rays[:] = torch.tensor([0.0, 50.0, 0.0, 1e-4, 0.0, 1.0, 0.0, 9.0], device="cuda")
+    rays[-len(tail):] = torch.from_numpy(tail).cuda()
+    hits = torch.empty((height, 8), dtype=torch.int32, device="cuda")
+    for natural in (True, False, False):
+        hits.fill_(7)
+        sc.trace_image(rays.data_ptr(), hits.data_ptr(), 1, height, natural_order=natural)
+        sc.sync()
+        assert bool((hits[:-len(tail), 1] == -1).all())
+        got = np.ascontiguousarray(hits[-len(tail):].cpu().numpy()).view(HIT_DTYPE).reshape(-1)
+        assert bit_equal(got, want).all(), hit_summary(got, want)
+    assert (want["primId"] != MISS).mean() > 0.02
+    sc.close()
