@@ -266,7 +266,7 @@ void rows_as_image(lrt_scene* s, cudaStream_t stream, uint64_t n, uint32_t flags
   uint64_t& last = d->lastRays[stream];
   const bool repeat = last == n;
   last = n;
-  const uint64_t slots = uint64_t(d->grid) * (kTraceThreads / 32);
+  const uint64_t slots = uint64_t(lrt_exact::lambert_wave(d->S, d->stackCap)) * (kTraceThreads / 32);
   if (repeat && !(flags & LRT_TRACE_NATURAL_ORDER) && (n + 31) / 32 > slots && (n + 7) / 8 <= 0xFFFFFFFFull) {
     width = 8;
     height = uint32_t((n + 7) / 8);

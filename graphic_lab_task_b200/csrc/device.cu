@@ -226,7 +226,7 @@ lrt_status launch(lrt_scene* s, const float4* rays, lrt_hit* hits, uint64_t n, c
   // with a stride across the launch's rays (k_trace).
   uint32_t group = 32;
   if (!img_w) {
-    const uint64_t slots = uint64_t(d->grid) * (kTraceThreads / 32);
+    const uint64_t slots = uint64_t(lrt_exact::row_wave(S, S.flags, d->stackCap)) * (kTraceThreads / 32);
     while (group > 8 && (n + group / 2 - 1) / (group / 2) <= slots) group /= 2;
   }
   const uint64_t warps = img_w ? uint64_t((img_w + kImgTileW - 1) / kImgTileW) * ((img_h + kImgTileH - 1) / kImgTileH)
@@ -234,7 +234,7 @@ lrt_status launch(lrt_scene* s, const float4* rays, lrt_hit* hits, uint64_t n, c
   const int blocks = blocks_for(warps);
   unsigned long long* work = &slot->work;
   cudaError_t e = cudaSuccess;
-  if (staged && !count && blocks <= d->grid)
+  if (staged && !count && blocks <= lrt_exact::row_wave(S, S.flags, d->stackCap))
     work = nullptr;
   else
     e = cudaMemsetAsync(work, 0, count ? offsetof(StreamSlot, err) : sizeof(unsigned long long), stream);
@@ -630,8 +630,7 @@ lrt_status device_upload(lrt_scene* s)
   // scenes: raise it once to the largest stack any scene may use.
   e = lrt_exact::set_trace_smem(kMaxStack + 1);
   if (e == cudaSuccess) e = lrt_fast::set_trace_smem(kMaxStack + 1);
-  int perSm = 0, sms = 0;
-  if (e == cudaSuccess) e = lrt_exact::trace_occupancy(d->stackCap, S.kind, &perSm);
+  int sms = 0;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
   if (e == cudaSuccess) e = cudaMalloc(&d->slots, sizeof(StreamSlot) * kMaxStreams);
   if (e == cudaSuccess) {
@@ -643,7 +642,6 @@ lrt_status device_upload(lrt_scene* s)
     device_release(s);
     return st;
   }
-  d->grid = std::max(1, perSm) * sms;
   S.sms = uint32_t(sms);
   // The allocation-free trace's static array is looked up here, with the
   // scene's device current, not in the trace call: under lazy module loading
@@ -757,7 +755,7 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
     uint64_t& last = d->lastRays[stream];
     const bool repeat = last == n;
     last = n;
-    const uint64_t slots = uint64_t(d->grid) * (kTraceThreads / 32);
+    const uint64_t slots = uint64_t(lrt_exact::row_wave(d->S, launch_flags(s), d->stackCap)) * (kTraceThreads / 32);
     if (repeat && !(flags & (LRT_TRACE_COUNT_WORK | LRT_TRACE_NATURAL_ORDER)) && (n + 15) / 16 > slots &&
         (n + 7) / 8 <= 0xFFFFFFFFull)
       return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot, 8, uint32_t((n + 7) / 8));

@@ -56,7 +56,6 @@ struct DeviceScene {
   std::vector<void*> allocs;
   DevScene S{};
   uint32_t stackCap = 0;
-  int grid = 0; // blocks in one wave of the scene's trace kernel
   StreamSlot* slots = nullptr; // device, kMaxStreams
   std::map<cudaStream_t, int> slotOf;
   const DevPair* pairsOrig = nullptr; // unpruned node pairs

@@ -12,7 +12,9 @@
                            uint32_t img_h = 0, const uint32_t* sched_rd = nullptr,                              \
                            uint32_t* sched_wr = nullptr, uint32_t group = 32);                                  \
   cudaError_t set_trace_smem(uint32_t stack_cap);                                                               \
-  cudaError_t trace_occupancy(uint32_t stack_cap, uint32_t kind, int* blocks_per_sm);                           \
+  /* blocks in one wave of the row-order trace and of the Lambert passes */                                       \
+  int row_wave(const lrt::DevScene& S, uint32_t flags, uint32_t stack_cap);                                     \
+  int lambert_wave(const lrt::DevScene& S, uint32_t stack_cap);                                                 \
   cudaError_t launch_eye_rays(const lrt::DevCamera& cam, float4* rays, cudaStream_t stream);                    \
   cudaError_t launch_trace_cameras(const lrt::DevScene& S, const lrt::DevBatchCamera* cams, uint32_t ncams,     \
                                    uint32_t ntiles, const lrt::DevBatchShape& shape, lrt_hit* hits,             \

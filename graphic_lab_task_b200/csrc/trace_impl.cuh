@@ -18,7 +18,12 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include "device_layout.h"
 #include "lrt_math.h"
@@ -1625,6 +1630,33 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_trac
   if (c.err) atomicOr(err_word, c.err);
 }
 
+// Blocks in one wave of a kernel on the scene's device: a persistent launch of
+// more would start blocks that find no work left, one of fewer would leave
+// warps unused.  Registers bound it below min_blocks or above (scenes without
+// bricks: 72 registers, 7 blocks where 6 were asked for), and the stacks of
+// deep trees below.  Asked once per kernel and stack capacity; the answer is the
+// same on every device that these kernels run on.
+inline int wave_blocks(const void* kernel, size_t smem, const DevScene& S)
+{
+  static std::mutex lock;
+  static std::map<std::pair<const void*, size_t>, int> known;
+  std::lock_guard<std::mutex> guard(lock);
+  int& perSm = known[{kernel, smem}];
+  if (perSm == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTraceThreads, smem) != cudaSuccess) {
+      cudaGetLastError(); // the launch will say what is wrong
+      perSm = 0;
+    }
+  }
+  return std::max(1, perSm) * int(S.sms);
+}
+// The grid of a launch that has work for `blocks`.
+template <class KERNEL>
+int grid_for(KERNEL kernel, size_t smem, const DevScene& S, int blocks)
+{
+  return std::min(blocks, wave_blocks(reinterpret_cast<const void*>(kernel), smem, S));
+}
+
 cudaError_t launch_trace_cameras(const DevScene& S, const DevBatchCamera* cams, uint32_t ncams, uint32_t ntiles,
                                  const DevBatchShape& shape, lrt_hit* hits, unsigned long long* work_counter,
                                  uint32_t* err_word, int blocks, cudaStream_t stream, const DevLights* lights,
@@ -1633,14 +1665,15 @@ cudaError_t launch_trace_cameras(const DevScene& S, const DevBatchCamera* cams, 
   const size_t smem = trace_smem_bytes(shape.stackCap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     if (image) {
       cudaError_t e = cudaFuncSetAttribute(k_trace_cameras<true, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            int(kMaxTraceSmem));
       if (e != cudaSuccess) return e;
+      const int grid = grid_for(k_trace_cameras<true, K>, smem, S, blocks);
       k_trace_cameras<true, K><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
                                                                    err_word, *lights, image);
     } else {
+      const int grid = grid_for(k_trace_cameras<false, K>, smem, S, blocks);
       k_trace_cameras<false, K><<<grid, kTraceThreads, smem, stream>>>(S, cams, ncams, ntiles, shape, hits, work_counter,
                                                                     err_word, DevLights{}, nullptr);
     }
@@ -2079,7 +2112,6 @@ cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const D
   const bool modes = rm && (rm->mode != LRT_RENDER_MODE_LAMBERT_NO_TEX || rm->samples != 1 || rm->transparency);
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, modes ? kModes : kFrame) * int(S.sms));
     auto kernel = modes ? k_render_rgba8<true, K> : k_render_rgba8<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
@@ -2087,7 +2119,7 @@ cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const D
     DevRenderModes one{};
     one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
     one.samples = 1;
-    kernel<<<grid, kTraceThreads, smem, stream>>>(S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd,
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd,
                                                   sched_wr, materials ? *materials : DevMaterials{}, rm ? *rm : one);
     return cudaGetLastError();
   });
@@ -2100,11 +2132,11 @@ cudaError_t launch_outline_fill(const DevScene& S, const DevCamera& cam, const D
 {
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
+    const size_t smem = trace_smem_bytes(stack_cap);
     cudaError_t e = cudaFuncSetAttribute(k_outline_fill<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    k_outline_fill<K><<<grid, kTraceThreads, trace_smem_bytes(stack_cap), stream>>>(
+    k_outline_fill<K><<<grid_for(k_outline_fill<K>, smem, S, blocks), kTraceThreads, smem, stream>>>(
         S, cam, lights, M, RM, smp, tm, col, work_counter, err_word, stack_cap, sched_rd, sched_wr);
     return cudaGetLastError();
   });
@@ -2127,10 +2159,10 @@ cudaError_t launch_fill_gbuffer_transparency(const DevScene& S, const DevCamera&
   const size_t smem = trace_smem_bytes(stack_cap);
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kFrame) * int(S.sms));
     cudaError_t e = cudaFuncSetAttribute(k_fill_gbuffer_transparency<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
+    const int grid = grid_for(k_fill_gbuffer_transparency<K>, smem, S, blocks);
     k_fill_gbuffer_transparency<K><<<grid, kTraceThreads, smem, stream>>>(S, cam, M, transparency, gbuffer, work_counter,
                                                                        err_word, stack_cap, sched_rd, sched_wr);
     return cudaGetLastError();
@@ -2148,12 +2180,11 @@ cudaError_t launch_render_lambert(const DevScene& S, const float4* rays, uint64_
   const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     auto kernel = img_w ? k_render_lambert<true, K> : k_render_lambert<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
                                                   img_h, sched_rd, sched_wr);
     return cudaGetLastError();
   });
@@ -2167,12 +2198,11 @@ cudaError_t launch_adjoint_lambert(const DevScene& S, const float4* rays, uint64
   const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    const int grid = std::min(blocks, min_blocks(K, kMany) * int(S.sms));
     auto kernel = img_w ? k_adjoint_lambert<true, K> : k_adjoint_lambert<false, K>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    kernel<<<grid, kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
                                                   img_w, img_h, sched_rd, sched_wr);
     return cudaGetLastError();
   });
@@ -2204,30 +2234,25 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
   const bool solvers = solver != kSolverST && solver != kSolverBBox;
   // image order (IMG) is its own instantiation, so that the tile schedule
   // costs the row-order kernel nothing
-  auto go = [&](auto kernel, int most) {
-    kernel<<<std::min(blocks, most * int(S.sms)), kTraceThreads, smem, stream>>>(
+  auto go = [&](auto kernel) {
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
         S, rays, hits, n, work_counter, counters, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr, group);
     return cudaGetLastError();
   };
   if (count) { // the counting kernels are compiled for all kinds
-    constexpr int B = min_blocks(kKindAll, kFrame);
     if (img_w)
-      return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>, B)
-                     : go(k_trace<true, false, true, kKindAll, kFrame>, B);
-    return solvers ? go(k_trace<true, true, false, kKindAll, kFrame>, B)
-                   : go(k_trace<true, false, false, kKindAll, kFrame>, B);
+      return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>) : go(k_trace<true, false, true, kKindAll, kFrame>);
+    return solvers ? go(k_trace<true, true, false, kKindAll, kFrame>) : go(k_trace<true, false, false, kKindAll, kFrame>);
   }
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    constexpr int F = min_blocks(K, kFrame), M = min_blocks(K, kMany);
     // the node solvers spill at any bound: their kernels keep the wider one
-    if (solvers)
-      return img_w ? go(k_trace<false, true, true, K, kFrame>, F) : go(k_trace<false, true, false, K, kFrame>, F);
+    if (solvers) return img_w ? go(k_trace<false, true, true, K, kFrame>) : go(k_trace<false, true, false, K, kFrame>);
     // only scenes without bricks gain from the narrow one here
     if constexpr (K == kKindNoBricks)
-      if (uint64_t(blocks) >= uint64_t(kManyWaves) * M * S.sms)
-        return img_w ? go(k_trace<false, false, true, K, kMany>, M) : go(k_trace<false, false, false, K, kMany>, M);
-    return img_w ? go(k_trace<false, false, true, K, kFrame>, F) : go(k_trace<false, false, false, K, kFrame>, F);
+      if (uint64_t(blocks) >= uint64_t(kManyWaves) * min_blocks(K, kMany) * S.sms)
+        return img_w ? go(k_trace<false, false, true, K, kMany>) : go(k_trace<false, false, false, K, kMany>);
+    return img_w ? go(k_trace<false, false, true, K, kFrame>) : go(k_trace<false, false, false, K, kFrame>);
   });
 }
 
@@ -2255,12 +2280,24 @@ cudaError_t set_trace_smem(uint32_t stack_cap)
   return e;
 }
 
-cudaError_t trace_occupancy(uint32_t stack_cap, uint32_t kind, int* blocks_per_sm)
+int row_wave(const DevScene& S, uint32_t flags, uint32_t stack_cap)
 {
   const size_t smem = trace_smem_bytes(stack_cap);
-  return with_kind(kind, [&](auto k) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        blocks_per_sm, k_trace<false, false, true, decltype(k)::value, kFrame>, kTraceThreads, smem);
+  const uint32_t solver = (flags >> kFlagSolverShift) & 7u;
+  const bool solvers = solver != kSolverST && solver != kSolverBBox;
+  return with_kind(S.kind, [&](auto k) {
+    constexpr uint32_t K = decltype(k)::value;
+    auto kernel = solvers ? k_trace<false, true, false, K, kFrame> : k_trace<false, false, false, K, kFrame>;
+    return wave_blocks(reinterpret_cast<const void*>(kernel), smem, S);
+  });
+}
+
+int lambert_wave(const DevScene& S, uint32_t stack_cap)
+{
+  return with_kind(S.kind, [&](auto k) {
+    constexpr uint32_t K = decltype(k)::value;
+    return wave_blocks(reinterpret_cast<const void*>(k_render_lambert<false, K>),
+                       trace_smem_bytes(stack_cap, shared_ray(K)), S);
   });
 }
 

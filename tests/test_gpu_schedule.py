@@ -113,3 +113,46 @@ def test_image_of_many_tiles(cuda):
         assert bit_equal(got, want).all(), hit_summary(got, want)
     assert (want["primId"] != MISS).mean() > 0.02
     sc.close()
+
+
+def test_deep_trees_launch_one_wave(cuda, buffers):
+    """A tree as deep as the traversal stack: its launches start the blocks
+    that its stacks leave room for, and every pixel is the oracle's."""
+    torch = cuda
+    sc = SceneRT(preset=parity_preset())
+    sc.AddInstance(sc.AddGeom_Triangles3f(*wl.noisy_sphere(24, seed=2)), wl.IDENTITY)
+    sc.CommitScene(host_only=True)
+    a = {k: v.copy() for k, v in sc.export_arrays().items()}
+    tree = a["allNodePairs"]
+    depth, todo = 0, [(0, 1)]
+    while todo:
+        k, d = todo.pop()
+        depth = max(depth, d)
+        todo += [(int(tree[side]["leftOffset"][k]), d + 1) for side in ("left", "right")
+                 if tree[side]["leftOffset"][k] < 0x80000000]
+    n = 80 - depth
+    chain = np.repeat(tree[:1], n)  # pairs that lead from one to the next and then to the mesh's root
+    for side in ("left", "right"):
+        chain[side]["boxMin"], chain[side]["boxMax"] = -2.0, 2.0
+        lo = tree[side]["leftOffset"]
+        tree[side]["leftOffset"] = np.where(lo < 0x80000000, lo + n, lo)
+    chain["left"]["leftOffset"], chain["right"]["leftOffset"] = np.arange(1, n + 1), 0xFFFFFFFF
+    a["allNodePairs"] = np.concatenate([chain, tree])
+    w, h = 640, 480
+    rays = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=w, height=h))
+    want = po.port_trace(a, rays)
+    sc = SceneRT(preset=parity_preset())
+    sc.upload_arrays(a)
+    r = torch.from_numpy(rays).cuda()
+    hits = torch.zeros(len(rays) * 8, dtype=torch.float32, device="cuda")
+    for _ in range(3):
+        hits.zero_()
+        sc.trace_image(r.data_ptr(), hits.data_ptr(), w, h)
+        sc.sync()
+        got = np.ascontiguousarray(hits.cpu().numpy()).view(HIT_DTYPE).reshape(-1)
+        assert bit_equal(got, want).all(), hit_summary(got, want)
+    # 81 + 16 words a thread, and 1 KB a block of the system's own
+    blocks = (228 * 1024) // ((81 + 16) * 128 * 4 + 1024)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert buffers(torch, sc, w, h)[0].cpu().numpy()[WARPS] == blocks * sms * 4
+    sc.close()
