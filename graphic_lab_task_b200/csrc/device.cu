@@ -219,16 +219,7 @@ lrt_status launch(lrt_scene* s, const float4* rays, lrt_hit* hits, uint64_t n, c
   if (n < kPrefetchMinRays)
     for (int r = 0; r < kPrefetchRanges; r++) S.pfBytes[r] = 0;
   const bool count = (flags & LRT_TRACE_COUNT_WORK) != 0;
-  // Row order: rays to a warp.  A launch of fewer rays than one wave of the
-  // kernel's warps can hold takes as long as its slowest warp, and a warp's
-  // time grows with the number of slow rays among its lanes, so such a launch
-  // gives each warp 16 or 8 rays while the warps still fit in one wave, taken
-  // with a stride across the launch's rays (k_trace).
-  uint32_t group = 32;
-  if (!img_w) {
-    const uint64_t slots = uint64_t(lrt_exact::row_wave(S, S.flags, d->stackCap)) * (kTraceThreads / 32);
-    while (group > 8 && (n + group / 2 - 1) / (group / 2) <= slots) group /= 2;
-  }
+  const uint32_t group = img_w ? 32 : rays_per_warp(n, S.sms);
   const uint64_t warps = img_w ? uint64_t((img_w + kImgTileW - 1) / kImgTileW) * ((img_h + kImgTileH - 1) / kImgTileH)
                                : (n + group - 1) / group;
   const int blocks = blocks_for(warps);
@@ -745,9 +736,9 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
   if (flags & LRT_TRACE_DEVICE_POINTERS) {
     if ((reinterpret_cast<uintptr_t>(rays) | reinterpret_cast<uintptr_t>(hits)) & 15)
       return fail(s, LRT_ERR_INVALID_ARGUMENT, "device rays/hits must be 16-byte aligned");
-    // A trace of a wave or more of 32-ray groups that repeats the previous
-    // trace's ray count on this stream (a renderer's frames) goes through the
-    // image-order kernel as an image 8 rays wide, whose 8x4 tiles are the same
+    // A trace whose warps take 32 rays each (rays_per_warp) and that repeats
+    // the previous trace's ray count on this stream (a renderer's frames) goes
+    // through the image-order kernel as an image 8 rays wide, whose 8x4 tiles are the same
     // 32 consecutive rays: the groups are then handed out in the stream's
     // schedule for this ray count (slowest groups first, the slowest split
     // over 2 to 8 warps when the previous launch was tail-bound).  Traces of
@@ -755,8 +746,7 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
     uint64_t& last = d->lastRays[stream];
     const bool repeat = last == n;
     last = n;
-    const uint64_t slots = uint64_t(lrt_exact::row_wave(d->S, launch_flags(s), d->stackCap)) * (kTraceThreads / 32);
-    if (repeat && !(flags & (LRT_TRACE_COUNT_WORK | LRT_TRACE_NATURAL_ORDER)) && (n + 15) / 16 > slots &&
+    if (repeat && !(flags & (LRT_TRACE_COUNT_WORK | LRT_TRACE_NATURAL_ORDER)) && rays_per_warp(n, d->S.sms) == 32 &&
         (n + 7) / 8 <= 0xFFFFFFFFull)
       return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot, 8, uint32_t((n + 7) / 8));
     return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot);

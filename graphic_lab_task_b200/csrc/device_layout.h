@@ -170,6 +170,25 @@ constexpr uint64_t kPrefetchMaxBytes = 48ull << 20;
 constexpr uint64_t kPrefetchMinRays = 4096;
 constexpr uint32_t kPrefetchChunk = 4096; // bytes per prefetch instruction
 
+// Row order: rays to a warp (16 or 8, strided across the launch's rays, while
+// that gives at most kRowWarps warps per SM, else 32 consecutive ones).  A
+// launch smaller than one wave lasts as long as its slowest warp, and a warp's
+// time grows with the slow rays among its lanes.  28 warps per SM are a wave of
+// the kernels without bricks; of the others, of which 20 fit, the last ones wait
+// for a warp to finish, and still gain.  Measured in limits of one wave / 28 /
+// 36 / 48 (us): 256^3 bricks, 39,100 rays 117 / 117 / 132 / 132, 56,064 rays 215
+// / 139 / 139 / 166, 65,536 rays 233 / 164 / 164 / 164, 99,840 rays natural 245
+// / 242 / 245 / 209; voxel set, 56,064 rays 101 / 101 / 101 / 123, 66,304 rays
+// 140 / 122 / 122 / 122; mixed scene, 23,940 rays 237 / 205 / 205 / 205, 56,064
+// rays 650 / 410 / 410 / 446, 89,600 rays repeated 470 / 470 / 470 / 526.
+constexpr uint32_t kRowWarps = 28;
+inline uint32_t rays_per_warp(uint64_t n, uint32_t sms)
+{
+  uint32_t group = 32;
+  while (group > 8 && (n + group / 2 - 1) / (group / 2) <= uint64_t(kRowWarps) * sms) group /= 2;
+  return group;
+}
+
 // Geometry kinds a trace kernel is compiled for.  The leaf code of every kind
 // shares the traversal's registers, and what does not fit is spilled in every
 // loop, so a scene without bricks, and one of bricks only, have kernels of

@@ -29,8 +29,22 @@ static void slots()
   expect(triangle_slots(h, 0) == 0, "a table of no triangles has slots");
 }
 
+// Rays to a warp around the sizes from which a launch takes larger groups,
+// whatever the scene's kernels (28 warps on each of 148 SMs).
+static void rows()
+{
+  const struct {
+    uint64_t n;
+    uint32_t group;
+  } want[] = {{1, 8},      {33152, 8},  {33153, 16}, {47000, 16},  {56832, 16},
+              {65536, 16}, {66304, 16}, {66305, 32}, {262144, 32}, {1ull << 33, 32}};
+  for (const auto& w : want) expect(rays_per_warp(w.n, 148) == w.group, "rays to a warp");
+  expect(rays_per_warp(66304, 74) == 32, "rays to a warp of half the SMs");
+}
+
 int main()
 {
   slots();
+  rows();
   return failed;
 }
