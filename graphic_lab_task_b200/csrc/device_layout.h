@@ -70,10 +70,12 @@ inline __host__ __device__ uint64_t sched_words(uint64_t tiles)
 // deferred SBS hit colour (object-space hit point, brick node index).
 constexpr uint32_t kNormalWords = 16;
 constexpr uint32_t kColourWord = 12;
-// After them, in the brick kernels for many waves, the ray's origin and
-// direction: they are only read when an instance is entered, and out of the
-// march's registers they let 7 blocks per SM run with few spills.
-constexpr uint32_t kRayWord = 16, kRayWords = 6;
+// After them, in the kernels for many waves of scenes with bricks, the ray's
+// origin, direction and inverse direction: they are only read when the TLAS is
+// walked on, and out of the march's registers they let 7 blocks per SM run with
+// few spills (6 with none where a scene holds other kinds too).  The inverse
+// spares three divisions per instance: mixed scenes 1-2%.
+constexpr uint32_t kRayWord = 16, kRayWords = 9;
 constexpr uint32_t kMaxStackDev = 80; // STACK_SIZE of raytrace_common.h:36
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kMaxVoxelSteps = 4096u; // voxel-march cap per brick (the reference loop is unbounded)

@@ -67,31 +67,40 @@ struct Hit {
 // the scene's geometry kind (device_layout.h) and what the launch waits for:
 // a frame of a few waves is as long as its slowest tiles' chains of dependent
 // steps and wants them free of spills, a launch of many waves wants warps.
-// Measured (us; 5 / 6 / 8 blocks of 128 threads = 96 / 80 / 64 registers):
-//   bricks: 512^3 model at 1920x1080 493 / 503 / -, fused render 382 / 402 / -,
-//     64 cameras (51 M rays) 13,319 / 12,546 / -, Lambert step 3,429 / 3,254 / -
-//     (these two with the ray in shared memory run 7 blocks: shared_ray)
-//   no bricks: 4096^2 instanced primary rays - / 5,737 / 5,573, sorted bounce
-//     - / 6,211 / 5,940, a 200k-triangle mesh at 256^2 - / 102 / 108, a voxel
-//     set at 1001x777 (ANALYTIC) - / 290 / 311
-//   all kinds: mixed scene at 1280x720 556 / 577 / 672 (7 blocks)
-//     and its render of all modes, LAMBERT with a transparent mesh, 1,669 /
-//     1,869 / 1,833 / 1,901 in 4 / 5 / 6 / 7 blocks (128 registers and up)
+// Measured (us; 4 / 5 / 6 / 7 / 8 blocks of 128 threads = 128 / 96 / 80 / 72 /
+// 64 registers, the ray in shared memory from where it says so):
+//   bricks: 512^3 model at 1920x1080 - / 493 / 503, fused render - / 382 / 402,
+//     64 cameras (51 M rays) - / 13,319 / 12,546 / 12,189 shared, Lambert step
+//     - / 3,429 / 3,254 / 2,603 shared
+//   no bricks: 4096^2 instanced primary rays - / - / 5,737 / - / 5,573, sorted
+//     bounce - / - / 6,211 / - / 5,940, a 200k-triangle mesh at 256^2 - / - /
+//     102 / - / 108, a voxel set at 1001x777 (ANALYTIC) - / - / 290 / - / 311
+//   all kinds, mixed scene of 24 instances: 640x360 - / 467 / 481 / 491 (6 and
+//     7 shared), 1280x720 - / 534 / 534 / 565, 2560x1440 - / 1,275 / 1,214 /
+//     1,262, 56,064 rays in rows - / 406 / 364 / 371; fused render 1280x720 - /
+//     579 / 581 / 609, 2560x1440 - / 1,400 / 1,400 / 1,426
+//   all kinds, render of all modes: LAMBERT with a transparent mesh, 640x360
+//     1,122 / 1,193 / 1,264 / 1,448, 1280x720 1,410 / 1,410 / 1,538 / 1,650,
+//     2560x1440 of 80 instances 9,330 / 8,960 / 9,608 / 9,516
 constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
 constexpr int kModes = 2;            // the render of all modes, samples and transparency
-constexpr int kManyWaves = 12;       // k_trace takes the kernel for many from here on
+constexpr int kManyWaves = 12;       // scenes without bricks: k_trace takes the kernel for many from here on
 constexpr int min_blocks(uint32_t kind, int size)
 {
   if (kind == kKindBricks) return size == kMany ? 7 : 5;
   if (kind == kKindNoBricks) return size == kMany ? 8 : 6;
-  return size == kModes ? 4 : 5;
+  return size == kModes ? 4 : size == kMany ? 6 : 5;
 }
 
-// The brick kernels for many waves keep the ray in shared memory: at 80
-// registers (6 blocks) with it in registers 64 cameras took 12,556 us and a
-// Lambert step 2,684; from shared memory 12,357 and 2,671, and at 72 (7 blocks)
-// 12,189 and 2,603.  Frames gain nothing (fused render 377 -> 384).
-constexpr bool shared_ray(uint32_t kind) { return kind == kKindBricks; }
+// The kernels for many waves that hold bricks keep the ray in shared memory: in
+// brick-only scenes at 80 registers (6 blocks) with it in registers 64 cameras
+// took 12,556 us and a Lambert step 2,684; from shared memory 12,357 and 2,671,
+// and at 72 (7 blocks) 12,189 and 2,603.  Frames gain nothing (fused render 377
+// -> 384).
+constexpr bool shared_ray(uint32_t kind, int size)
+{
+  return size == kMany && kind != kKindNoBricks;
+}
 
 // f(std::integral_constant<uint32_t, kind>) for a scene's kernel kind.
 template <class F>
@@ -539,14 +548,24 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
   const float* dense = S.sbsDense + sb.denseBase + uint64_t(primId) * sb.denseStride;
   float values[8];
   uint32_t steps = 0;
-  // The march goes on to the next voxel whose sphere trace may hit, in which
-  // the warp's lanes then trace together.
+  // In brick-only scenes the march goes on to the next voxel whose sphere trace
+  // may hit, in which the warp's lanes then trace together.  The kernels of all
+  // kinds trace in each voxel: what the march has to keep until the trace took
+  // 100 bytes of spills more in them (mixed scene at 2560x1440 in 7 blocks 1,408
+  // -> 1,250 us, the latter with the ray in shared memory).
+  constexpr bool kToCandidate = CTX::kKind == kKindBricks;
   while (bnf.x < bnf.y && hit.t == old_t) {
     bool found = false;
     f3 start_q = mk3(0, 0, 0);
     f2 fNearFar = mk2(0, 0);
     float qFar = 0, start_sign = 1, start_dist = 0;
     uint32_t vx = 0, vy = 0, vz = 0;
+    auto trace = [&] {
+      local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, 0.0f, qFar, fNearFar, start_q, start_sign,
+                    start_dist, hit);
+      if (CTX::kRecord && hit.t < old_t)
+        c.nrec[0] = __uint_as_float(__float_as_uint(c.nrec[0]) | (vx << 3) | (vy << 7) | (vz << 11));
+    };
     do {
       if (steps++ >= S.voxelStepCap) {
         c.err |= kErrVoxelCap;
@@ -585,16 +604,13 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
         const f3 start_pos = ray_pos + fNearFar.x * ray_dir;
         start_q = (start_pos - min_pos) * scale;
         qFar = (fNearFar.y - fNearFar.x) * scale;
-        found = surface_start<CTX::kKind == kKindBricks>(c, ray_dir, values, 0.0f, qFar, start_q, start_sign, start_dist);
+        found = surface_start<kToCandidate>(c, ray_dir, values, 0.0f, qFar, start_q, start_sign, start_dist);
+        if constexpr (!kToCandidate) trace(); // (found: only the reach test rejects)
       }
       bnf.x += smax(0.0f, vfar - bnf.x) + 1e-6f;
-    } while (CTX::kKind == kKindBricks && !found && bnf.x < bnf.y);
-    if (found) {
-      local_surface(c, g.type, ray_dir, instId, geomId, values, primId, d, 0.0f, qFar, fNearFar, start_q, start_sign,
-                    start_dist, hit);
-      if (CTX::kRecord && hit.t < old_t)
-        c.nrec[0] = __uint_as_float(__float_as_uint(c.nrec[0]) | (vx << 3) | (vy << 7) | (vz << 11));
-    }
+    } while (kToCandidate && !found && bnf.x < bnf.y);
+    if constexpr (kToCandidate)
+      if (found) trace();
   }
   if (hit.t < old_t && sb.colorLayout) {
     // The colour of the hit (indexed layouts) is evaluated once the traversal
@@ -898,6 +914,8 @@ __device__ __forceinline__ void walk_begin(CTX& c, Walk& w, float4 pn, float4 df
     float* rw = c.nrec + kRayWord * st;
     rw[0] = pn.x, rw[st] = pn.y, rw[2 * st] = pn.z;
     rw[3 * st] = df.x, rw[4 * st] = df.y, rw[5 * st] = df.z;
+    const f3 inv = safe_inverse(mk3(df.x, df.y, df.z));
+    rw[6 * st] = inv.x, rw[7 * st] = inv.y, rw[8 * st] = inv.z;
   } else {
     w.pos = mk3(pn.x, pn.y, pn.z);
     w.dir = mk3(df.x, df.y, df.z);
@@ -918,17 +936,18 @@ template <class CTX>
 __device__ __forceinline__ uint32_t walk_tlas(CTX& c, Walk& w, uint32_t* stack)
 {
   const DevScene& S = c.S;
-  f3 pos, dir;
+  f3 pos, dir, inv;
   if constexpr (CTX::kSharedRay) {
     const uint32_t st = blockDim.x;
     const float* rw = c.nrec + kRayWord * st;
     pos = mk3(rw[0], rw[st], rw[2 * st]);
     dir = mk3(rw[3 * st], rw[4 * st], rw[5 * st]);
+    inv = mk3(rw[6 * st], rw[7 * st], rw[8 * st]);
   } else {
     pos = w.pos;
     dir = w.dir;
+    inv = safe_inverse(dir);
   }
-  const f3 inv = safe_inverse(dir);
   const bool fast = fast_nodes(S, pos, dir, inv);
   uint32_t travFlags = 0, leftOffset = 0;
   if (fast)
@@ -1085,7 +1104,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_trace
   extern __shared__ uint32_t smem_stack[];
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<COUNT, false, SOLVERS, KIND> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<COUNT, false, SOLVERS, KIND, shared_ray(KIND, SIZE)> c(S, normal_words(smem_stack, stack_cap));
   __shared__ WarpClock wclock[IMG ? kTraceThreads / 32 : 1];
   const uint64_t tilesX = (uint64_t(img_w) + kImgTileW - 1) / kImgTileW;
   if (IMG && lane == 0) {
@@ -1591,7 +1610,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_trac
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false, false, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, shape.stackCap));
+  Ctx<false, false, false, KIND, shared_ray(KIND, kMany)> c(S, normal_words(smem_stack, shape.stackCap));
   for (;;) {
     unsigned long long tile = 0;
     if (lane == 0) tile = atomicAdd(work_counter, 1ull);
@@ -1662,7 +1681,7 @@ cudaError_t launch_trace_cameras(const DevScene& S, const DevBatchCamera* cams, 
                                  uint32_t* err_word, int blocks, cudaStream_t stream, const DevLights* lights,
                                  uint32_t* image)
 {
-  const size_t smem = trace_smem_bytes(shape.stackCap, shared_ray(S.kind));
+  const size_t smem = trace_smem_bytes(shape.stackCap, shared_ray(S.kind, kMany));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     if (image) {
@@ -1712,8 +1731,8 @@ __device__ __forceinline__ float lambert(const lrt_hit& h, f3 dir, f3 L)
 // triangle and turned towards the viewer as in loadNormalTcFromGbuffer :27-75,
 // SDF normals decoded from the hit) and Tonemap (:536-542) into RGBA8.  A warp
 // takes 8x4-pixel tiles from a global counter.
-template <bool MODES, uint32_t KIND>
-__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, MODES ? kModes : kFrame)) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
+template <bool MODES, uint32_t KIND, int SIZE>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_render_rgba8(DevScene S, DevCamera cam, DevLights L,
                                                                 uint32_t* __restrict__ image,
                                                                 unsigned long long* __restrict__ work_counter,
                                                                 uint32_t* __restrict__ err_word, uint32_t stack_cap,
@@ -1724,7 +1743,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, MODES ? kModes
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND, shared_ray(KIND, SIZE)> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1795,8 +1814,8 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, MODES ? kModes
 // does (the OUTLINE_PRIM colour), or the background for a miss.  The colour
 // is resolved here, with the trace's context, because a triangle's normal
 // needs the triangle record the traversal found.
-template <uint32_t KIND>
-__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_outline_fill(DevScene S, DevCamera cam, DevLights L,
+template <uint32_t KIND, int SIZE>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_outline_fill(DevScene S, DevCamera cam, DevLights L,
                                                                 DevMaterials M, DevRenderModes RM, uint32_t smp,
                                                                 float2* __restrict__ tm, float4* __restrict__ col,
                                                                 unsigned long long* __restrict__ work_counter,
@@ -1808,7 +1827,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_out
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND, shared_ray(KIND, SIZE)> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1883,8 +1902,8 @@ __global__ void __launch_bounds__(256) k_outline_resolve(const float2* __restric
 
 // kernel1D_FillGbufferWithTransparency (MultiRenderer.cpp:204-221) for one
 // sample: anyhit_loop per pixel of the camera (8x4-pixel tiles per warp).
-template <uint32_t KIND>
-__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_fill_gbuffer_transparency(
+template <uint32_t KIND, int SIZE>
+__global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, SIZE)) k_fill_gbuffer_transparency(
     DevScene S, DevCamera cam, DevMaterials M, float4* __restrict__ transparency, lrt_hit* __restrict__ gbuffer,
     unsigned long long* __restrict__ work_counter, uint32_t* __restrict__ err_word, uint32_t stack_cap,
     const uint32_t* __restrict__ sched_rd, uint32_t* sched_wr)
@@ -1893,7 +1912,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kFrame)) k_fil
   l2_prefetch_scene(S);
   uint32_t* stack = smem_stack + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
-  Ctx<false, false, false, KIND> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND, shared_ray(KIND, SIZE)> c(S, normal_words(smem_stack, stack_cap));
   const uint32_t tilesX = (cam.width + 7) / 8, ntiles = tilesX * ((cam.height + 3) / 4);
   __shared__ WarpClock wclock[kTraceThreads / 32];
   if (lane == 0) {
@@ -1982,7 +2001,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_rend
     wc->longest = 0;
     wc->busy = 0;
   }
-  Ctx<false, false, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, stack_cap));
+  Ctx<false, false, false, KIND, shared_ray(KIND, kMany)> c(S, normal_words(smem_stack, stack_cap));
   const f3 L = mk3(light.x, light.y, light.z);
   uint64_t i = 0;
   bool valid = false;
@@ -2037,7 +2056,7 @@ __global__ void __launch_bounds__(kTraceThreads, min_blocks(KIND, kMany)) k_adjo
     if (!valid) continue;
     const float dLdI = __ldg(dimage + i);
     if (dLdI == 0.0f) continue;
-    Ctx<false, true, false, KIND, shared_ray(KIND)> c(S, normal_words(smem_stack, stack_cap));
+    Ctx<false, true, false, KIND, shared_ray(KIND, kMany)> c(S, normal_words(smem_stack, stack_cap));
     const float4 pn = __ldg(rays + 2 * i), df = __ldg(rays + 2 * i + 1);
     lrt_hit h;
     trace_one(c, stack, blockDim.x, stack_cap, pn, df, h);
@@ -2105,23 +2124,25 @@ cudaError_t launch_render_rgba8(const DevScene& S, const DevCamera& cam, const D
                                 cudaStream_t stream, const uint32_t* sched_rd, uint32_t* sched_wr,
                                 const DevMaterials* materials, const DevRenderModes* rm)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
   // one sample of LAMBERT_NO_TEX keeps its own instantiation (the benchmarked
   // render); the other modes, several samples and transparency share the
   // general one
   const bool modes = rm && (rm->mode != LRT_RENDER_MODE_LAMBERT_NO_TEX || rm->samples != 1 || rm->transparency);
+  DevRenderModes one{};
+  one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
+  one.samples = 1;
+  auto go = [&](auto kernel, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxTraceSmem));
+    if (e != cudaSuccess) return e;
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
+        S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd, sched_wr,
+        materials ? *materials : DevMaterials{}, rm ? *rm : one);
+    return cudaGetLastError();
+  };
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    auto kernel = modes ? k_render_rgba8<true, K> : k_render_rgba8<false, K>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(kMaxTraceSmem));
-    if (e != cudaSuccess) return e;
-    DevRenderModes one{};
-    one.mode = LRT_RENDER_MODE_LAMBERT_NO_TEX;
-    one.samples = 1;
-    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, cam, lights, image, work_counter, err_word, stack_cap, sched_rd,
-                                                  sched_wr, materials ? *materials : DevMaterials{}, rm ? *rm : one);
-    return cudaGetLastError();
+    return modes ? go(k_render_rgba8<true, K, kModes>, trace_smem_bytes(stack_cap, shared_ray(K, kModes)))
+                 : go(k_render_rgba8<false, K, kFrame>, trace_smem_bytes(stack_cap, shared_ray(K, kFrame)));
   });
 }
 
@@ -2130,15 +2151,16 @@ cudaError_t launch_outline_fill(const DevScene& S, const DevCamera& cam, const D
                                unsigned long long* work_counter, uint32_t* err_word, uint32_t stack_cap, int blocks,
                                cudaStream_t stream, const uint32_t* sched_rd, uint32_t* sched_wr)
 {
-  return with_kind(S.kind, [&](auto kind) {
-    constexpr uint32_t K = decltype(kind)::value;
-    const size_t smem = trace_smem_bytes(stack_cap);
-    cudaError_t e = cudaFuncSetAttribute(k_outline_fill<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(kMaxTraceSmem));
+  auto go = [&](auto kernel, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    k_outline_fill<K><<<grid_for(k_outline_fill<K>, smem, S, blocks), kTraceThreads, smem, stream>>>(
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
         S, cam, lights, M, RM, smp, tm, col, work_counter, err_word, stack_cap, sched_rd, sched_wr);
     return cudaGetLastError();
+  };
+  return with_kind(S.kind, [&](auto kind) {
+    constexpr uint32_t K = decltype(kind)::value;
+    return go(k_outline_fill<K, kFrame>, trace_smem_bytes(stack_cap, shared_ray(K, kFrame)));
   });
 }
 
@@ -2156,16 +2178,16 @@ cudaError_t launch_fill_gbuffer_transparency(const DevScene& S, const DevCamera&
                                              uint32_t* err_word, uint32_t stack_cap, int blocks, cudaStream_t stream,
                                              const uint32_t* sched_rd, uint32_t* sched_wr)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
+  auto go = [&](auto kernel, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxTraceSmem));
+    if (e != cudaSuccess) return e;
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
+        S, cam, M, transparency, gbuffer, work_counter, err_word, stack_cap, sched_rd, sched_wr);
+    return cudaGetLastError();
+  };
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    cudaError_t e = cudaFuncSetAttribute(k_fill_gbuffer_transparency<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(kMaxTraceSmem));
-    if (e != cudaSuccess) return e;
-    const int grid = grid_for(k_fill_gbuffer_transparency<K>, smem, S, blocks);
-    k_fill_gbuffer_transparency<K><<<grid, kTraceThreads, smem, stream>>>(S, cam, M, transparency, gbuffer, work_counter,
-                                                                       err_word, stack_cap, sched_rd, sched_wr);
-    return cudaGetLastError();
+    return go(k_fill_gbuffer_transparency<K, kFrame>, trace_smem_bytes(stack_cap, shared_ray(K, kFrame)));
   });
 }
 
@@ -2177,7 +2199,7 @@ cudaError_t launch_render_lambert(const DevScene& S, const float4* rays, uint64_
                                   cudaStream_t stream, uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd,
                                   uint32_t* sched_wr)
 {
-  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
+  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind, kMany));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     auto kernel = img_w ? k_render_lambert<true, K> : k_render_lambert<false, K>;
@@ -2195,7 +2217,7 @@ cudaError_t launch_adjoint_lambert(const DevScene& S, const float4* rays, uint64
                                    uint32_t* err_word, uint32_t stack_cap, int blocks, cudaStream_t stream,
                                    uint32_t img_w, uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr)
 {
-  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind));
+  const size_t smem = trace_smem_bytes(stack_cap, shared_ray(S.kind, kMany));
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
     auto kernel = img_w ? k_adjoint_lambert<true, K> : k_adjoint_lambert<false, K>;
@@ -2227,38 +2249,47 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
                                 uint32_t stack_cap, int blocks, cudaStream_t stream, bool count, uint32_t img_w,
                                 uint32_t img_h, const uint32_t* sched_rd, uint32_t* sched_wr, uint32_t group)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
   // the ANALYTIC / NEWTON / IT node solvers live in their own instantiation,
   // so that the sphere-tracing kernel keeps its registers
   const uint32_t solver = (S.flags >> kFlagSolverShift) & 7u;
   const bool solvers = solver != kSolverST && solver != kSolverBBox;
   // image order (IMG) is its own instantiation, so that the tile schedule
   // costs the row-order kernel nothing
-  auto go = [&](auto kernel) {
+  auto go = [&](auto kernel, bool sharedRay) {
+    const size_t smem = trace_smem_bytes(stack_cap, sharedRay);
     kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
         S, rays, hits, n, work_counter, counters, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr, group);
     return cudaGetLastError();
   };
   if (count) { // the counting kernels are compiled for all kinds
+    constexpr bool R = shared_ray(kKindAll, kFrame);
     if (img_w)
-      return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>) : go(k_trace<true, false, true, kKindAll, kFrame>);
-    return solvers ? go(k_trace<true, true, false, kKindAll, kFrame>) : go(k_trace<true, false, false, kKindAll, kFrame>);
+      return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>, R)
+                     : go(k_trace<true, false, true, kKindAll, kFrame>, R);
+    return solvers ? go(k_trace<true, true, false, kKindAll, kFrame>, R)
+                   : go(k_trace<true, false, false, kKindAll, kFrame>, R);
   }
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
+    constexpr bool R = shared_ray(K, kFrame);
     // the node solvers spill at any bound: their kernels keep the wider one
-    if (solvers) return img_w ? go(k_trace<false, true, true, K, kFrame>) : go(k_trace<false, true, false, K, kFrame>);
-    // only scenes without bricks gain from the narrow one here
-    if constexpr (K == kKindNoBricks)
-      if (uint64_t(blocks) >= uint64_t(kManyWaves) * min_blocks(K, kMany) * S.sms)
-        return img_w ? go(k_trace<false, false, true, K, kMany>) : go(k_trace<false, false, false, K, kMany>);
-    return img_w ? go(k_trace<false, false, true, K, kFrame>) : go(k_trace<false, false, false, K, kFrame>);
+    if (solvers)
+      return img_w ? go(k_trace<false, true, true, K, kFrame>, R) : go(k_trace<false, true, false, K, kFrame>, R);
+    // (brick-only scenes gain nothing from the narrow one here, mixed ones as
+    // soon as the launch is more than a wave of the wide one: min_blocks)
+    if constexpr (K != kKindBricks) {
+      constexpr bool RM = shared_ray(K, kMany);
+      const uint64_t wave = K == kKindAll ? min_blocks(K, kFrame) : kManyWaves * min_blocks(K, kMany);
+      if (uint64_t(blocks) > wave * S.sms)
+        return img_w ? go(k_trace<false, false, true, K, kMany>, RM) : go(k_trace<false, false, false, K, kMany>, RM);
+    }
+    return img_w ? go(k_trace<false, false, true, K, kFrame>, R) : go(k_trace<false, false, false, K, kFrame>, R);
   });
 }
 
 cudaError_t set_trace_smem(uint32_t stack_cap)
 {
-  const int smem = int(trace_smem_bytes(stack_cap));
+  const int smem = int(trace_smem_bytes(stack_cap, true));
   cudaError_t e = cudaSuccess;
   auto set = [&](auto kernel) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -2269,6 +2300,8 @@ cudaError_t set_trace_smem(uint32_t stack_cap)
   set(k_trace<true, true, true, kKindAll, kFrame>);
   set(k_trace<false, false, false, kKindNoBricks, kMany>);
   set(k_trace<false, false, true, kKindNoBricks, kMany>);
+  set(k_trace<false, false, false, kKindAll, kMany>);
+  set(k_trace<false, false, true, kKindAll, kMany>);
   for (uint32_t kind : {kKindBricks, kKindNoBricks, kKindAll})
     with_kind(kind, [&](auto k) {
       constexpr uint32_t K = decltype(k)::value;
@@ -2282,13 +2315,12 @@ cudaError_t set_trace_smem(uint32_t stack_cap)
 
 int row_wave(const DevScene& S, uint32_t flags, uint32_t stack_cap)
 {
-  const size_t smem = trace_smem_bytes(stack_cap);
   const uint32_t solver = (flags >> kFlagSolverShift) & 7u;
   const bool solvers = solver != kSolverST && solver != kSolverBBox;
   return with_kind(S.kind, [&](auto k) {
     constexpr uint32_t K = decltype(k)::value;
     auto kernel = solvers ? k_trace<false, true, false, K, kFrame> : k_trace<false, false, false, K, kFrame>;
-    return wave_blocks(reinterpret_cast<const void*>(kernel), smem, S);
+    return wave_blocks(reinterpret_cast<const void*>(kernel), trace_smem_bytes(stack_cap, shared_ray(K, kFrame)), S);
   });
 }
 
@@ -2297,7 +2329,7 @@ int lambert_wave(const DevScene& S, uint32_t stack_cap)
   return with_kind(S.kind, [&](auto k) {
     constexpr uint32_t K = decltype(k)::value;
     return wave_blocks(reinterpret_cast<const void*>(k_render_lambert<false, K>),
-                       trace_smem_bytes(stack_cap, shared_ray(K)), S);
+                       trace_smem_bytes(stack_cap, shared_ray(K, kMany)), S);
   });
 }
 

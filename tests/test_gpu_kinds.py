@@ -103,3 +103,39 @@ def test_split_tiles_of_repeated_frames_match_oracle(cuda, kind, width, height):
         sc.sync()
         assert np.array_equal(image.cpu().numpy(), shade)
     sc.close()
+
+
+@pytest.mark.parametrize("rays", [47361, 52001, 66305])
+def test_rows_around_a_wave_match_oracle(cuda, rays):
+    """Rows on scenes of all kinds whose warps of 16 rays are more than a wave
+    of the frames' kernel, and the first size of 32 rays to a warp."""
+    sc = _scene(KINDS["all"])
+    r = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=320, height=240))[:rays]
+    got = _trace(cuda, sc, r, 0, 0, True, 1)
+    want = po.port_trace(sc.export_arrays(), r)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+    sc.close()
+
+
+def test_mixed_batches_match_oracle(cuda):
+    """Cameras and Lambert passes of a scene of all kinds, whose kernels keep
+    the ray and its inverse in shared memory."""
+    torch = cuda
+    from graphic_lab_task_b200.lrt import CameraBatch
+    sc = _scene(KINDS["all"])
+    cams = wl.sphere_cameras(5, radius=3.2, res_min=17, res_max=90, seed=8)
+    b = CameraBatch(sc, cams)
+    h = torch.zeros(b.total_rays * 8, dtype=torch.float32, device="cuda")
+    b.trace(h.data_ptr())
+    b.sync()
+    rays = np.concatenate([wl.eye_rays_host(c) for c in cams])
+    want = po.port_trace(sc.export_arrays(), rays)
+    got = h.cpu().numpy().view(HIT_DTYPE).reshape(-1)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+    image = torch.zeros(len(rays), dtype=torch.float32, device="cuda")
+    r = torch.from_numpy(rays).cuda()
+    sc.render_lambert(r.data_ptr(), len(rays), wl.LIGHT, image.data_ptr())
+    sc.sync()
+    assert np.array_equal(image.cpu().numpy(), po.port_render_lambert(sc.export_arrays(), rays, wl.LIGHT))
+    b.close()
+    sc.close()
