@@ -79,16 +79,20 @@ struct Hit {
 //     7 shared), 1280x720 - / 534 / 534 / 565, 2560x1440 - / 1,275 / 1,214 /
 //     1,262, 56,064 rays in rows - / 406 / 364 / 371; fused render 1280x720 - /
 //     579 / 581 / 609, 2560x1440 - / 1,400 / 1,400 / 1,426
-//   all kinds, render of all modes: LAMBERT with a transparent mesh, 640x360
+//   render of all modes, LAMBERT with a transparent material: all kinds, 640x360
 //     1,122 / 1,193 / 1,264 / 1,448, 1280x720 1,410 / 1,410 / 1,538 / 1,650,
-//     2560x1440 of 80 instances 9,330 / 8,960 / 9,608 / 9,516
+//     2560x1440 of 80 instances 9,330 / 8,960 / 9,608 / 9,516; 256^3 bricks,
+//     640x360 2,050 / 2,400 / - / 2,700, 1920x1080 4,860 / 5,370 / - / 5,060,
+//     2560x1440 7,730 / 7,880 / - / 7,430; 200k-triangle mesh, 1280x720 - / 393 /
+//     452 / 474, 2560x1440 - / 815 / 815 / 825; 256 instances, 1280x720 - / 888 /
+//     1,132 / 1,189
 constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
 constexpr int kModes = 2;            // the render of all modes, samples and transparency
 constexpr int kManyWaves = 12;       // scenes without bricks: k_trace takes the kernel for many from here on
 constexpr int min_blocks(uint32_t kind, int size)
 {
-  if (kind == kKindBricks) return size == kMany ? 7 : 5;
-  if (kind == kKindNoBricks) return size == kMany ? 8 : 6;
+  if (kind == kKindBricks) return size == kModes ? 4 : size == kMany ? 7 : 5;
+  if (kind == kKindNoBricks) return size == kModes ? 5 : size == kMany ? 8 : 6;
   return size == kModes ? 4 : size == kMany ? 6 : 5;
 }
 
