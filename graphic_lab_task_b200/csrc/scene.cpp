@@ -500,7 +500,12 @@ bool need_normal(const lrt_preset& p)
 
 namespace {
 
-constexpr size_t kParallelPairs = 1u << 15;
+// From this many leaves on a geometry is validated by all cores, whose start
+// and end take about 10 us.  Measured (host part of a commit, one core / eight):
+// 5,500 leaves 0.11 / 0.09 ms, 10,900 0.28 / 0.12, 32,500 1.05 / 0.22.  (A
+// geometry's own size counts: by the scene's, a commit of 4,000 meshes of 12
+// triangles went to all cores 8,000 times, 0.4 -> 9.9 ms.)
+constexpr size_t kParallelLeaves = 8192;
 
 // The checks of validate's walk over geometry g's BLAS on all cores: from the
 // root breadth first until there are subtrees for every core, then each
@@ -541,7 +546,7 @@ bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVe
     }
     level.swap(next);
   }
-#pragma omp parallel for schedule(dynamic, 1) reduction(max : deepest) reduction(&& : ok)
+#pragma omp parallel for schedule(dynamic, 1) reduction(max : deepest) reduction(&& : ok) if (level.size() > 1)
   for (size_t i = 0; i < level.size(); i++) {
     std::vector<Item> todo{level[i]};
     while (ok && !todo.empty()) {
@@ -628,7 +633,7 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
   }
   const size_t P = geomChecked ? 0 : h.allNodePairs.size();
   HostVec<uint32_t> pairGeom(P);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (P >= 4 * kParallelLeaves)
   for (size_t i = 0; i < P; i++) pairGeom[i] = ~0u;
   for (size_t g = 0; g < G && !geomChecked; g++) {
     const lrt_geom_data& gd = h.geomData[g];
@@ -642,8 +647,9 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
     uint32_t maxDepth = 0;
     // The largest trees are walked by all cores first; only if that finds the
     // tree sound (it marks every pair it reaches) is the walk below left out.
-    const bool sound = P >= kParallelPairs && walk_blas(h, uint32_t(g), a0, a1, pairGeom, maxDepth);
-    if (P >= kParallelPairs && !sound)
+    const bool large = a1 - a0 >= kParallelLeaves;
+    const bool sound = large && walk_blas(h, uint32_t(g), a0, a1, pairGeom, maxDepth);
+    if (large && !sound)
       for (size_t i = 0; i < P; i++)
         if (pairGeom[i] == uint32_t(g)) pairGeom[i] = ~0u;
     std::vector<std::pair<uint32_t, uint32_t>> st;
@@ -677,19 +683,22 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
       I.hasTriangles = true;
       if (gd.type != LRT_TYPE_MESH_TRIANGLE) return fail(s, LRT_ERR_BAD_SCENE, "triangle geometry %zu has type %u", g, gd.type);
       if (gd.offset[0] % 3 != 0) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu index offset not a multiple of 3", g);
-      // all cores first; only a leaf that fails is looked for again, in order
-      bool sound2 = true;
-      const uint64_t nidx = h.indices.size(), nprim = h.primIndices.size(), nvert = h.vertPos.size() / 4;
+      // large ones by all cores first; only a leaf that fails is looked for again, in order
+      bool sound2 = false;
+      if (large) {
+        sound2 = true;
+        const uint64_t nidx = h.indices.size(), nprim = h.primIndices.size(), nvert = h.vertPos.size() / 4;
 #pragma omp parallel for schedule(static) reduction(&& : sound2)
-      for (uint32_t a = a0; a < a1; a++) {
-        const uint32_t pk = h.primIdCount[a];
-        const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
-        if (cnt && (uint64_t(gd.offset[0]) + (st0 + cnt) * 3 > nidx || uint64_t(gd.offset[0]) / 3 + st0 + cnt > nprim)) {
-          sound2 = false;
-          continue;
+        for (uint32_t a = a0; a < a1; a++) {
+          const uint32_t pk = h.primIdCount[a];
+          const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
+          if (cnt && (uint64_t(gd.offset[0]) + (st0 + cnt) * 3 > nidx || uint64_t(gd.offset[0]) / 3 + st0 + cnt > nprim)) {
+            sound2 = false;
+            continue;
+          }
+          for (uint64_t q = 3 * st0; q < 3 * (st0 + cnt); q++)
+            sound2 = sound2 && uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + q] < nvert;
         }
-        for (uint64_t q = 3 * st0; q < 3 * (st0 + cnt); q++)
-          sound2 = sound2 && uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + q] < nvert;
       }
       for (uint32_t a = a0; a < a1 && !sound2; a++) {
         const uint32_t pk = h.primIdCount[a];

@@ -1,5 +1,7 @@
 """Validation of trees large enough for the walk on all cores: faults are
 found and named as by the sequential walk."""
+import time
+
 import numpy as np
 import pytest
 
@@ -85,3 +87,22 @@ def test_depth_of_a_large_tree(arrays):
     with pytest.raises(LrtError) as e:
         sc.upload_arrays(a)
     assert e.value.status == 2 and "depth 90" in str(e.value)
+
+
+def test_many_small_meshes_are_validated_by_one_core():
+    """4,000 meshes of 12 triangles: starting all cores for each of them made
+    the commit take a tenth of the time that the adders take (0.5% without; the
+    bound is six times that)."""
+    v, t = wl.noisy_sphere(3, seed=1)
+    ratio = []
+    for _ in range(5):
+        sc = SceneRT()
+        t0 = time.perf_counter()
+        for _ in range(4000):
+            g = sc.AddGeom_Triangles3f(v, t)
+        sc.AddInstance(g, wl.IDENTITY)
+        t1 = time.perf_counter()
+        sc.CommitScene(host_only=True)
+        ratio.append((time.perf_counter() - t1) / (t1 - t0))
+        sc.close()
+    assert min(ratio) < 0.03, ratio
