@@ -122,9 +122,16 @@ struct DevGeom {
   uint32_t triBase;   // triangles: GeomData.offset.x / 3
   uint32_t sdfId;     // SDF: GeomData.offset.x (index into roots/headers)
   uint32_t sdfRoot;   // SDF: root node index of this model
-  uint32_t _pad;
+  uint32_t firstVert; // triangles: GeomData.offset.y
 };
 static_assert(sizeof(DevGeom) == 32, "DevGeom is 32 bytes");
+
+// One block of the kernel that makes the triangle soup: up to kSoupThreads
+// entries of the leaf table of one triangle geometry.
+constexpr uint32_t kSoupThreads = 256;
+struct SoupBlock {
+  uint32_t geom, firstLeaf;
+};
 
 struct DevSbs {
   uint64_t denseBase;   // first float of node `root` in sbsDense

@@ -2,9 +2,11 @@
 // host (compiled with -ffp-contract=off so every float is computed exactly
 // as the reference computes it on the fly).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <functional>
 #include <limits>
+#include <utility>
 
 #include "layout.h"
 
@@ -23,6 +25,7 @@ void build_geoms(const HostArrays& h, std::vector<DevGeom>& out)
     d.aabbBase = h.startEnd[2 * g];
     if (d.tag == LRT_TAG_TRIANGLE) {
       d.triBase = gd.offset[0] / 3;
+      d.firstVert = gd.offset[1];
     } else {
       d.sdfId = gd.offset[0];
       if (d.tag == LRT_TAG_SDF_BRICK) d.sdfRoot = h.sdfSBSRoots[d.sdfId];
@@ -41,6 +44,80 @@ uint64_t triangle_slots(const HostArrays& h, size_t g)
     if (cnt) ntri = std::max<uint64_t>(ntri, uint64_t(pk & kStartMask) + cnt);
   }
   return ntri;
+}
+
+// {A, B-A, C-A} per reordered triangle slot; IntersectAllTrianglesInLeaf
+// computes exactly these differences (BVH2Common.cpp:1585-1589).
+void build_tri_soup(const HostArrays& h, std::vector<float>& soup)
+{
+  soup.assign(h.indices.size() / 3 * 12, 0.0f);
+  for (size_t g = 0; g < h.geomData.size(); g++) {
+    if (h.geomTags[g] != LRT_TAG_TRIANGLE) continue;
+    const uint64_t base = h.geomData[g].offset[0] / 3, firstVert = h.geomData[g].offset[1];
+    for (uint32_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a++) {
+      const uint32_t pk = h.primIdCount[a];
+      const uint64_t first = base + (pk & kStartMask), end = first + ((pk & kSizeMask) >> 28);
+      for (uint64_t t = first; t < end; t++) {
+        const float* P[3];
+        for (int c = 0; c < 3; c++) P[c] = h.vertPos.data() + 4 * (firstVert + h.indices[3 * t + c]);
+        float* o = soup.data() + 12 * t;
+        for (int k = 0; k < 3; k++) {
+          o[k] = P[0][k];
+          o[4 + k] = P[1][k] - P[0][k];
+          o[8 + k] = P[2][k] - P[0][k];
+        }
+      }
+    }
+  }
+}
+
+bool build_soup_blocks(const HostArrays& h, std::vector<SoupBlock>& blocks)
+{
+  blocks.clear();
+  std::vector<std::pair<uint64_t, uint64_t>> ranges; // slots
+  size_t meshes = 0;
+  for (uint32_t tag : h.geomTags) meshes += tag == LRT_TAG_TRIANGLE;
+  for (size_t g = 0; g < h.geomData.size(); g++) {
+    if (h.geomTags[g] != LRT_TAG_TRIANGLE) continue;
+    for (uint64_t a = h.startEnd[2 * g]; a < h.startEnd[2 * g + 1]; a += kSoupThreads)
+      blocks.push_back({uint32_t(g), uint32_t(a)});
+    const uint64_t base = h.geomData[g].offset[0] / 3, slots = meshes > 1 ? triangle_slots(h, g) : 0;
+    if (slots) ranges.push_back({base, base + slots});
+  }
+  std::sort(ranges.begin(), ranges.end());
+  for (size_t i = 1; i < ranges.size(); i++)
+    if (ranges[i].first < ranges[i - 1].second) return false;
+  return true;
+}
+
+bool build_node_records(const HostArrays& h, const std::vector<DevGeom>& geoms, const HostVec<uint32_t>& owner,
+                        HostVec<lrt_bvh_node_pair>& records, bool& clean)
+{
+  records.resize(h.allNodePairs.size());
+  clean = true;
+  bool fits = true;
+  for (size_t i = 0; i < records.size(); i++) {
+    const lrt_bvh_node* in[2] = {&h.allNodePairs[i].left, &h.allNodePairs[i].right};
+    lrt_bvh_node* out[2] = {&records[i].left, &records[i].right};
+    for (int j = 0; j < 2; j++) {
+      const lrt_bvh_node n = *in[j];
+      uint32_t word = n.leftOffset;
+      if ((word & kLeafBit) && word != kLeafNormal) {
+        if (owner[i] != ~0u)
+          word = kLeafBit | (h.primIdCount[geoms[owner[i]].aabbBase + (word & kStartMask)] & ~kLeafBit);
+        fits = fits && word != kLeafNormal;
+      }
+      int nans = 0;
+      for (int k = 0; k < 3; k++) nans += std::isnan(n.boxMin[k]) + std::isnan(n.boxMax[k]);
+      clean = clean && (nans == 0 || nans == 6);
+      const float box[6] = {n.boxMin[0], n.boxMax[0], n.boxMin[1], n.boxMax[1], n.boxMin[2], n.boxMax[2]};
+      char* o = reinterpret_cast<char*>(out[j]);
+      std::memcpy(o, box, sizeof(box));
+      std::memcpy(o + 24, &word, 4);
+      std::memcpy(o + 28, &n.escapeIndex, 4);
+    }
+  }
+  return fits;
 }
 
 // Surface-voxel masks of every brick from its dense corner grid (see

@@ -11,6 +11,17 @@ void build_geoms(const HostArrays& h, std::vector<DevGeom>& out);
 // Records of triangle geometry g in the triangle soup (one past the largest
 // leaf range of its leaf table).
 uint64_t triangle_slots(const HostArrays& h, size_t g);
+// The triangle soup, made on the host: the slots that a leaf covers (geometry
+// by geometry), zeros elsewhere.
+void build_tri_soup(const HostArrays& h, std::vector<float>& soup);
+// The blocks that make it on the device, geometry by geometry.  False if two
+// geometries share slots: their blocks must then run in that order.
+bool build_soup_blocks(const HostArrays& h, std::vector<SoupBlock>& blocks);
+// The node records of a scene without bricks (owner: the geometry of each
+// pair), made on the host.  clean: no box has some but not six NaN coordinates.
+// False if a leaf entry would read as the empty leaf's word.
+bool build_node_records(const HostArrays& h, const std::vector<DevGeom>& geoms, const HostVec<uint32_t>& owner,
+                        HostVec<lrt_bvh_node_pair>& records, bool& clean);
 void build_sbs_dense(const HostArrays& h, std::vector<DevSbs>& sbs, std::vector<float>& dense);
 void build_sbs_masks(const HostArrays& h, std::vector<DevSbs>& sbs, const std::vector<float>& dense,
                      std::vector<uint32_t>& mask);
