@@ -284,14 +284,13 @@ lrt_status finish(lrt_scene* s, cudaStream_t stream, StreamSlot* slot, bool coun
   return LRT_OK;
 }
 
-// Host-pointer trace of ordinary memory, of fewer rays than the pipeline
-// takes: the rays are
+// Host-pointer trace of ordinary memory, of at most kStageMaxRays: the rays are
 // copied into page-locked memory, from which the kernel reads them and into
 // which it writes the hits and its error word, so that the call is one launch
 // and one synchronisation.  Device staging took two pageable copies, a memset
 // and a read of the slot's state around the same kernel, each with a
 // synchronisation of its own.  Measured (us, device staging -> this): one
-// ray 55.6 -> 34.8, 4,099 rays 164 -> 112.  False if the memory cannot be
+// ray 55.6 -> 28-35, 4,099 rays 125-164 -> 90-112.  False if the memory cannot be
 // had (the caller then stages on the device).
 bool host_stage(DeviceScene* d, uint64_t n)
 {
@@ -789,7 +788,7 @@ lrt_status lrt_trace_nearest(lrt_scene* s, const float* rays, lrt_hit* hits, uin
       return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot, 8, uint32_t((n + 7) / 8));
     return launch(s, reinterpret_cast<const float4*>(rays), hits, n, stream, flags, slot);
   }
-  if (n < kPipeMinRays && !(flags & LRT_TRACE_COUNT_WORK) && pageable(rays) && pageable(hits) && host_stage(d, n))
+  if (n <= kStageMaxRays && !(flags & LRT_TRACE_COUNT_WORK) && pageable(rays) && pageable(hits) && host_stage(d, n))
     return trace_host_staged(s, rays, hits, n, stream, flags, slot);
   if (n > d->cap) {
     if (d->rays) cudaFree(d->rays);

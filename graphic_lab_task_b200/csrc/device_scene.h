@@ -31,10 +31,17 @@ constexpr int kPipeStreams = kPipeTrace + kPipeTraceStreams;
 constexpr uint64_t kPipeChunk = 262144;   // 8 MiB of rays in, 8 MiB of hits out
 constexpr uint64_t kPipeChunkMin = 32768; // first and last chunks
 constexpr uint64_t kPipeMinRays = 262144;
-// Host-pointer traces of fewer rays go through page-locked memory that the
-// kernel reads and writes over the bus; its size in rays grows in powers of
-// two from kStageMinRays.
+// Host-pointer traces of at most kStageMaxRays go through page-locked memory
+// that the kernel reads and writes over the bus; its size in rays grows in
+// powers of two from kStageMinRays.  From there on the copies to and from the
+// device are the faster way: one thread's copies to and from the staging memory
+// and the kernel's reads over the bus cost more than the calls they spare.
+// Measured (us, device / staged): 200k-triangle mesh, 8,192 rays 145 / 107,
+// 32,768 263 / 250, 50,000 349 / 390, 262,143 1,128 / 1,314; 256^3 bricks, 32,768
+// 382 / 367, 65,536 571 / 605, 262,143 1,514 / 1,605; mixed scene, 32,768 619 /
+// 614, 50,000 708 / 729, 262,143 2,324 / 2,505.
 constexpr uint64_t kStageMinRays = 4096;
+constexpr uint64_t kStageMaxRays = 32768;
 constexpr uint64_t kStageHeader = 256; // error word
 
 // Tile schedule of the image-order launches of one image size on one stream

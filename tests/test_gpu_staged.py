@@ -1,5 +1,6 @@
 """Host-pointer traces of fewer rays than the pipeline takes (page-locked
-staging that the kernel reads and writes over the bus) equal device traces."""
+staging that the kernel reads and writes over the bus, and above its size
+buffers on the device) equal device traces."""
 import numpy as np
 import pytest
 
@@ -20,7 +21,7 @@ def test_staged_sizes_match_device_trace(cuda):
                    wl.similarity(0.5, (1.0, 0.5, 0.2)))
     sc.CommitScene()
     rng = np.random.default_rng(5)
-    for n in (1, 2, 37, 4096, 4097, 20000, 94719, 94721, 150001, 262143, 3):
+    for n in (1, 2, 37, 4096, 4097, 20000, 32768, 32769, 94719, 94721, 150001, 262143, 3):
         o = rng.normal(size=(n, 3))
         o *= 3.0 / np.linalg.norm(o, axis=1, keepdims=True)
         d = rng.uniform(-1.2, 1.2, (n, 3)) - o
