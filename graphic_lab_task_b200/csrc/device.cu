@@ -54,14 +54,13 @@ bool boxes_clean(const lrt_bvh_node* n, size_t count)
 }
 
 // Turns `count` uploaded nodes into node records in place (device_layout.h).
-// owner: the geometry of each node pair.
-// flags |= 1 for a box with some but not six NaN coordinates, |= 2 for a leaf
-// entry that would read as the empty leaf's word.
+// owner: the geometry of each node pair.  *unclean: a box has some but not six
+// NaN coordinates.
 __global__ void __launch_bounds__(256) k_node_records(float4* __restrict__ nodes, uint64_t count,
                                                       const uint32_t* __restrict__ owner,
                                                       const DevGeom* __restrict__ geoms,
                                                       const uint32_t* __restrict__ leafTable,
-                                                      uint32_t* __restrict__ flags)
+                                                      uint32_t* __restrict__ unclean)
 {
   const uint64_t i = uint64_t(blockIdx.x) * 256 + threadIdx.x;
   if (i >= count) return;
@@ -70,10 +69,9 @@ __global__ void __launch_bounds__(256) k_node_records(float4* __restrict__ nodes
   if ((word & kLeafBit) && word != kLeafNormal) {
     const uint32_t g = owner[i >> 1];
     if (g != ~0u) word = kLeafBit | (leafTable[geoms[g].aabbBase + (word & kStartMask)] & ~kLeafBit);
-    if (word == kLeafNormal) atomicOr(flags, 2u);
   }
   const int nans = isnan(a.x) + isnan(a.y) + isnan(a.z) + isnan(b.x) + isnan(b.y) + isnan(b.z);
-  if (nans != 0 && nans != 6) atomicOr(flags, 1u);
+  if (nans != 0 && nans != 6) *unclean = 1u;
   nodes[2 * i] = make_float4(a.x, b.x, a.y, b.y);
   nodes[2 * i + 1] = make_float4(a.z, b.z, __uint_as_float(word), b.w);
 }
@@ -504,11 +502,6 @@ lrt_status tri_soup(lrt_scene* s)
   return LRT_OK;
 }
 
-lrt_status records_fail(lrt_scene* s)
-{
-  return fail(s, LRT_ERR_UNSUPPORTED, "a BLAS leaf of 7 primitives starts at 2^28 - 1");
-}
-
 // Makes the node records of a scene without bricks from its uploaded BLAS
 // pairs and finds whether their boxes are clean.
 lrt_status node_records(lrt_scene* s, uint64_t count)
@@ -529,8 +522,7 @@ lrt_status node_records(lrt_scene* s, uint64_t count)
   cudaFree(owner);
   cudaFree(flags);
   if (e != cudaSuccess) return cuda_fail(s, e, "node records");
-  if (found & 2u) return records_fail(s);
-  d->pairsClean = !(found & 1u);
+  d->pairsClean = !found;
   return LRT_OK;
 }
 
@@ -556,11 +548,7 @@ lrt_status device_upload(lrt_scene* s)
   build_geoms(h, geoms);
   build_sbs_dense(h, sbs, dense);
   build_sbs_masks(h, sbs, dense, mask);
-  uint32_t kinds = 0;
-  for (uint32_t t : h.geomTags)
-    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
-           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
-  S.kind = kinds == kKindBricks ? kKindBricks : !(kinds & kKindBricks) ? kKindNoBricks : kKindAll;
+  S.kind = kernel_kind(h);
   // Only a brick geometry's pairs are pruned.  (SBS arrays that no geometry
   // names change nothing: the scene's pairs become node records then, of which
   // there is one copy.)
@@ -570,10 +558,7 @@ lrt_status device_upload(lrt_scene* s)
   // (records of few pairs are made on the host, before the upload)
   const bool hostRecords = S.kind == kKindNoBricks && h.allNodePairs.size() < kHostRecordPairs;
   HostVec<lrt_bvh_node_pair> records;
-  if (hostRecords && !build_node_records(h, geoms, s->pairGeom, records, d->pairsClean)) {
-    device_release(s);
-    return records_fail(s);
-  }
+  if (hostRecords) d->pairsClean = build_node_records(h, geoms, s->pairGeom, records);
   const HostVec<lrt_bvh_node_pair>& pairs = prune ? pruned : hostRecords ? records : h.allNodePairs;
   lrt_status st = LRT_OK;
 #define UP(dst, vec, T, name)                                                                        \

@@ -90,23 +90,33 @@ bool build_soup_blocks(const HostArrays& h, std::vector<SoupBlock>& blocks)
   return true;
 }
 
+uint32_t kernel_kind(const HostArrays& h)
+{
+  uint32_t kinds = 0;
+  for (uint32_t t : h.geomTags)
+    kinds |= t == LRT_TAG_TRIANGLE ? kKindTriangles : t == LRT_TAG_SDF_NODE ? kKindNodes
+           : t == LRT_TAG_SDF_BRICK ? kKindBricks : 0u;
+  if (kinds == kKindBricks) return kKindBricks;
+  if (kinds & kKindBricks) return kKindAll;
+  // (of 7 primitives from 2^28 - 1 on, or of a geometry without leaf code)
+  bool asEmpty = false;
+  for (uint32_t entry : h.primIdCount) asEmpty |= (entry | kLeafBit) == kLeafNormal;
+  return asEmpty ? kKindAll : kKindNoBricks;
+}
+
 bool build_node_records(const HostArrays& h, const std::vector<DevGeom>& geoms, const HostVec<uint32_t>& owner,
-                        HostVec<lrt_bvh_node_pair>& records, bool& clean)
+                        HostVec<lrt_bvh_node_pair>& records)
 {
   records.resize(h.allNodePairs.size());
-  clean = true;
-  bool fits = true;
+  bool clean = true;
   for (size_t i = 0; i < records.size(); i++) {
     const lrt_bvh_node* in[2] = {&h.allNodePairs[i].left, &h.allNodePairs[i].right};
     lrt_bvh_node* out[2] = {&records[i].left, &records[i].right};
     for (int j = 0; j < 2; j++) {
       const lrt_bvh_node n = *in[j];
       uint32_t word = n.leftOffset;
-      if ((word & kLeafBit) && word != kLeafNormal) {
-        if (owner[i] != ~0u)
-          word = kLeafBit | (h.primIdCount[geoms[owner[i]].aabbBase + (word & kStartMask)] & ~kLeafBit);
-        fits = fits && word != kLeafNormal;
-      }
+      if ((word & kLeafBit) && word != kLeafNormal && owner[i] != ~0u)
+        word = kLeafBit | (h.primIdCount[geoms[owner[i]].aabbBase + (word & kStartMask)] & ~kLeafBit);
       int nans = 0;
       for (int k = 0; k < 3; k++) nans += std::isnan(n.boxMin[k]) + std::isnan(n.boxMax[k]);
       clean = clean && (nans == 0 || nans == 6);
@@ -117,7 +127,7 @@ bool build_node_records(const HostArrays& h, const std::vector<DevGeom>& geoms, 
       std::memcpy(o + 28, &n.escapeIndex, 4);
     }
   }
-  return fits;
+  return clean;
 }
 
 // Surface-voxel masks of every brick from its dense corner grid (see

@@ -17,11 +17,14 @@ void build_tri_soup(const HostArrays& h, std::vector<float>& soup);
 // The blocks that make it on the device, geometry by geometry.  False if two
 // geometries share slots: their blocks must then run in that order.
 bool build_soup_blocks(const HostArrays& h, std::vector<SoupBlock>& blocks);
-// The node records of a scene without bricks (owner: the geometry of each
-// pair), made on the host.  clean: no box has some but not six NaN coordinates.
-// False if a leaf entry would read as the empty leaf's word.
+// The kind of kernels that trace the scene: kKindBricks, kKindNoBricks or
+// kKindAll.  The last serves all scenes, and also one without bricks whose leaf
+// table holds an entry that would read as the empty leaf's word in a record.
+uint32_t kernel_kind(const HostArrays& h);
+// The node records of a scene of kKindNoBricks (owner: the geometry of each
+// pair), made on the host.  False if a box has some but not six NaN coordinates.
 bool build_node_records(const HostArrays& h, const std::vector<DevGeom>& geoms, const HostVec<uint32_t>& owner,
-                        HostVec<lrt_bvh_node_pair>& records, bool& clean);
+                        HostVec<lrt_bvh_node_pair>& records);
 void build_sbs_dense(const HostArrays& h, std::vector<DevSbs>& sbs, std::vector<float>& dense);
 void build_sbs_masks(const HostArrays& h, std::vector<DevSbs>& sbs, const std::vector<float>& dense,
                      std::vector<uint32_t>& mask);

@@ -103,7 +103,7 @@ static void soup()
 static void records()
 {
   HostArrays h;
-  h.primIdCount = {0x12345u, 0xA0000007u, 0x7FFFFFFFu};
+  h.primIdCount = {0x12345u, 0xA0000007u};
   h.allNodePairs.resize(3);
   HostVec<uint32_t> owner(3);
   owner[0] = owner[1] = 0, owner[2] = ~0u;
@@ -118,8 +118,7 @@ static void records()
       n.escapeIndex = 77 + i;
     }
   HostVec<lrt_bvh_node_pair> out;
-  bool clean = false;
-  expect(build_node_records(h, geoms, owner, out, clean) && clean, "records of sound pairs");
+  expect(build_node_records(h, geoms, owner, out), "records of sound pairs");
   const uint32_t want[3][2] = {{1u, 0xA0000007u}, {kLeafNormal, 0x80012345u}, {0x80000002u, 0x80000000u}};
   for (uint32_t i = 0; i < 3; i++)
     for (uint32_t j = 0; j < 2; j++) {
@@ -133,9 +132,32 @@ static void records()
       expect(w[6] == want[i][j] && w[7] == 77 + i, "words of a record");
     }
   h.allNodePairs[1].left.boxMin[1] = NAN;
-  expect(build_node_records(h, geoms, owner, out, clean) && !clean, "a box with one NaN is not clean");
+  expect(!build_node_records(h, geoms, owner, out), "a box with one NaN is not clean");
   for (int k = 0; k < 3; k++) h.allNodePairs[1].left.boxMin[k] = h.allNodePairs[1].left.boxMax[k] = NAN;
-  expect(build_node_records(h, geoms, owner, out, clean) && clean, "a box of NaNs is clean");
+  expect(build_node_records(h, geoms, owner, out), "a box of NaNs is clean");
+}
+
+// Kernels by geometry kind; those for all kinds where a leaf entry would read
+// as the empty leaf's word.
+static void kinds()
+{
+  HostArrays h;
+  h.primIdCount = {1u, 0x7FFFFFFEu};
+  const struct {
+    std::vector<uint32_t> tags;
+    uint32_t kind;
+  } want[] = {{{LRT_TAG_TRIANGLE}, kKindNoBricks},
+              {{LRT_TAG_SDF_NODE, LRT_TAG_TRIANGLE}, kKindNoBricks},
+              {{LRT_TAG_NONE}, kKindNoBricks},
+              {{LRT_TAG_SDF_BRICK}, kKindBricks},
+              {{LRT_TAG_SDF_BRICK, LRT_TAG_SDF_NODE}, kKindAll}};
+  for (uint32_t odd : {0u, 0x7FFFFFFFu, 0xFFFFFFFFu}) {
+    h.primIdCount.back() = odd;
+    for (const auto& w : want) {
+      h.geomTags = w.tags;
+      expect(kernel_kind(h) == (odd && w.kind == kKindNoBricks ? kKindAll : w.kind), "kernels of a scene");
+    }
+  }
 }
 
 // Rays to a warp around the sizes from which a launch takes larger groups,
@@ -156,6 +178,7 @@ int main()
   slots();
   soup();
   records();
+  kinds();
   rows();
   return failed;
 }

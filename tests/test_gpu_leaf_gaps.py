@@ -90,3 +90,25 @@ def test_many_small_meshes_are_uploaded_together(cuda):
         ratio.append((time.perf_counter() - t1) / (t1 - t0))
         sc.close()
     assert min(ratio) < 0.15, ratio
+
+
+@pytest.mark.parametrize("entry", [0x7FFFFFFF, 0xFFFFFFFF, 0x7FFFFFFE])
+def test_entries_that_read_as_an_empty_leaf(cuda, entry):
+    """A geometry without leaf code may have any leaf entries: the scene is
+    taken, and the others' hits are the oracle's."""
+    sc = SceneRT()
+    for k in range(2):
+        sc.AddInstance(sc.AddGeom_Triangles3f(*wl.noisy_sphere(12, seed=k)), wl.similarity(0.6, (1.1 * k - 0.6, 0, 0)))
+    sc.CommitScene(host_only=True)
+    a = {k: v.copy() for k, v in sc.export_arrays().items()}
+    a["geomTags"][1] = 0
+    first = int(a["startEnd"].reshape(-1, 2)[1, 0])
+    a["primIdCount"][first:] = entry
+    rays = wl.eye_rays_host(wl.camera((0.3, 0.4, 3.5), width=90, height=70))
+    want = po.port_trace(a, rays)
+    sc = SceneRT()
+    sc.upload_arrays(a)
+    got = sc.RayQuery_NearestHitBatch(rays)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+    assert (want["primId"] != MISS).mean() > 0.03
+    sc.close()
