@@ -510,8 +510,8 @@ constexpr size_t kParallelLeaves = 8192;
 // The checks of validate's walk over geometry g's BLAS on all cores: from the
 // root breadth first until there are subtrees for every core, then each
 // subtree by itself.  A pair reached twice (by whichever core comes second),
-// an index out of range or a depth over the bound gives false, and validate's
-// own walk then says which.
+// an index out of range or a depth over the bound gives false, as does a core
+// that gets no memory, and validate's own walk then says which.
 bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVec<uint32_t>& pairGeom,
                uint32_t& maxDepth)
 {
@@ -548,12 +548,16 @@ bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVe
   }
 #pragma omp parallel for schedule(dynamic, 1) reduction(max : deepest) reduction(&& : ok) if (level.size() > 1)
   for (size_t i = 0; i < level.size(); i++) {
-    std::vector<Item> todo{level[i]};
-    while (ok && !todo.empty()) {
-      const Item it = todo.back();
-      todo.pop_back();
-      deepest = std::max(deepest, it.second);
-      ok = visit(it, todo);
+    try {
+      std::vector<Item> todo{level[i]};
+      while (ok && !todo.empty()) {
+        const Item it = todo.back();
+        todo.pop_back();
+        deepest = std::max(deepest, it.second);
+        ok = visit(it, todo);
+      }
+    } catch (const std::bad_alloc&) { // (must not leave the parallel region)
+      ok = false;
     }
   }
   maxDepth = deepest;

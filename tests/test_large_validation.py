@@ -1,11 +1,14 @@
 """Validation of trees large enough for the walk on all cores: faults are
 found and named as by the sequential walk."""
+import os
+import subprocess
 import time
 
 import numpy as np
 import pytest
 
-from graphic_lab_task_b200 import LrtError, SceneRT, workloads as wl
+from conftest import ROOT
+from graphic_lab_task_b200 import LrtError, SceneRT, build as b, workloads as wl
 
 
 def _arrays():
@@ -106,3 +109,12 @@ def test_many_small_meshes_are_validated_by_one_core():
         ratio.append((time.perf_counter() - t1) / (t1 - t0))
         sc.close()
     assert min(ratio) < 0.03, ratio
+
+
+def test_cores_without_memory_leave_the_walk_to_the_caller(tmp_path):
+    exe, so = str(tmp_path / "host_alloc_failure"), os.path.dirname(b.LIB)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I" + b.INCLUDE, os.path.join(ROOT, "tests", "host_alloc_failure.cpp"),
+                    "-o", exe, b.LIB, "-Wl,-rpath," + so, "-lpthread"], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, env=dict(os.environ, OMP_NUM_THREADS="4"))
+    assert r.returncode == 0 and "status 0" in r.stdout, (r.returncode, r.stdout, r.stderr)
+    assert int(r.stdout.split()[-1]) > 0  # cores were refused memory
