@@ -669,14 +669,19 @@ const char* lbvh_build(const float* boxes6, uint32_t n, std::vector<uint32_t>& o
   return run(in, n, 0, false, order, &inner, nullptr, nullptr);
 }
 
-const char* lbvh_build_blas(const float* verts4, uint32_t nverts, const uint32_t* tris, uint32_t n, uint32_t maxLeaf,
+const char* lbvh_build_blas(const float* boxes6, const float* verts4, uint32_t nverts, const uint32_t* tris, uint32_t n,
+                            uint32_t maxLeaf,
                             const std::function<LbvhPairOut*(size_t)>& pairsAt, std::vector<uint32_t>& startCount,
                             std::vector<uint32_t>& order)
 {
   BuildInput in;
-  in.verts4 = verts4;
-  in.nverts = nverts;
-  in.tris = tris;
+  if (boxes6) {
+    in.boxes6 = boxes6;
+  } else {
+    in.verts4 = verts4;
+    in.nverts = nverts;
+    in.tris = tris;
+  }
   return run(in, n, std::max(1u, maxLeaf), true, order, nullptr, &pairsAt, &startCount);
 }
 

@@ -29,16 +29,18 @@ struct LbvhPairOut {
   float node[2][8];
 };
 
-// Builds the tree over the boxes of n triangles (three indices each into
-// nverts float4 vertices, all in range; host memory) as lbvh_build does and
-// emits a triangle BLAS from it on the device, exactly as the host emitter would from the same tree with inner
-// nodes of at most maxLeaf boxes collapsed into leaves: the pairs (relative
-// child indices; copied to pairsAt(count), which the caller makes room for),
-// the leaf table entries Pack(start, count) in leaf-id order (`startCount`)
-// and the box order of the leaves (`order`: position -> box).  Needs
-// n > maxLeaf (a root that is one leaf has no pairs to emit).  Returns nullptr
-// on success, else a message.
-const char* lbvh_build_blas(const float* verts4, uint32_t nverts, const uint32_t* tris, uint32_t n, uint32_t maxLeaf,
+// Builds the tree over the boxes of n triangles as lbvh_build does and emits a
+// triangle BLAS from it on the device, exactly as the host emitter would from
+// the same tree with inner nodes of at most maxLeaf boxes collapsed into
+// leaves.  The boxes are boxes6, or (nullptr) are made on the device from the
+// triangles: three indices each into nverts float4 vertices, all in range (host
+// memory).  Out come the pairs (relative child indices; copied to
+// pairsAt(count), which the caller makes room for), the leaf table entries
+// Pack(start, count) in leaf-id order (`startCount`) and the box order of the
+// leaves (`order`: position -> box).  Needs n > maxLeaf (a root that is one leaf
+// has no pairs to emit).  Returns nullptr on success, else a message.
+const char* lbvh_build_blas(const float* boxes6, const float* verts4, uint32_t nverts, const uint32_t* tris, uint32_t n,
+                            uint32_t maxLeaf,
                             const std::function<LbvhPairOut*(size_t)>& pairsAt, std::vector<uint32_t>& startCount,
                             std::vector<uint32_t>& order);
 

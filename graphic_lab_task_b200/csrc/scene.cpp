@@ -975,9 +975,12 @@ lrt_status lrt_add_geom_triangles3f(lrt_scene* s, const float* vpos, size_t nver
 
   const size_t nt = nidx / 3;
   const float* V = h.vertPos.data() + 4 * oldV;
-  // (the device builder makes the boxes itself)
+  // The device builder makes the boxes itself, unless that takes more vertices
+  // there than the triangles can use: its scratch is kept, and stays in
+  // proportion to the triangles.
   const bool onDevice = (flags & LRT_BUILD_LOW) && nt > s->primsInLeaf;
-  std::vector<Aabb> boxes(onDevice ? 0 : nt);
+  const bool deviceBoxes = onDevice && nvert <= 3 * nt;
+  std::vector<Aabb> boxes(deviceBoxes ? 0 : nt);
 #pragma omp parallel for schedule(static)
   for (size_t t = 0; t < boxes.size(); t++) {
     boxes[t].reset();
@@ -1013,7 +1016,8 @@ lrt_status lrt_add_geom_triangles3f(lrt_scene* s, const float* vpos, size_t nver
       static_assert(sizeof(LbvhPairOut) == sizeof(lrt_bvh_node_pair), "a pair is 64 bytes");
       const size_t base = h.allNodePairs.size();
       err = lbvh_build_blas(
-          V, uint32_t(nvert), tri, uint32_t(nt), s->primsInLeaf,
+          deviceBoxes ? nullptr : reinterpret_cast<const float*>(boxes.data()), V, uint32_t(nvert), tri, uint32_t(nt),
+          s->primsInLeaf,
           [&](size_t count) {
             h.allNodePairs.resize(base + count);
             lrt_bvh_node_pair* p = h.allNodePairs.data() + base;

@@ -170,3 +170,24 @@ def test_device_build_is_much_faster_on_large_meshes(cuda):
             best = min(best, time.perf_counter() - t0)
         times[flags] = best
     assert times[BUILD_LOW] < 0.5 * times[BUILD_HIGH], times
+
+
+def test_unused_vertices_take_no_scratch(cuda):
+    """A few triangles of a large vertex array: the same BLAS as over the used
+    vertices alone, and no device memory kept for the others."""
+    torch = cuda
+    v, t = wl.noisy_sphere(20, seed=2)
+    few = SceneRT()
+    few.AddGeom_Triangles3f(v, t, flags=BUILD_LOW)
+    want = few.export_arrays()
+    many = np.zeros((12 << 20, 3), np.float32)  # 192 MB as float4
+    many[:len(v)] = v
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    sc = SceneRT()
+    sc.AddGeom_Triangles3f(many, t, flags=BUILD_LOW)
+    got = sc.export_arrays()
+    for k in ("allNodePairs", "primIdCount", "indices", "primIndices"):
+        assert np.array_equal(got[k].view(np.uint8), want[k].view(np.uint8)), k
+    assert free - torch.cuda.mem_get_info()[0] < 64 << 20
+    sc.close()
