@@ -564,6 +564,34 @@ bool walk_blas(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1, HostVe
   return ok;
 }
 
+// The checks of validate over triangle geometry g's leaves on all cores.
+// (Parallel loops stand outside validate: what they take by address is loaded
+// again in every step of its other loops, 16.8 -> 22 ms for 256^3 bricks.)
+bool leaves_sound(const HostArrays& h, uint32_t g, uint32_t a0, uint32_t a1)
+{
+  const lrt_geom_data& gd = h.geomData[g];
+  const uint64_t nidx = h.indices.size(), nprim = h.primIndices.size(), nvert = h.vertPos.size() / 4;
+  bool sound = true;
+#pragma omp parallel for schedule(static) reduction(&& : sound)
+  for (uint32_t a = a0; a < a1; a++) {
+    const uint32_t pk = h.primIdCount[a];
+    const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
+    if (cnt && (uint64_t(gd.offset[0]) + (st0 + cnt) * 3 > nidx || uint64_t(gd.offset[0]) / 3 + st0 + cnt > nprim)) {
+      sound = false;
+      continue;
+    }
+    for (uint64_t q = 3 * st0; q < 3 * (st0 + cnt); q++)
+      sound = sound && uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + q] < nvert;
+  }
+  return sound;
+}
+
+void no_owners(HostVec<uint32_t>& pairGeom)
+{
+#pragma omp parallel for schedule(static) if (pairGeom.size() >= 4 * kParallelLeaves)
+  for (size_t i = 0; i < pairGeom.size(); i++) pairGeom[i] = ~0u;
+}
+
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -637,8 +665,7 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
   }
   const size_t P = geomChecked ? 0 : h.allNodePairs.size();
   HostVec<uint32_t> pairGeom(P);
-#pragma omp parallel for schedule(static) if (P >= 4 * kParallelLeaves)
-  for (size_t i = 0; i < P; i++) pairGeom[i] = ~0u;
+  no_owners(pairGeom);
   for (size_t g = 0; g < G && !geomChecked; g++) {
     const lrt_geom_data& gd = h.geomData[g];
     const uint32_t tag = h.geomTags[g];
@@ -688,22 +715,7 @@ lrt_status validate(lrt_scene* s, SceneInfo* info)
       if (gd.type != LRT_TYPE_MESH_TRIANGLE) return fail(s, LRT_ERR_BAD_SCENE, "triangle geometry %zu has type %u", g, gd.type);
       if (gd.offset[0] % 3 != 0) return fail(s, LRT_ERR_BAD_SCENE, "geometry %zu index offset not a multiple of 3", g);
       // large ones by all cores first; only a leaf that fails is looked for again, in order
-      bool sound2 = false;
-      if (large) {
-        sound2 = true;
-        const uint64_t nidx = h.indices.size(), nprim = h.primIndices.size(), nvert = h.vertPos.size() / 4;
-#pragma omp parallel for schedule(static) reduction(&& : sound2)
-        for (uint32_t a = a0; a < a1; a++) {
-          const uint32_t pk = h.primIdCount[a];
-          const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
-          if (cnt && (uint64_t(gd.offset[0]) + (st0 + cnt) * 3 > nidx || uint64_t(gd.offset[0]) / 3 + st0 + cnt > nprim)) {
-            sound2 = false;
-            continue;
-          }
-          for (uint64_t q = 3 * st0; q < 3 * (st0 + cnt); q++)
-            sound2 = sound2 && uint64_t(gd.offset[1]) + h.indices[gd.offset[0] + q] < nvert;
-        }
-      }
+      const bool sound2 = large && leaves_sound(h, uint32_t(g), a0, a1);
       for (uint32_t a = a0; a < a1 && !sound2; a++) {
         const uint32_t pk = h.primIdCount[a];
         const uint64_t st0 = pk & kStartMask, cnt = (pk & kSizeMask) >> 28;
