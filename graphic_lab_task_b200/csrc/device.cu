@@ -656,6 +656,7 @@ lrt_status device_upload(lrt_scene* s)
     return st;
   }
   S.sms = uint32_t(sms);
+  S.instCount = uint32_t(d->instCount);
   // The allocation-free trace's static array is looked up here, with the
   // scene's device current, not in the trace call: under lazy module loading
   // the first lookup loads this file's module and places the array in device
@@ -704,6 +705,7 @@ lrt_status device_update_instances(lrt_scene* s)
   put(h.instanceData.data(), h.instanceData.size(), sizeof(lrt_instance_data), d->instCount,
       reinterpret_cast<const void**>(&d->S.instances), "instances");
   if (st != LRT_OK) return st;
+  d->S.instCount = uint32_t(d->instCount);
   d->cleanBoxes = d->pairsClean && boxes_clean(h.nodesTLAS.data(), h.nodesTLAS.size());
   return LRT_OK;
 }

@@ -71,11 +71,10 @@ inline __host__ __device__ uint64_t sched_words(uint64_t tiles)
 constexpr uint32_t kNormalWords = 16;
 constexpr uint32_t kColourWord = 12;
 // After them, in the kernels for many waves of scenes with bricks, the ray's
-// origin, direction and inverse direction: they are only read when the TLAS is
-// walked on, and out of the march's registers they let 7 blocks per SM run with
-// few spills (6 with none where a scene holds other kinds too).  The inverse
-// spares three divisions per instance: mixed scenes 1-2%.
-constexpr uint32_t kRayWord = 16, kRayWords = 9;
+// origin and direction, and where a scene holds other kinds too its inverse
+// direction: they are only read when the TLAS is walked on, and out of the
+// march's registers they let 7 blocks per SM run with few spills (6 with none).
+constexpr uint32_t kRayWord = 16, kRayWords = 6, kRayInverseWords = 9;
 constexpr uint32_t kMaxStackDev = 80; // STACK_SIZE of raytrace_common.h:36
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kMaxVoxelSteps = 4096u; // voxel-march cap per brick (the reference loop is unbounded)
@@ -206,13 +205,13 @@ constexpr uint32_t kKindTriangles = 1, kKindNodes = 2; // triangles; frame-octre
 constexpr uint32_t kKindBricks = 4, kKindNoBricks = kKindTriangles | kKindNodes, kKindAll = 7;
 
 // Dynamic shared memory of a trace kernel with stack_cap stack entries per
-// thread; sharedRay: with the words of kRayWord.
-constexpr size_t trace_smem_bytes(uint32_t stack_cap, bool sharedRay = false)
+// thread and ray_words of the words at kRayWord.
+constexpr size_t trace_smem_bytes(uint32_t stack_cap, uint32_t ray_words = 0)
 {
-  return size_t(stack_cap + kNormalWords + (sharedRay ? kRayWords : 0u)) * kTraceThreads * sizeof(uint32_t);
+  return size_t(stack_cap + kNormalWords + ray_words) * kTraceThreads * sizeof(uint32_t);
 }
 // What any of them may ask for.
-constexpr size_t kMaxTraceSmem = trace_smem_bytes(kMaxStackDev + 1, true);
+constexpr size_t kMaxTraceSmem = trace_smem_bytes(kMaxStackDev + 1, kRayInverseWords);
 
 struct DevNode { // a node record
   float4 a, b;
@@ -243,6 +242,7 @@ struct DevScene {
   uint32_t voxelStepCap; // bounded SBS voxel march (kMaxVoxelSteps unless set)
   uint32_t kind;         // kernel kind of the scene: kKindBricks, kKindNoBricks or kKindAll
   uint32_t sms;          // the device's multiprocessors (persistent grids are multiples of it)
+  uint32_t instCount;    // instances (chooses between kernels)
   // byte ranges streamed into L2 at the start of a trace launch (16-byte
   // aligned bases, sizes multiples of 16; 0 bytes: none)
   const char* pfPtr[kPrefetchRanges];

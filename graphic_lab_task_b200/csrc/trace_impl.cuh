@@ -88,7 +88,16 @@ struct Hit {
 //     1,132 / 1,189
 constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
 constexpr int kModes = 2;            // the render of all modes, samples and transparency
-constexpr int kManyWaves = 12;       // scenes without bricks: k_trace takes the kernel for many from here on
+// Scenes without bricks: k_trace takes the kernel for many (8 blocks) in
+// launches of more than kManyWaves of its waves on more than kManyInstances
+// instances.  What it gains are long walks over many instances; single models
+// are slower with it at every size.  Measured (us, 6-7 blocks / 8): 1,024
+// instances, 1920x1080 752 / 757 (14 waves), 2560x1440 1,088 / 1,071 (24), 4096^2
+// 5,600 / 5,490, their sorted bounce 5,920 / 5,640; 512 instances, 1920x1080 459 /
+// 471, 4096x2304 1,300 / 1,285; 256, 2560x1440 498 / 502, 4096x2304 892 / 886; a
+// 200k-triangle mesh 1920x1080 236 / 248, 4096^2 1,253 / 1,285.
+constexpr int kManyWaves = 20;
+constexpr uint32_t kManyInstances = 256;
 constexpr int min_blocks(uint32_t kind, int size)
 {
   if (kind == kKindBricks) return size == kModes ? 4 : size == kMany ? 7 : 5;
@@ -101,9 +110,13 @@ constexpr int min_blocks(uint32_t kind, int size)
 // took 12,556 us and a Lambert step 2,684; from shared memory 12,357 and 2,671,
 // and at 72 (7 blocks) 12,189 and 2,603.  Frames gain nothing (fused render 377
 // -> 384).
-constexpr bool shared_ray(uint32_t kind, int size)
+// The kernels for all kinds keep the inverse direction beside it: mixed scenes
+// gain 1-2% by the three divisions that each further instance is spared, the
+// one instance of a brick set loses as much by the larger shared memory.
+// Returns the words per thread (kRayWord).
+constexpr uint32_t shared_ray(uint32_t kind, int size)
 {
-  return size == kMany && kind != kKindNoBricks;
+  return size != kMany || kind == kKindNoBricks ? 0 : kind == kKindBricks ? kRayWords : kRayInverseWords;
 }
 
 // f(std::integral_constant<uint32_t, kind>) for a scene's kernel kind.
@@ -120,9 +133,10 @@ auto with_kind(uint32_t kind, F f)
 // there); the plain trace kernel instantiates none.  nrec points at this thread's
 // kNormalWords shared-memory words (thread-strided), where a sphere-traced
 // hit leaves what its normal is computed from once the traversal has ended.
-template <bool COUNT, bool RECORD = false, bool SOLVERS = false, uint32_t KIND = kKindAll, bool SHARED_RAY = false>
+template <bool COUNT, bool RECORD = false, bool SOLVERS = false, uint32_t KIND = kKindAll, uint32_t SHARED_RAY = 0>
 struct Ctx {
-  static constexpr bool kSharedRay = SHARED_RAY; // the ray is in the words of kRayWord
+  static constexpr bool kSharedRay = SHARED_RAY != 0; // the ray is in the words of kRayWord
+  static constexpr bool kSharedInverse = SHARED_RAY == kRayInverseWords; // and its inverse direction
   static constexpr uint32_t kKind = KIND;
   static constexpr bool kCount = COUNT;
   static constexpr bool kRecord = RECORD;
@@ -554,7 +568,8 @@ __device__ void octree_brick(CTX& c, const DevGeom& g, f3 ray_pos, f3 ray_dir, f
   uint32_t steps = 0;
   // In brick-only scenes the march goes on to the next voxel whose sphere trace
   // may hit, in which the warp's lanes then trace together.  The kernels of all
-  // kinds trace in each voxel: what the march has to keep until the trace took
+  // kinds trace in each voxel, without the reach test (with it images of a mixed
+  // scene took 1-4% longer, Lambert passes 1-7%): what the march has to keep until the trace took
   // 100 bytes of spills more in them (mixed scene at 2560x1440 in 7 blocks 1,408
   // -> 1,250 us, the latter with the ray in shared memory).
   constexpr bool kToCandidate = CTX::kKind == kKindBricks;
@@ -918,8 +933,10 @@ __device__ __forceinline__ void walk_begin(CTX& c, Walk& w, float4 pn, float4 df
     float* rw = c.nrec + kRayWord * st;
     rw[0] = pn.x, rw[st] = pn.y, rw[2 * st] = pn.z;
     rw[3 * st] = df.x, rw[4 * st] = df.y, rw[5 * st] = df.z;
-    const f3 inv = safe_inverse(mk3(df.x, df.y, df.z));
-    rw[6 * st] = inv.x, rw[7 * st] = inv.y, rw[8 * st] = inv.z;
+    if constexpr (CTX::kSharedInverse) {
+      const f3 inv = safe_inverse(mk3(df.x, df.y, df.z));
+      rw[6 * st] = inv.x, rw[7 * st] = inv.y, rw[8 * st] = inv.z;
+    }
   } else {
     w.pos = mk3(pn.x, pn.y, pn.z);
     w.dir = mk3(df.x, df.y, df.z);
@@ -946,12 +963,12 @@ __device__ __forceinline__ uint32_t walk_tlas(CTX& c, Walk& w, uint32_t* stack)
     const float* rw = c.nrec + kRayWord * st;
     pos = mk3(rw[0], rw[st], rw[2 * st]);
     dir = mk3(rw[3 * st], rw[4 * st], rw[5 * st]);
-    inv = mk3(rw[6 * st], rw[7 * st], rw[8 * st]);
+    if constexpr (CTX::kSharedInverse) inv = mk3(rw[6 * st], rw[7 * st], rw[8 * st]);
   } else {
     pos = w.pos;
     dir = w.dir;
-    inv = safe_inverse(dir);
   }
+  if constexpr (!CTX::kSharedInverse) inv = safe_inverse(dir);
   const bool fast = fast_nodes(S, pos, dir, inv);
   uint32_t travFlags = 0, leftOffset = 0;
   if (fast)
@@ -2259,14 +2276,14 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
   const bool solvers = solver != kSolverST && solver != kSolverBBox;
   // image order (IMG) is its own instantiation, so that the tile schedule
   // costs the row-order kernel nothing
-  auto go = [&](auto kernel, bool sharedRay) {
-    const size_t smem = trace_smem_bytes(stack_cap, sharedRay);
+  auto go = [&](auto kernel, uint32_t rayWords) {
+    const size_t smem = trace_smem_bytes(stack_cap, rayWords);
     kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
         S, rays, hits, n, work_counter, counters, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr, group);
     return cudaGetLastError();
   };
   if (count) { // the counting kernels are compiled for all kinds
-    constexpr bool R = shared_ray(kKindAll, kFrame);
+    constexpr uint32_t R = shared_ray(kKindAll, kFrame);
     if (img_w)
       return solvers ? go(k_trace<true, true, true, kKindAll, kFrame>, R)
                      : go(k_trace<true, false, true, kKindAll, kFrame>, R);
@@ -2275,16 +2292,16 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
   }
   return with_kind(S.kind, [&](auto kind) {
     constexpr uint32_t K = decltype(kind)::value;
-    constexpr bool R = shared_ray(K, kFrame);
+    constexpr uint32_t R = shared_ray(K, kFrame);
     // the node solvers spill at any bound: their kernels keep the wider one
     if (solvers)
       return img_w ? go(k_trace<false, true, true, K, kFrame>, R) : go(k_trace<false, true, false, K, kFrame>, R);
     // (brick-only scenes gain nothing from the narrow one here, mixed ones as
     // soon as the launch is more than a wave of the wide one: min_blocks)
     if constexpr (K != kKindBricks) {
-      constexpr bool RM = shared_ray(K, kMany);
+      constexpr uint32_t RM = shared_ray(K, kMany);
       const uint64_t wave = K == kKindAll ? min_blocks(K, kFrame) : kManyWaves * min_blocks(K, kMany);
-      if (uint64_t(blocks) > wave * S.sms)
+      if (uint64_t(blocks) > wave * S.sms && (K == kKindAll || S.instCount > kManyInstances))
         return img_w ? go(k_trace<false, false, true, K, kMany>, RM) : go(k_trace<false, false, false, K, kMany>, RM);
     }
     return img_w ? go(k_trace<false, false, true, K, kFrame>, R) : go(k_trace<false, false, false, K, kFrame>, R);
@@ -2293,7 +2310,7 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
 
 cudaError_t set_trace_smem(uint32_t stack_cap)
 {
-  const int smem = int(trace_smem_bytes(stack_cap, true));
+  const int smem = int(trace_smem_bytes(stack_cap, kRayInverseWords));
   cudaError_t e = cudaSuccess;
   auto set = [&](auto kernel) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

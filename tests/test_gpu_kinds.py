@@ -14,7 +14,7 @@ KINDS = {"triangles": "t", "nodes": "ov", "triangles+nodes": "tov", "bricks": "b
          "bricks+triangles": "bt", "all": "tovb"}
 
 
-def _scene(letters, preset=None):
+def _scene(letters, preset=None, count=None):
     sc = SceneRT(preset=preset or parity_preset())
     sph = wl.spheres(12, seed=4)
     make = {"t": lambda: sc.AddGeom_Triangles3f(*wl.noisy_sphere(24, seed=2)),
@@ -22,7 +22,8 @@ def _scene(letters, preset=None):
             "v": lambda: sc.AddGeom_SdfSVS(wl.svs_from_spheres(sph, 4)),
             "b": lambda: sc.AddGeom_SdfSBS(*wl.sbs_from_spheres(sph, grid_res=32))}
     geoms = [make[k]() for k in letters]
-    for i, m in enumerate(wl.random_instances(3 * len(geoms), seed=6, scale=(0.3, 0.6), trans=1.0)):
+    small = (0.05, 0.1) if count else (0.3, 0.6)
+    for i, m in enumerate(wl.random_instances(count or 3 * len(geoms), seed=6, scale=small, trans=1.0)):
         sc.AddInstance(geoms[i % len(geoms)], m)
     sc.CommitScene()
     return sc
@@ -44,8 +45,7 @@ def _trace(torch, sc, rays, width, height, row, repeat=2):
 @pytest.mark.parametrize("kind", sorted(KINDS))
 @pytest.mark.parametrize("width,height,row", [(53, 41, False), (53, 41, True), (1537, 1237, False), (1537, 1237, True)])
 def test_kinds_match_oracle(cuda, kind, width, height, row):
-    """Ragged frames below and above the size from which scenes without
-    bricks take the kernel for many waves; every pixel of the small frame,
+    """Ragged frames of one wave and of many; every pixel of the small frame,
     every 61st of the large one."""
     sc = _scene(KINDS[kind])
     rays = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=width, height=height))
@@ -138,4 +138,21 @@ def test_mixed_batches_match_oracle(cuda):
     sc.sync()
     assert np.array_equal(image.cpu().numpy(), po.port_render_lambert(sc.export_arrays(), rays, wl.LIGHT))
     b.close()
+    sc.close()
+
+
+@pytest.mark.parametrize("instances", [256, 257])
+@pytest.mark.parametrize("row", [False, True])
+def test_many_waves_of_many_instances_match_oracle(cuda, instances, row):
+    """Scenes without bricks around the instance count from which launches of
+    this size take the kernel for many waves; every 61st ray."""
+    sc = _scene(KINDS["triangles+nodes"], count=instances)
+    width, height = 2051, 1489  # over 20 waves of 8 blocks on 148 SMs
+    assert (width + 7) // 8 * ((height + 3) // 4) > 4 * 20 * 8 * 148
+    rays = wl.eye_rays_host(wl.camera((0.4, 0.6, 3.2), width=width, height=height))
+    got = _trace(cuda, sc, rays, width, height, row)[7::61]
+    want = po.port_trace(sc.export_arrays(), rays[7::61])
+    got = np.ascontiguousarray(got)
+    assert bit_equal(got, want).all(), hit_summary(got, want)
+    assert (want["primId"] != MISS).mean() > 0.02
     sc.close()
