@@ -12,7 +12,7 @@ namespace lrt {
 // Longest-first order of the tiles of an image-order launch.  Each launch
 // times its tiles on lane 0 and sorts the slow ones into three classes by
 // their cost against the previous launch's longest tile (at least 5/8, 3/8,
-// 3/16 of it); the next launch of the same image size on the same stream
+// 1/8 of it); the next launch of the same image size on the same stream
 // (rd) hands out class 0, then 1, then 2, each in the order the tiles
 // finished, then every other tile in natural order (a bitmap skips the
 // listed ones).  If the previous launch was tail-bound (its longest tile
@@ -65,7 +65,7 @@ __device__ __forceinline__ void sched_record(const uint32_t* __restrict__ rd, ui
   }
   const uint32_t mx = rd ? __ldg(rd) : 0u;
   if (mx) {
-    const int cls = listed >= mx / 8 * 5 ? 0 : listed >= mx / 8 * 3 ? 1 : listed >= mx / 16 * 3 ? 2 : 3;
+    const int cls = listed >= mx / 8 * 5 ? 0 : listed >= mx / 8 * 3 ? 1 : listed >= mx / 8 ? 2 : 3;
     if (cls < 3) {
       const uint32_t slot = atomicAdd(wr + 1 + cls, 1u);
       if (slot < tiles) wr[lists + cls * tiles + slot] = tile;

@@ -89,13 +89,13 @@ struct Hit {
 constexpr int kFrame = 0, kMany = 1; // launches of a few waves, of many
 constexpr int kModes = 2;            // the render of all modes, samples and transparency
 // Scenes without bricks: k_trace takes the kernel for many (8 blocks) in
-// launches of more than kManyWaves of its waves on more than kManyInstances
-// instances.  What it gains are long walks over many instances; single models
+// launches of more than kManyWaves of its waves on kManyInstances instances or
+// more.  What it gains are long walks over many instances; single models
 // are slower with it at every size.  Measured (us, 6-7 blocks / 8): 1,024
 // instances, 1920x1080 752 / 757 (14 waves), 2560x1440 1,088 / 1,071 (24), 4096^2
 // 5,600 / 5,490, their sorted bounce 5,920 / 5,640; 512 instances, 1920x1080 459 /
-// 471, 4096x2304 1,300 / 1,285; 256, 2560x1440 498 / 502, 4096x2304 892 / 886; a
-// 200k-triangle mesh 1920x1080 236 / 248, 4096^2 1,253 / 1,285.
+// 471, 4096x2304 1,300 / 1,285; 256, 2560x1440 498 / 502, 4096x2304 892 / 886,
+// 4096^2 in rows 1,925 / 1,851; a 200k-triangle mesh 1920x1080 236 / 248, 4096^2 1,253 / 1,285.
 constexpr int kManyWaves = 20;
 constexpr uint32_t kManyInstances = 256;
 constexpr int min_blocks(uint32_t kind, int size)
@@ -2301,7 +2301,7 @@ cudaError_t launch_trace(const DevScene& S, const float4* rays, lrt_hit* hits, u
     if constexpr (K != kKindBricks) {
       constexpr uint32_t RM = shared_ray(K, kMany);
       const uint64_t wave = K == kKindAll ? min_blocks(K, kFrame) : kManyWaves * min_blocks(K, kMany);
-      if (uint64_t(blocks) > wave * S.sms && (K == kKindAll || S.instCount > kManyInstances))
+      if (uint64_t(blocks) > wave * S.sms && (K == kKindAll || S.instCount >= kManyInstances))
         return img_w ? go(k_trace<false, false, true, K, kMany>, RM) : go(k_trace<false, false, false, K, kMany>, RM);
     }
     return img_w ? go(k_trace<false, false, true, K, kFrame>, R) : go(k_trace<false, false, false, K, kFrame>, R);

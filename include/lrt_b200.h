@@ -366,7 +366,7 @@ lrt_status lrt_trace_sync(lrt_scene* scene, void* stream, int32_t read_counters)
  * (MultiRenderer.cpp:185-202); every hit equals lrt_trace_nearest's for the
  * same ray.  Tiles are scheduled longest first: each launch measures its
  * tiles' durations, and the next launch of the same image size on the same
- * stream starts with the tiles that took at least 5/8, then 3/8, then 3/16 of
+ * stream starts with the tiles that took at least 5/8, then 3/8, then 1/8 of
  * the longest (the rest follow in row order), so that a few slow tiles do
  * not finish last; when the longest tile took longer than the warps were
  * busy on average, the tiles of the first group are each traced by 2 to 8 warps
