@@ -39,7 +39,7 @@ def build(with_reference=True):
     build (oracle/Makefile)."""
     targets = ["port", "wl"]
     src = reference_src() if with_reference else ""
-    if src and os.path.isdir(src):
+    if src and os.path.exists(os.path.join(src, "MultiRenderer", "BVH2Common.cpp")):
         targets += ["ref", "dropin"]
     subprocess.run(["make", "-s", "-C", HERE, "-j8"] + targets, check=True)
 

@@ -153,3 +153,11 @@ def test_transparency_loop_matches_its_statement():
         assert bit_equal(got_h[i:i + 1], h.reshape(1)).all()
     # several layers on some rays: the loop composited more than one surface
     assert (got_t[:, 3] < 0.99).sum() > 20 and np.unique(got_t[:, :3].round(4), axis=0).shape[0] > 10
+
+
+def test_build_without_reference_sources(tmp_path, monkeypatch):
+    """An absent or empty reference checkout leaves the reference build out."""
+    for src in (tmp_path / "absent", tmp_path):
+        monkeypatch.setenv("LRT_REFERENCE", str(src))
+        assert po.reference_src() == str(src)
+        po.build(with_reference=True)
