@@ -42,8 +42,8 @@ SOURCES = {
     "layout.cpp": None,
     "workloads.cpp": None,
 }
-HEADERS = ["trace_impl.cuh", "device_layout.h", "lrt_math.h", "scene.h", "layout.h", "trace_api.h", "device_scene.h", "tile_schedule.h",
-           "lbvh.h"]
+HEADERS = ["trace_impl.cuh", "device_layout.h", "lrt_math.h", "scene.h", "layout.h", "trace_api.h", "device_scene.h",
+           "tile_schedule.h", "lbvh.h"]
 
 
 def _stale(obj, src):

@@ -2227,8 +2227,8 @@ cudaError_t launch_render_lambert(const DevScene& S, const float4* rays, uint64_
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, rays, n, light, image, work_counter, err_word, stack_cap, img_w,
-                                                  img_h, sched_rd, sched_wr);
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
+        S, rays, n, light, image, work_counter, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr);
     return cudaGetLastError();
   });
 }
@@ -2245,8 +2245,8 @@ cudaError_t launch_adjoint_lambert(const DevScene& S, const float4* rays, uint64
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(kMaxTraceSmem));
     if (e != cudaSuccess) return e;
-    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap,
-                                                  img_w, img_h, sched_rd, sched_wr);
+    kernel<<<grid_for(kernel, smem, S, blocks), kTraceThreads, smem, stream>>>(
+        S, rays, n, light, dimage, grad, work_counter, err_word, stack_cap, img_w, img_h, sched_rd, sched_wr);
     return cudaGetLastError();
   });
 }

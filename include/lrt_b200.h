@@ -323,11 +323,11 @@ lrt_status lrt_scene_export(const lrt_scene* scene, lrt_scene_arrays* out);
  * legacy default stream).  With host pointers the call is synchronous.  A
  * warp traces 32 consecutive rays; a trace of at most 448 rays per SM (66,304
  * rays on 148 SMs) gives each warp 16 or 8 rays strided across the call, and a
- * device-pointer trace of more rays that repeats the previous device-pointer trace's ray
- * count on the stream hands its 32-ray groups out in a schedule kept per
- * stream and ray count, as lrt_trace_nearest_image does with its tiles
- * (slowest groups first; LRT_TRACE_NATURAL_ORDER turns it off).  The order
- * never changes a hit. */
+ * device-pointer trace of more rays that repeats the previous device-pointer
+ * trace's ray count on the stream hands its 32-ray groups out in a schedule
+ * kept per stream and ray count, as lrt_trace_nearest_image does with its
+ * tiles (slowest groups first; LRT_TRACE_NATURAL_ORDER turns it off).  The
+ * order never changes a hit. */
 lrt_status lrt_trace_nearest(lrt_scene* scene, const float* rays, lrt_hit* hits, uint64_t n, void* stream,
                              uint32_t flags);
 
